@@ -1,39 +1,69 @@
-// Permanent modulo 3 by Ryser's formula with bit-sliced F_3 row sums.
+// Permanent modulo 3 by Glynn's formula with table lookups over 1024 states.
 //
-//   per(A) = (-1)^n sum_{S subset of columns} (-1)^|S| prod_i sum_{j in S} a_ij
-// over F_3 (rivin-perm perm_mod3.py:143-228, perm_mod3_omp.c, CUDA kernel
-// perm_mod3_cuda.cu:52-131).  Each element of F_3 is two bits (magnitude,
-// sign): 0 = (0, either), 1 = (1,0), -1 = 2 = (1,1); the n row sums of a
-// subset are two n-bit words, and adding or subtracting a canonical column
-// is a few bitwise operations on them (the bipedal formulas of
+//   per(A) = 2^(1-n) sum_d (prod_k d_k) prod_i s_i(d)   over F_3,
+// s_i(d) = sum_j d_j a_ij, last sign fixed: 2^(n-1) sign vectors (2 is a unit
+// modulo 3, 2^(1-n) = (-1)^(n-1)), half of the 2^n subsets of the Ryser walk
+// of rivin-perm perm_mod3.py:143-228, perm_mod3_omp.c and
+// perm_mod3_cuda.cu:52-131.  An element of F_3 is two bits (magnitude, sign):
+// 0 = (0, either), 1 = (1,0), 2 = (1,1); adding or subtracting a canonical
+// element is a few bitwise operations (the bipedal formulas of
 // arXiv:2407.20205; their truth table over every row-sum encoding and
-// canonical column is checked on the host in the tests).  A subset
-// contributes iff every row sum is nonzero (magnitude word full), and then
-// every sign bit is meaningful: sign (-1)^(popcount(sign word) + |S|).
+// canonical column is checked on the host in the tests).
 //
-// GB300 organisation: the 2^n Gray-ordered subsets are cut into aligned
-// chunks, each thread walks a contiguous balanced range of chunks; inside a
-// chunk the walk is unrolled by 8, so the toggled column of 7 of every 8
-// steps (columns 0..2) is a compile-time register operand and only the
-// eighth reads shared memory (uniform across the warp).  Words are 32-bit
-// for n <= 32 (one ALU op per bitwise step) and 64-bit above.  Each thread
-// counts its terms as 1 (for +1) or 2 (for -1), the count mod 3 is reduced
-// per block and added atomically.
+// A term counts only when no row sum is zero, about (2/3)^n of the states
+// for random entries, so the walk is a search for states without a zero row.
+// The low ten columns' signs are spread over a warp: bit k of lane l's word is
+// the state with low signs (k | l << 5).  The high columns are common to the
+// warp, so row i's sum is h_i + low_i(lane, bit), and "row i is nonzero" is a
+// word that depends only on the lane and on h_i in {0, 1, 2}.  For groups of
+// four rows the 81 AND-ed words per lane sit in shared memory ([81][32] words,
+// lane-minor: no bank conflicts).  One high state (1024 sign vectors) is five
+// loads and ANDs for the first 20 rows; (2/3)^20 of the states, about one in
+// four warps, go on to the next groups, and only states with every row
+// nonzero read the rows' sign words.  The 32 lanes hold the high row sums of
+// 32 consecutive high states (row-sliced, one column update per 32 of them)
+// and publish their table offsets through shared memory.
+//
+// Bound by shared-memory loads: 6 loads and ~20 instructions per 1024 states.
+// 35 x 35 random: 22.9 ms a call with the row-sliced Ryser walk (17.5 instructions
+// per subset, ALU pipe 91 % busy), 0.67 ms now (whole call).  Groups of five rows (243
+// words per lane) need 31 KB each and do not fit from order 36 on.  A matrix
+// whose states all survive (equal rows) reads every row's sign word for
+// every high state: ~10 instructions per row and 1024 states, still well
+// below the row-sliced walk, so no other path is kept.
 #include "pg_internal.h"
 
 #include <cstring>
 
 namespace pg {
 
+constexpr int MOD3_THREADS = 1024;   // one block per SM: the tables take up to 212 KB
+constexpr int MOD3_LOW = 10;         // columns spread over word bits (5) and lanes (5)
+constexpr int MOD3_FIRST = 5;        // row groups looked up before the first vote
+constexpr int MOD3_DIGITS = 81;      // states of a group of four rows' high sums
+
 struct Mod3Args {
     const uint64_t *cols;     // [2][n]: magnitude words, then sign words
     int n;
-    uint64_t chunks;
-    int log_len;              // >= 3
+    uint64_t batches;         // 32 high states each
+    int steps;                // high states per batch: 32, fewer below order 16
     unsigned long long *acc;  // zeroed
     int *status;
     volatile const int *abort_flag;
 };
+
+__host__ __device__ constexpr int mod3_groups(int n) {
+    return (n + 3) / 4 < MOD3_FIRST ? MOD3_FIRST : (n + 3) / 4;
+}
+// per-row words [n][3][32]; the magnitude words' space later holds the warps'
+// offset lists (one uint4 per high state)
+__host__ __device__ constexpr size_t mod3_row_bytes(int n) { return (size_t)n * 3 * 32 * 4; }
+__host__ __device__ constexpr size_t mod3_list_bytes(int n) {
+    return mod3_row_bytes(n) > MOD3_THREADS * 16 ? mod3_row_bytes(n) : MOD3_THREADS * 16;
+}
+__host__ __device__ constexpr size_t mod3_smem(int n) {
+    return (size_t)mod3_groups(n) * MOD3_DIGITS * 128 + mod3_row_bytes(n) + mod3_list_bytes(n);
+}
 
 // row sums (m, s) += or -= column (cm, cs) over F_3, bitwise per row
 template <typename W>
@@ -51,89 +81,158 @@ __device__ __forceinline__ void f3_sub(W &m, W &s, W cm, W cs) {
     m = mo;
 }
 
-template <typename W>
-__device__ __forceinline__ int f3_parity(W s) {
-    if constexpr (sizeof(W) == 8) return __popcll((unsigned long long)s) & 1;
-    else return __popc((unsigned)s) & 1;
+// word of the states k = 0..31 whose bit j is set
+__device__ __forceinline__ uint32_t mod3_pattern(int j) {
+    return j == 0 ? 0xaaaaaaaau : j == 1 ? 0xccccccccu : j == 2 ? 0xf0f0f0f0u
+         : j == 3 ? 0xff00ff00u : 0xffff0000u;
 }
 
 template <typename W>
-__global__ void __launch_bounds__(256) mod3_kernel(Mod3Args a) {
-    constexpr int LOGU = 3, U = 1 << LOGU;
-    __shared__ W cm_s[64], cs_s[64];
-    const int n = a.n;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        cm_s[j] = (W)a.cols[j];
-        cs_s[j] = (W)a.cols[n + j];
+__global__ void __launch_bounds__(MOD3_THREADS, 1) mod3_kernel(Mod3Args a) {
+    extern __shared__ uint4 mod3_shared[];
+    const int n = a.n, G = mod3_groups(n);
+    uint32_t *gtab = reinterpret_cast<uint32_t *>(mod3_shared);      // [G][81][32]
+    uint32_t *rsgn = gtab + (size_t)G * MOD3_DIGITS * 32;             // [n][3][32]
+    uint32_t *rmag = rsgn + (size_t)n * 96;                           // [n][3][32], build only
+    uint4 *lists = reinterpret_cast<uint4 *>(rmag);                   // [warps][32]
+    __shared__ uint16_t dmap[256];      // (magnitudes | signs << 4) -> byte offset in a group
+    __shared__ uint64_t cm_s[64], cs_s[64];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = MOD3_THREADS / 32;
+    for (int j = threadIdx.x; j < n; j += MOD3_THREADS) {
+        cm_s[j] = a.cols[j];
+        cs_s[j] = a.cols[n + j];
+    }
+    if (threadIdx.x < 256) {
+        int idx = 0, p3 = 1;
+        for (int t = 0; t < 4; t++, p3 *= 3)
+            if ((threadIdx.x >> t) & 1) idx += p3 * (1 + ((threadIdx.x >> (t + 4)) & 1));
+        dmap[threadIdx.x] = (uint16_t)(idx * 128);
     }
     __syncthreads();
-    const W mask = (W)(n >= 64 ? ~0ull : ((1ull << n) - 1));
-    W c0m = cm_s[0], c0s = cs_s[0], c1m = cm_s[1], c1s = cs_s[1], c2m = cm_s[2], c2s = cs_s[2];
+    const int low = n - 1 < MOD3_LOW ? n - 1 : MOD3_LOW;
+    for (int r = warp; r < n; r += warps) {
+        uint32_t m = 0, s = 0;
+        for (int j = 0; j < low; j++) {
+            if (!((cm_s[j] >> r) & 1)) continue;
+            const uint32_t minus = j < 5 ? mod3_pattern(j) : 0u - ((lane >> (j - 5)) & 1u);
+            f3_add(m, s, 0xffffffffu, ((cs_s[j] >> r) & 1) ? ~minus : minus);
+        }
+        for (int d = 0; d < 3; d++) {
+            uint32_t md = m, sd = s;
+            if (d) f3_add(md, sd, 0xffffffffu, d == 2 ? 0xffffffffu : 0u);
+            rmag[(r * 3 + d) * 32 + lane] = md;
+            rsgn[(r * 3 + d) * 32 + lane] = sd;
+        }
+    }
+    __syncthreads();
+    for (int e = warp; e < G * MOD3_DIGITS; e += warps) {
+        const int g = e / MOD3_DIGITS;
+        int d = e - g * MOD3_DIGITS;
+        uint32_t w = 0xffffffffu;
+        for (int t = 0; t < 4; t++, d /= 3) {
+            const int r = 4 * g + t;
+            if (r < n) w &= rmag[(r * 3 + d % 3) * 32 + lane];
+        }
+        gtab[e * 32 + lane] = w;
+    }
+    __syncthreads();
 
-    const uint64_t T = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t c_begin = tid * a.chunks / T;
-    const uint64_t c_end = (tid + 1) * a.chunks / T;
+    // low states that exist (n - 1 < 10: fewer lanes or word bits) and those
+    // with an odd number of minus signs
+    const uint32_t exist = low < 5 ? (lane == 0 ? (1u << (1 << low)) - 1u : 0u)
+                                   : (lane < (1 << (low - 5)) ? 0xffffffffu : 0u);
+    const uint32_t odd = 0x96696996u ^ (0u - (__popc(lane) & 1u));
+
+    // one contiguous, balanced range of batches per warp
+    const uint64_t TW = (uint64_t)gridDim.x * warps;
+    const uint64_t wid = (uint64_t)blockIdx.x * warps + warp;
+    const uint64_t b_begin = wid * a.batches / TW, b_end = (wid + 1) * a.batches / TW;
+    const char *tab = reinterpret_cast<const char *>(gtab + lane);
+    constexpr int GB = MOD3_DIGITS * 128;
+    uint4 *list = lists + warp * 32;
     unsigned long long count = 0;   // sum of 1 (term +1) or 2 (term -1)
     bool aborted = false;
-    if (c_begin < c_end) {
-        W m = 0, s = 0;
-        const uint64_t start = c_begin << a.log_len;
-        const uint64_t gs = start ^ (start >> 1);
-        for (int j = 0; j < n; j++)
-            if ((gs >> j) & 1) f3_add(m, s, cm_s[j], cs_s[j]);
-        const uint32_t blocks = (1u << a.log_len) >> LOGU;
-        // the host-mapped abort word is read once per 2^20 subsets (per chunk
-        // for longer chunks), from the thread's second period on
-        const uint64_t poll = a.log_len >= 20 ? 0 : (1ull << (20 - a.log_len)) - 1;
-        for (uint64_t c = c_begin; c < c_end; c++) {
-            if (c != c_begin && ((c - c_begin) & poll) == 0 && *a.abort_flag) {
+    // high signs of lane l in batch b: l | gray(b) << 5, bit t the sign of
+    // column 10 + t; the last column's sign is +
+    W m = 0, s = 0;
+    if (b_begin < b_end) {
+        m = (W)cm_s[n - 1];
+        s = (W)cs_s[n - 1];
+        const uint64_t minus = (uint64_t)lane | ((b_begin ^ (b_begin >> 1)) << 5);
+        for (int j = MOD3_LOW; j < n - 1; j++) {
+            if ((minus >> (j - MOD3_LOW)) & 1) f3_sub(m, s, (W)cm_s[j], (W)cs_s[j]);
+            else f3_add(m, s, (W)cm_s[j], (W)cs_s[j]);
+        }
+    }
+
+    // The states `alive` of high state k after the first groups: the other
+    // groups, then the signs.  Everything but the words is warp-uniform.
+    auto finish = [&](int k, uint32_t alive, uint32_t flip) {
+        const W km = __shfl_sync(0xffffffffu, m, k), ks = __shfl_sync(0xffffffffu, s, k);
+        for (int g = MOD3_FIRST; g < G; g++) {
+            const uint32_t e = (uint32_t)((km >> (4 * g)) & 15) | (uint32_t)((ks >> (4 * g)) & 15) << 4;
+            alive &= *reinterpret_cast<const uint32_t *>(tab + g * GB + dmap[e]);
+            if (!__any_sync(0xffffffffu, alive != 0)) return;
+        }
+        uint32_t neg = odd ^ flip ^ (0u - (__popc(k) & 1u));
+        for (int r = 0; r < n; r++) {
+            const int d = ((km >> r) & 1) ? 1 + (int)((ks >> r) & 1) : 0;
+            neg ^= rsgn[(r * 3 + d) * 32 + lane];
+        }
+        count += (unsigned long long)(__popc(alive) + __popc(alive & neg));
+    };
+
+    for (uint64_t b = b_begin; b < b_end; b++) {
+        if (b != b_begin) {
+            // the host-mapped abort word is read once per 2^12 batches, from
+            // the warp's second period on
+            if (((b - b_begin) & 4095) == 0 && __any_sync(0xffffffffu, *a.abort_flag != 0)) {
                 aborted = true;
                 break;
             }
-            for (uint32_t q = 0; q < blocks; q++) {
-                const uint64_t base = (c << a.log_len) | ((uint64_t)q << LOGU);
-#pragma unroll
-                for (int r = 0; r < U; r++) {
-                    const uint64_t i = base | (uint64_t)r;
-                    if (r == 0) {
-                        if (i != start) {
-                            const int j = __ffsll((long long)i) - 1;   // >= LOGU
-                            if (((i >> (j + 1)) & 1) == 0) f3_add(m, s, cm_s[j], cs_s[j]);
-                            else f3_sub(m, s, cm_s[j], cs_s[j]);
-                        }
-                    } else {
-                        const int j = r & 1 ? 0 : (r & 2 ? 1 : 2);
-                        // added when bit j+1 of i is 0 (bit LOGU of i for j = 2)
-                        const bool add = j + 1 < LOGU ? ((r >> (j + 1)) & 1) == 0
-                                                      : ((i >> LOGU) & 1) == 0;
-                        const W cmj = j == 0 ? c0m : (j == 1 ? c1m : c2m);
-                        const W csj = j == 0 ? c0s : (j == 1 ? c1s : c2s);
-                        if (add) f3_add(m, s, cmj, csj);
-                        else f3_sub(m, s, cmj, csj);
-                    }
-                    // Bits above row n stay 0 in both words, so "every row sum
-                    // nonzero" is m == mask.  That is rare (about (2/3)^n for
-                    // random entries), so the sign work sits behind a branch
-                    // that is almost never taken.
-                    // Subset sign (-1)^|S| = (-1)^popcount(gray(i)) = (-1)^r.
-                    if (m == mask) count += (unsigned long long)(1 + (f3_parity(s) ^ (r & 1)));
-                }
-            }
+            // column j turns minus: -2 a = a is added, else 2 a = -a
+            const int z = __ffsll((long long)b) - 1, j = MOD3_LOW + 5 + z;
+            if (((b >> (z + 1)) & 1) == 0) f3_add(m, s, (W)cm_s[j], (W)cs_s[j]);
+            else f3_sub(m, s, (W)cm_s[j], (W)cs_s[j]);
         }
+        uint32_t off[MOD3_FIRST];
+#pragma unroll
+        for (int g = 0; g < MOD3_FIRST; g++)
+            off[g] = dmap[(uint32_t)((m >> (4 * g)) & 15) | (uint32_t)((s >> (4 * g)) & 15) << 4];
+        list[lane] = make_uint4(off[0] | off[1] << 16, off[2] | off[3] << 16, off[4], 0);
+        __syncwarp();
+        const uint32_t flip = 0u - (uint32_t)(b & 1);     // parity of gray(b)
+        for (int k0 = 0; k0 < a.steps; k0 += 4) {
+            uint32_t alive[4];
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                // beyond a.steps (below order 13) the list still holds valid offsets
+                const uint4 o = list[k0 + t];
+                const auto at = [&](int g, uint32_t off) {
+                    return *reinterpret_cast<const uint32_t *>(tab + g * GB + off);
+                };
+                alive[t] = at(0, o.x & 0xffffu) & at(1, o.x >> 16) & at(2, o.y & 0xffffu) &
+                           at(3, o.y >> 16) & at(4, o.z);
+            }
+#pragma unroll
+            for (int t = 0; t < 4; t++)
+                if (k0 + t < a.steps && __any_sync(0xffffffffu, (alive[t] & exist) != 0))
+                    finish(k0 + t, alive[t] & exist, flip);
+        }
+        __syncwarp();
     }
     count %= 3;
-    __shared__ unsigned long long red[8];
+    __shared__ unsigned long long red[MOD3_THREADS / 32];
     __shared__ int any_abort;
     if (threadIdx.x == 0) any_abort = 0;
     __syncthreads();
     if (aborted) any_abort = 1;
-    for (int off = 16; off > 0; off >>= 1) count += __shfl_down_sync(0xffffffffu, count, off);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = count;
+    for (int o = 16; o > 0; o >>= 1) count += __shfl_down_sync(0xffffffffu, count, o);
+    if (lane == 0) red[warp] = count;
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned long long t = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += red[w];
+        for (int w = 0; w < warps; w++) t += red[w];
         atomicAdd(a.acc, t);
         if (any_abort) atomicExch(a.status, 1);
     }
@@ -141,15 +240,12 @@ __global__ void __launch_bounds__(256) mod3_kernel(Mod3Args a) {
 
 template <typename W>
 static cudaError_t launch_mod3(const Mod3Args &a, int sm_count, cudaStream_t s) {
-    int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mod3_kernel<W>, 256, 0);
+    const size_t smem = mod3_smem(a.n);
+    cudaError_t e = cudaFuncSetAttribute(mod3_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem);
     if (e != cudaSuccess) return e;
-    if (per_sm < 1) per_sm = 1;
-    uint64_t blocks = (uint64_t)per_sm * sm_count;
-    const uint64_t max_blocks = (a.chunks + 255) / 256;
-    if (blocks > max_blocks) blocks = max_blocks;
-    if (blocks < 1) blocks = 1;
-    mod3_kernel<W><<<(unsigned)blocks, 256, 0, s>>>(a);
+    const uint64_t blocks = a.batches < (uint64_t)sm_count ? a.batches : (uint64_t)sm_count;
+    mod3_kernel<W><<<(unsigned)blocks, MOD3_THREADS, smem, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -170,13 +266,12 @@ static int mod3_impl(const uint64_t *mags, const uint64_t *sgns, int n, int *out
     std::memset(h, 0, total);
     std::memcpy(h, mags, (size_t)n * 8);
     std::memcpy(h + (size_t)n * 8, sgns, (size_t)n * 8);
-    // 2^n subsets in at most 2^24 aligned chunks of >= 8 subsets
-    const ChunkPlan pl = plan_chunks(n, 3, 1ull << 22);
+    const int high = n - 1 - MOD3_LOW;          // columns common to a warp
     Mod3Args a;
     a.cols = (const uint64_t *)d;
     a.n = n;
-    a.chunks = pl.chunks;
-    a.log_len = pl.log_len;
+    a.batches = high > 5 ? 1ull << (high - 5) : 1;
+    a.steps = high >= 5 ? 32 : high > 0 ? 1 << high : 1;
     a.acc = (unsigned long long *)(d + off_acc);
     a.status = (int *)(d + off_status);
     a.abort_flag = abort_dev;
@@ -187,8 +282,9 @@ static int mod3_impl(const uint64_t *mags, const uint64_t *sgns, int n, int *out
                             ws->stream));
     PG_CUDA(cudaStreamSynchronize(ws->stream));
     if (*(int *)(h + off_status)) return fail(PG_EABORT, "launch aborted by pg_abort()");
+    // 2^(1-n) = (-1)^(n-1) modulo 3
     const unsigned long long total3 = *(unsigned long long *)(h + off_acc) % 3;
-    *out = (int)((n & 1) ? (3 - total3) % 3 : total3);
+    *out = (int)((n & 1) ? total3 : (3 - total3) % 3);
     return PG_OK;
 }
 

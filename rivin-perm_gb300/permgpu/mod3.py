@@ -6,8 +6,8 @@ validation and results:
   permanent_mod3_fast(matrix, num_threads=None)   perm_mod3.py:355-383
   encode_matrix_f3(matrix) / decode_f3_element    perm_mod3.py:62-115
 
-The evaluation is ``pg_permanent_mod3`` (Ryser over F_3 with bit-sliced row
-sums, one launch); there is no CPU path.
+The evaluation is ``pg_permanent_mod3`` (Glynn over F_3 by table lookups, one
+launch); there is no CPU path.
 """
 
 from __future__ import annotations

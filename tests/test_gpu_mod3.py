@@ -41,3 +41,29 @@ def test_identities_up_to_order_40(lib):
         assert lib.permanent_mod3(2 * np.eye(n, dtype=np.int64)) == pow(2, n, 3)
         p = np.eye(n, dtype=np.int64)[np.random.default_rng(n).permutation(n)]
         assert lib.permanent_mod3(-p) == pow(2, n, 3)
+
+
+@pytest.mark.parametrize("n", [3, 5, 6, 7, 10, 11, 12, 15, 16, 17, 20, 21, 24])
+def test_many_survivors_at_table_edges(lib, n):
+    # orders around the table's edges (word bits, lanes, the 32 high states of
+    # a batch, the last row group) with repeated rows, so that most states
+    # keep every row nonzero and reach the sign words
+    rng = np.random.default_rng(900 + n)
+    base = rng.integers(1, 3, (2, n))
+    a = base[rng.integers(0, 2, n)]
+    assert lib.permanent_mod3(a) == oracle.permanent_mod_p(a, 3, 8)
+    a[n // 2, : n // 2] = 0
+    assert lib.permanent_mod3(a) == oracle.permanent_mod_p(a, 3, 8)
+
+
+def test_expansion_beyond_one_word(lib):
+    # per of a block-diagonal matrix is the product of the blocks', at orders
+    # whose rows take more than one 32-bit word
+    rng = np.random.default_rng(33)
+    for n, k in ((33, 13), (36, 18), (38, 19)):
+        a = np.zeros((n, n), np.int64)
+        a[:k, :k] = rng.integers(0, 3, (k, k))
+        a[k:, k:] = rng.integers(0, 3, (n - k, n - k))
+        want = lib.permanent_mod3(a[:k, :k]) * lib.permanent_mod3(a[k:, k:]) % 3
+        p, q = rng.permutation(n), rng.permutation(n)
+        assert lib.permanent_mod3(a[p][:, q]) == want
