@@ -191,10 +191,13 @@ static uint32_t float_bits(int64_t v) {
 struct ExactPlan {
     int n = 0, G = 0, NG = 0, NL = 0, need_bits = 0;
     int fr = 0;                  // float rows per group (0: integer rows)
-    // bit-sliced 0/1 kernel (binary_glynn.cuh): offset planes K > 0,
-    // tracking words W, tracked (even-degree) rows, padded rows
-    int planes = 0, words_tracked = 0, ntracked = 0, npad = 0, bin_split = 0;
-    size_t off_deg = 0, off_cm = 0, off_trm = 0, off_toff = 0;
+    // 0/1 kernel (binary_glynn.cuh): bits of the largest even row's half
+    // degree (0: the general kernel), tracked (even-degree) rows, padded
+    // rows, table entries and list words, Gray window
+    int planes = 0, ntracked = 0, npad = 0, entries = 0, list_words = 0, sparse = 0,
+        warps = 0;
+    size_t off_deg = 0, off_trk = 0;
+    uint64_t lo = 0, hi = 0;
     ChunkPlan chunks{};
     uint64_t chunk0 = 0;
     uint64_t blocks = 0;
@@ -209,13 +212,44 @@ struct ExactPlan {
     volatile int *abort_dev = nullptr;
 };
 
-// The bit-sliced kernel for a 0/1 matrix of order BINARY_MIN_N..48: the
-// even-degree rows are tracked for zero row sums, rows are padded to NPAD
-// (degree 1, no columns) and grouped by degree like the exact kernel; the
-// last column keeps the fixed sign.  The share of states with no zero row
-// is estimated from 1024 sampled states: above BINARY_MAX_SURVIVORS the
-// exact evaluations would cost more than the general kernel, which then
-// runs (as it does when the matrix is not 0/1 or no compiled shape fits).
+int binary_pack_groups(int NPAD, const int *caps, int rows, int *group, int *warps) {
+    std::vector<int> by(rows);
+    for (int e = 0; e < rows; e++) by[e] = e;
+    std::stable_sort(by.begin(), by.end(), [&](int x, int y) { return caps[x] > caps[y]; });
+    // rows in descending order, each into the group with the smallest table
+    const auto pack = [&](int T) -> size_t {
+        std::vector<double> size(T, 1.0);
+        for (int e : by) {
+            const int g = (int)(std::min_element(size.begin(), size.end()) - size.begin());
+            size[g] *= caps[e] + 1;
+            group[e] = g;
+        }
+        double total = 1;
+        for (double v : size) total += v;
+        return total < 65536 ? (size_t)total : 65536;
+    };
+    const int most = binary_max_threads(NPAD) / 32;
+    for (int w = most; w >= most / 4; w -= most / 4)
+        for (int T = 1; T <= rows; T++) {
+            const int words = (T + 3) / 4 * 4;
+            if (binary_smem(NPAD, (int)pack(T), words, w) > BIN_SMEM) continue;
+            // the lookups run in fours: use all of them, with smaller tables
+            const int T4 = words < rows ? words : rows;
+            *warps = w;
+            if (T4 == T || binary_smem(NPAD, (int)pack(T4), words, w) <= BIN_SMEM) return T4;
+            pack(T);
+            return T;
+        }
+    return 0;
+}
+
+// The 0/1 kernel for a 0/1 matrix of order BINARY_MIN_N..48: the even-degree
+// rows are packed into zero-row tables, rows are padded to NPAD (degree 1,
+// no columns) and grouped by degree like the exact kernel; the last column
+// keeps the fixed sign.  The share of states with no zero row is estimated
+// from 1024 sampled states: above BINARY_MAX_SURVIVORS the exact evaluations
+// would cost more than the general kernel, which then runs (as it does when
+// the matrix is not 0/1 or no compiled shape fits).
 static bool plan_build_binary(const int64_t *A, int n, ExactPlan *P) {
     if (!EXACT_BINARY || n < BINARY_MIN_N || n > 48) return false;
     for (size_t i = 0; i < (size_t)n * n; i++)
@@ -240,7 +274,6 @@ static bool plan_build_binary(const int64_t *A, int n, ExactPlan *P) {
     if (tracked.empty()) return false;          // no row can vanish: every state counts
     int K = 2;
     while ((1 << K) <= maxh) K++;
-    const int W = tracked.size() > 32 ? 2 : 1;
     // sampled share of states with no zero row (fixed LCG, Gray words)
     uint64_t x = 0x9e3779b97f4a7c15ull;
     int survive = 0;
@@ -255,45 +288,57 @@ static bool plan_build_binary(const int64_t *A, int n, ExactPlan *P) {
         survive += !zero;
     }
     if (survive > BINARY_MAX_SURVIVORS * samples) return false;
-    // evaluation from the warp's common high bits pays from a survivor
-    // share of about 1/64 (40x40 Bernoulli(1/2): ~8 %; the grid: ~0.1 %)
-    P->bin_split = survive * 64 >= samples;
     std::vector<int> order(NPAD);
     int G = 0;
     for (int g : {10, 8, 7, 6, 5}) {
-        if (!binary_compiled(NPAD, g, K, W)) continue;
+        if (!binary_compiled(NPAD, g)) continue;
         if (exact_group_rows(deg.data(), NPAD, g, order.data())) { G = g; break; }
     }
     if (!G) return false;
+    const int nt = (int)tracked.size();
+    constexpr uint64_t low_mask = (1ull << BIN_LOW) - 1;
+    std::vector<int> caps(nt), group(nt);
+    for (int e = 0; e < nt; e++) caps[e] = __builtin_popcountll(rows[tracked[e]] & low_mask) + 1;
+    const int groups = binary_pack_groups(NPAD, caps.data(), nt, group.data(), &P->warps);
+    if (!groups) return false;
     P->planes = K;
-    P->words_tracked = W;
-    P->ntracked = (int)tracked.size();
+    P->ntracked = nt;
     P->npad = NPAD;
     P->G = G;
     P->NG = (NPAD + G - 1) / G;
     P->NL = P->NG + (NPAD > 32 ? 2 : 1);
     P->off_deg = align_up((size_t)NPAD * 8, 16);
-    P->off_cm = align_up(P->off_deg + (size_t)NPAD * 4, 256);
-    P->off_trm = align_up(P->off_cm + 64 * 8, 256);
-    P->off_toff = align_up(P->off_trm + 64 * 8, 16);
-    P->off_acc = align_up(P->off_toff + 64 * 4, 256);
+    P->off_trk = align_up(P->off_deg + (size_t)NPAD * 4, 256);
+    P->off_acc = align_up(P->off_trk + 48 * sizeof(BinTrack), 256);
     P->image.assign(P->off_acc, 0);
     uint64_t *rm = (uint64_t *)P->image.data();
     int32_t *dg = (int32_t *)(P->image.data() + P->off_deg);
-    uint64_t *cm = (uint64_t *)(P->image.data() + P->off_cm);
-    uint64_t *trm = (uint64_t *)(P->image.data() + P->off_trm);
-    int32_t *toff = (int32_t *)(P->image.data() + P->off_toff);
+    BinTrack *trk = (BinTrack *)(P->image.data() + P->off_trk);
     for (int i = 0; i < NPAD; i++) {
         rm[i] = rows[order[i]];
         dg[i] = (int32_t)deg[order[i]];
     }
-    for (size_t e = 0; e < tracked.size(); e++) {
-        const int r = tracked[e];
-        trm[e] = rows[r];
-        toff[e] = (int32_t)(deg[r] / 2);        // u = deg/2 - (ones in minus columns)
-        for (int j = 0; j < n - 1; j++)
-            if ((rows[r] >> j) & 1) cm[j] |= 1ull << e;
+    int w = 0, entries = 1;                      // entry 0: all ones
+    for (int g = 0; g < groups; g++) {
+        int stride = 1;
+        for (int e = 0; e < nt; e++) {
+            if (group[e] != g) continue;
+            BinTrack &t = trk[w++];
+            t.high = rows[tracked[e]] >> BIN_LOW;
+            t.low = (uint16_t)(rows[tracked[e]] & low_mask);
+            t.half = (uint8_t)(deg[tracked[e]] / 2);
+            t.cap = (uint8_t)caps[e];
+            t.stride = (uint16_t)stride;
+            t.base = stride == 1 ? (uint16_t)entries : 0xffff;
+            stride *= caps[e] + 1;
+        }
+        entries += stride;
     }
+    P->entries = entries;
+    P->sparse = survive * 64 < samples;
+    P->list_words = (groups + 3) / 4 * 4;
+    P->lo = 0;
+    P->hi = 1ull << (n - 1);
     return true;
 }
 
@@ -377,17 +422,10 @@ static int plan_build(const int64_t *A, int n, ExactPlan *P) {
         P->off_out = align_up(P->off_status + 16, 256);
         P->total = align_up(P->off_out + (size_t)(P->NL + 1) * 8, 256);
         P->image.resize(P->total, 0);
-        const int occ = occupancy_binary_any(P->npad, P->G, P->planes, P->words_tracked);
-        uint64_t blocks = 0;
-        int log_len = 0;
-        exact_launch_shape(n - 1, occ, dev.sm_count, &blocks, &P->threads, &log_len);
-        // chunks of 2^10 states (each starts from a closed-form tracker
-        // state) while every thread still gets 16 of them round-robin
-        const uint64_t T = blocks * (uint64_t)P->threads;
-        while (log_len < 10 && ((1ull << (n - 1)) >> (log_len + 1)) >= 16 * T) log_len++;
-        P->chunks.log_len = log_len;
-        P->chunks.chunks = 1ull << (n - 1 - log_len);
-        P->blocks = blocks;
+        // one block per SM: the warps share its tables
+        P->chunks.log_len = BIN_LOW;
+        P->chunks.chunks = 1ull << (n - 1 - BIN_LOW);
+        P->blocks = (uint64_t)dev.sm_count;
         add_block_slots(P);
         return PG_OK;
     }
@@ -459,30 +497,32 @@ static int plan_launch(ExactPlan *P, cudaStream_t stream) {
         BinaryArgs b;
         b.rmask = (const uint64_t *)P->dev;
         b.deg = (const int32_t *)(P->dev + P->off_deg);
-        b.cmask = (const uint64_t *)(P->dev + P->off_cm);
-        b.trmask = (const uint64_t *)(P->dev + P->off_trm);
-        b.toff = (const int32_t *)(P->dev + P->off_toff);
+        b.trk = (const BinTrack *)(P->dev + P->off_trk);
         b.ntracked = P->ntracked;
-        b.n = P->n;
+        b.entries = P->entries;
+        b.list_words = P->list_words;
+        b.sparse = P->sparse;
+        b.warps = P->warps;
         b.acc = (unsigned long long *)(P->dev + P->off_acc);
         b.status = (int *)(P->dev + P->off_status);
         b.part = (unsigned long long *)(P->dev + P->off_part);
-        // the chunk-group counter of the split instantiation shares the
-        // status slot's second 8 bytes
+        // the work counter shares the status slot's second 8 bytes
         b.next = (unsigned long long *)(P->dev + P->off_status + 8);
         b.abort_flag = P->abort_dev;
-        b.chunks = P->chunks.chunks;
-        b.log_len = P->chunks.log_len;
-        b.chunk0 = P->chunk0;
-        b.threads = P->threads;
-        // evaluation from the warp's common high Gray bits: the window must
-        // start on a multiple of 32 chunks
-        const bool split = P->bin_split && (P->chunk0 & 31) == 0 && P->chunks.log_len + 5 <= 31;
-        PG_CUDA(launch_binary_any(P->npad, P->G, P->planes, P->words_tracked, b, split,
-                                  (int)P->blocks, stream));
+        b.state_lo = P->lo;
+        b.state_hi = P->hi;
+        // batches of 32 chunks (one per lane) while every warp gets two of
+        // them, shorter ones below; several batches to a unit on long walks,
+        // so that the counter's atomics stay rare
+        const uint64_t chunks = ((P->hi - P->lo) >> BIN_LOW) + 1;
+        const uint64_t warps = P->blocks * (uint64_t)P->warps;
+        b.log_steps = 5;
+        while (b.log_steps > 2 && (chunks >> b.log_steps) < 2 * warps) b.log_steps--;
+        b.log_unit = 0;
+        while (b.log_unit < 3 && (chunks >> (6 + b.log_unit)) >= 32 * warps) b.log_unit++;
+        PG_CUDA(launch_binary_any(P->npad, P->G, b, (int)P->blocks, stream));
         PG_CUDA(exact_finish(b.part, (int)P->blocks, P->NL, b.acc, b.status,
-                             (unsigned long long *)(P->dev + P->off_out), stream,
-                             split ? b.next : nullptr));
+                             (unsigned long long *)(P->dev + P->off_out), stream, b.next));
         return PG_OK;
     }
     ExactArgs args;
@@ -513,6 +553,8 @@ static int plan_restrict(ExactPlan *P, uint64_t lo, uint64_t hi) {
     const int logu = (P->n - 1) < EXACT_LOGU ? (P->n - 1) : EXACT_LOGU;
     if (ll < logu || ll < 1)
         return fail(PG_EINVAL, "state range bounds must be multiples of 4");
+    P->lo = lo;                  // the 0/1 kernel masks the states of a part-covered chunk
+    P->hi = hi;
     P->chunks.log_len = ll;
     P->chunk0 = lo >> ll;
     P->chunks.chunks = (hi - lo) >> ll;

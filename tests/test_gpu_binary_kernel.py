@@ -111,3 +111,37 @@ def test_zero_rows_permutations_and_ones(lib):
     sparse = _even_rows(40, 4, 4)                        # K = 2, nearly every state zero
     assert _planes(lib, sparse) == 2
     assert _exact(lib, sparse) == _via_general_kernel(lib, sparse)
+
+
+@pytest.mark.parametrize("n,degree", [(24, 6), (40, 20), (48, 24)])
+def test_windows_inside_a_chunk(lib, n, degree):
+    # windows that start and end inside a 1024-state chunk, stay in one, or
+    # cover one exactly, against the general kernel's windows
+    from permgpu import shard
+    a = _even_rows(n, degree, n + degree)
+    assert _planes(lib, a) >= 2
+    b = a.copy()
+    b[0] *= 2
+    top = 1 << (n - 1)
+    for lo, hi in ((4, 8), (1020, 1028), (512, 1024), (2048, 3072), (5 * 1024 + 12, 5 * 1024 + 700),
+                   (3 * 1024 + 4, 40 * 1024 - 4), (top - 1500, top), (top // 2 - 2052, top // 2 + 36)):
+        v = shard.words_value(shard.exact_partial_words(a, lo, hi))
+        w = shard.words_value(shard.exact_partial_words(b, lo, hi))
+        assert 2 * v == w, (lo, hi)
+
+
+def test_whole_chunks_survive(lib):
+    # even rows with ones only in columns beyond the ten low ones: a chunk's
+    # 1024 states survive together and overflow the queue's fast path; and
+    # even rows with ones only in the low columns
+    rng = np.random.default_rng(26)
+    for first in (12, 2):
+        n = 26
+        a = (rng.random((n, n)) < 0.5).astype(np.int64)
+        odd = a.sum(1) % 2 == 0
+        a[odd, 25] ^= 1
+        for i in range(4):
+            a[i] = 0
+            a[i, first + 2 * i: first + 2 * i + 2] = 1
+        assert _planes(lib, a) >= 2
+        assert _exact(lib, a) == _via_general_kernel(lib, a)
