@@ -1,0 +1,369 @@
+// FP64-accurate Glynn permanent with its gradient, real matrices of order
+// 2..32, in one walk.
+//
+//   d per / d a_ij = 2^(1-n) sum_g (-1)^g d_j(g) E_i(g),
+//   E_i(g) = prod_{l != i} s_l(g)                     (no reference counterpart)
+//
+// Row sums are kept on fixed FP32 grids as in the forward kernel
+// (f64_forward.cuh): three additions per row and Gray step, no drift.  P
+// lanes (1, 2 or 4) walk one Gray range together, each with RW = ceil(N / P)
+// rows.  Per state a lane forms the prefix products of its rows, the lanes
+// exchange their products (log2 P shuffles), and a suffix pass that starts
+// from the other lanes' product yields E_i: 3 products per row, no division,
+// so zero row sums need no second path.
+//
+// Gradient columns by a pairwise tree over the Gray range.  With w = (-1)^g
+// E_i(g), two neighbouring blocks A, B of 2^t states have opposite signs of
+// column t, so
+//   sum over both of w       = S_A + S_B,
+//   sum over both of d_t w   = +-(S_A - S_B),
+// and column t takes one double-float addition of the difference per 2^(t+1)
+// states: 3 additions per row and state for the first four columns together
+// (1 + M = 5 when every state adds to each).  Columns 4..R-1 take the
+// 16-state sums, the columns above the range's 2^R states its total.  The
+// tree's waiting sums and the accumulators of columns 1..R-1 live in shared
+// memory ([slot][row][thread]: no bank conflicts).  After each range the warp
+// adds its walkers' sums (shuffles, double-float) and folds them into the
+// warp's FP64 Kahan sums in global memory.
+//
+// FP32-pipe bound: about 46 operations per row and state.  16 x 26x26: 114.4
+// -> 32.2 ms against a lane per row with a shuffle butterfly for the product
+// and a double-float division per row for E_i; error against 64 bits 4.7e-12
+// -> 3.4e-12.
+#pragma once
+
+#include "f64_forward.cuh"
+
+namespace pg {
+
+struct GradArgs {
+    const double *A;           // [batch][n][n] row-major, device
+    int batch;
+    int blocks_per;            // thread blocks per matrix
+    int log_range;             // 2^R states of a walker's range, R <= GradShape::RMAX
+    double *slots;             // [batch][blocks_per][GRAD_WARPS][grad_slot(n)], zeroed
+    volatile const int *abort_flag;
+    int *status;
+};
+
+constexpr int GRAD_WARPS = 4;  // warps of a thread block
+constexpr int GRAD_TREE = 4;   // levels of the pairwise tree
+
+// per-warp slot: sum, sum |term|, then per entry the Kahan sum and its
+// compensation, then the rows' sums of |E|
+__host__ __device__ constexpr int grad_slot(int n) { return 2 + 2 * n * n + n; }
+
+template <int N>
+struct GradShape {
+    static constexpr int LP = N <= 8 ? 0 : N <= 16 ? 1 : 2;    // log2 of a walker's lanes
+    static constexpr int P = 1 << LP, LW = 5 - LP, WK = 1 << LW;
+    static constexpr int RW = (N + P - 1) / P;
+    static constexpr int RP = (RW + 3) & ~3;
+    static constexpr int COL = P * 3 * RP;                     // floats of a column
+    // two blocks of 128 threads per SM: (RMAX + waiting slots) rows of 8
+    // bytes per thread and the table in 113 KB
+    static constexpr int RCAP = RW == 8 ? 8 : 10;
+    static constexpr int RMAX = N - 1 - LW < 0 ? 0 : N - 1 - LW < RCAP ? N - 1 - LW : RCAP;
+    static constexpr int WAIT = LW + 1 > GRAD_TREE - 1 ? LW + 1 : GRAD_TREE - 1;
+    static constexpr int SLOTS = RMAX + WAIT;
+    static constexpr size_t smem =
+        sizeof(float) * (size_t)N * COL + (size_t)SLOTS * RW * 32 * GRAD_WARPS * sizeof(float2);
+};
+
+// sum += f x, f = +-1
+__device__ __forceinline__ void df_accumulate(df &sum, float f, df x) {
+    const float t = fmaf(f, x.hi, sum.hi);
+    const float b = t - sum.hi;
+    sum.lo += (sum.hi - (t - b)) + fmaf(f, x.hi, -b);
+    sum.lo = fmaf(f, x.lo, sum.lo);
+    sum.hi = t;
+}
+// a + f b, unnormalised low word
+__device__ __forceinline__ df df_sum(df a, float f, df b) {
+    df_accumulate(a, f, b);
+    return a;
+}
+
+template <int N>
+__global__ void __launch_bounds__(32 * GRAD_WARPS, 2) glynn_gradient_kernel(GradArgs a) {
+    using S = GradShape<N>;
+    constexpr int P = S::P, RW = S::RW, RP = S::RP, COL = S::COL, WK = S::WK, LW = S::LW;
+    constexpr int BL = fwd_bound_log(false), T = 32 * GRAD_WARPS;
+    extern __shared__ float4 grad_smem[];
+    float *tab = reinterpret_cast<float *>(grad_smem);   // [N][P][3][RP]; column N-1: all-plus sums
+    __shared__ int row_exp[N];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int p = lane & (P - 1), w = lane >> S::LP;
+    // this thread's column of the slots: slot t, row r at [(t RW + r) T]
+    float2 *mine = reinterpret_cast<float2 *>(tab + N * COL) + threadIdx.x;
+    const float2 *warp0 = mine - lane;
+    const int b = blockIdx.x / a.blocks_per, part = blockIdx.x - b * a.blocks_per;
+    const double *A = a.A + (size_t)b * N * N;
+    for (int r = threadIdx.x; r < N; r += T) row_exp[r] = fwd_row_exponent(A + r * N, nullptr, N, BL);
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < N * P * RP; idx += T) {
+        const int j = idx / (P * RP), q = idx - j * (P * RP), lp = q / RP, r = q - lp * RP;
+        float *t = tab + j * COL + lp * 3 * RP + r;
+        const int row = lp * RW + r;
+        if (r < RW && row < N) {
+            fwd_split(ldexp(A[row * N + j], row_exp[row]), BL, t, RP);
+        } else {
+            // rows beyond N: s = 1
+            t[0] = j == N - 1 && r < RW ? 1.f : 0.f;
+            t[RP] = t[2 * RP] = 0.f;
+        }
+    }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < COL; idx += T) {
+        float sum = tab[(N - 1) * COL + idx];
+        for (int j = 0; j < N - 1; j++) {
+            const float v = tab[j * COL + idx];
+            sum += v;
+            tab[j * COL + idx] = 2.f * v;
+        }
+        tab[(N - 1) * COL + idx] = sum;
+    }
+    __syncthreads();
+
+    const int R = a.log_range, M = R < GRAD_TREE ? R : GRAD_TREE;
+    // below 2^LW states (N - 1 < LW) the walkers beyond them are idle
+    const bool active = N - 1 >= LW || w < (1 << (N - 1));
+    const uint64_t states = 1ull << (N - 1);
+    const uint64_t tasks = states >> R >> LW ? states >> R >> LW : 1;
+    double *slot = a.slots + ((size_t)blockIdx.x * GRAD_WARPS + warp) * grad_slot(N);
+    const float *own = tab + p * 3 * RP;
+    double fsum = 0.0, fcomp = 0.0, fabs_sum = 0.0, gabs[RW];
+#pragma unroll
+    for (int r = 0; r < RW; r++) gabs[r] = 0.0;
+    bool aborted = false;
+    const uint64_t first = (uint64_t)part * GRAD_WARPS + warp;
+    for (uint64_t k = first; k < tasks; k += (uint64_t)a.blocks_per * GRAD_WARPS) {
+        if (k != first && *a.abort_flag) { aborted = true; break; }
+        const uint64_t g0 = active ? ((k << LW) + w) << R : 0;
+        float s[3][RW];
+        auto load = [&](const float *col, int c, int v) {
+            return reinterpret_cast<const float4 *>(col + c * RP)[v];
+        };
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+#pragma unroll
+            for (int v = 0; v < RP / 4; v++) {
+                const float4 x = load(own + (N - 1) * COL, c, v);
+                s[c][4 * v] = x.x;
+                if (4 * v + 1 < RW) s[c][4 * v + 1] = x.y;
+                if (4 * v + 2 < RW) s[c][4 * v + 2] = x.z;
+                if (4 * v + 3 < RW) s[c][4 * v + 3] = x.w;
+            }
+        auto step = [&](int j, float f) {
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+#pragma unroll
+                for (int v = 0; v < RP / 4; v++) {
+                    const float4 x = load(own + j * COL, c, v);
+                    s[c][4 * v] = fmaf(f, x.x, s[c][4 * v]);
+                    if (4 * v + 1 < RW) s[c][4 * v + 1] = fmaf(f, x.y, s[c][4 * v + 1]);
+                    if (4 * v + 2 < RW) s[c][4 * v + 2] = fmaf(f, x.z, s[c][4 * v + 2]);
+                    if (4 * v + 3 < RW) s[c][4 * v + 3] = fmaf(f, x.w, s[c][4 * v + 3]);
+                }
+        };
+        const uint64_t gr = g0 ^ (g0 >> 1);
+        for (int j = 0; j < N - 1; j++)
+            if (__any_sync(0xffffffffu, (gr >> j) & 1)) step(j, ((gr >> j) & 1) ? -1.f : 0.f);
+
+        df V0[RW], WT[RW], ft = df{0.f, 0.f};
+        float ga[RW], fa = 0.f;
+#pragma unroll
+        for (int r = 0; r < RW; r++) {
+            V0[r] = WT[r] = df{0.f, 0.f};
+            ga[r] = 0.f;
+        }
+        for (int t = 1; t < R; t++)
+#pragma unroll
+            for (int r = 0; r < RW; r++) mine[(t * RW + r) * T] = make_float2(0.f, 0.f);
+
+        // E[r] of the current state; adds f times the term
+        auto products = [&](df *E, float f) {
+            df x[RW], pre[RW];          // pre[r] = x[0] ... x[r]
+#pragma unroll
+            for (int r = 0; r < RW; r++) {
+                const float h = s[0][r] + s[1][r];
+                x[r] = df{h, (s[1][r] - (h - s[0][r])) + s[2][r]};
+                pre[r] = x[r];
+                if (r > 0) {
+                    pre[r] = pre[r - 1];
+                    df_chain(pre[r], x[r]);
+                }
+            }
+            df full = df_renorm(pre[RW - 1]), q = df{1.f, 0.f};
+            if constexpr (P > 1) {
+                q = df_shfl_xor(full, 1);
+                df_chain(full, q);
+                full = df_renorm(full);
+                if constexpr (P > 2) {
+                    const df o = df_shfl_xor(full, 2);
+                    df_chain(q, o);
+                    q = df_renorm(q);
+                    df_chain(full, o);
+                    full = df_renorm(full);
+                }
+            }
+#pragma unroll
+            for (int r = RW - 1; r > 0; r--) {
+                if (P == 1 && r == RW - 1) {
+                    E[r] = pre[r - 1];
+                    q = x[r];
+                } else {
+                    E[r] = pre[r - 1];
+                    df_chain(E[r], q);
+                    df_chain(q, x[r]);
+                }
+            }
+            E[0] = q;
+            df_accumulate(ft, f, full);
+            fa += fabsf(full.hi);
+#pragma unroll
+            for (int r = 0; r < RW; r++) ga[r] += fabsf(E[r].hi);
+        };
+
+        df Ea[RW];
+        if (R == 0) {
+            const float f = (g0 & 1) ? -1.f : 1.f;
+            products(Ea, f);
+#pragma unroll
+            for (int r = 0; r < RW; r++) df_accumulate(WT[r], f, Ea[r]);
+        }
+        for (uint32_t i = 0; i < (1u << R) >> 1 << 1; i += 2) {
+            const uint64_t g = g0 + i;
+            if (i) {
+                const int j = __ffs(i) - 1;
+                step(j, ((g >> (j + 1)) & 1) ? 1.f : -1.f);
+            }
+            products(Ea, 1.f);
+            step(0, ((g >> 1) & 1) ? 1.f : -1.f);
+            df Eb[RW];
+            products(Eb, -1.f);
+            const float f0 = ((g >> 1) & 1) ? -1.f : 1.f;
+#pragma unroll
+            for (int r = 0; r < RW; r++) {
+                df_accumulate(V0[r], f0, df_sum(Ea[r], 1.f, Eb[r]));
+                Ea[r] = df_sum(Ea[r], -1.f, Eb[r]);
+            }
+            // Ea: the sum of this pair; join it with the waiting sums
+            int t = 1;
+            for (; t < M && ((i >> t) & 1); t++) {
+                const float f = ((g >> (t + 1)) & 1) ? -1.f : 1.f;
+#pragma unroll
+                for (int r = 0; r < RW; r++) {
+                    const float2 hv = mine[((S::RMAX + t - 1) * RW + r) * T];
+                    float2 &vv = mine[(t * RW + r) * T];
+                    const df h = df{hv.x, hv.y};
+                    df v = df{vv.x, vv.y};
+                    df_accumulate(v, f, df_sum(h, -1.f, Ea[r]));
+                    vv = make_float2(v.hi, v.lo);
+                    Ea[r] = df_sum(h, 1.f, Ea[r]);
+                }
+            }
+            if (t < M) {
+#pragma unroll
+                for (int r = 0; r < RW; r++)
+                    mine[((S::RMAX + t - 1) * RW + r) * T] = make_float2(Ea[r].hi, Ea[r].lo);
+            } else {
+#pragma unroll
+                for (int r = 0; r < RW; r++) df_accumulate(WT[r], 1.f, Ea[r]);
+                const uint64_t gm = g ^ (g >> 1);
+                for (t = M; t < R; t++) {
+                    const float f = ((gm >> t) & 1) ? -1.f : 1.f;
+#pragma unroll
+                    for (int r = 0; r < RW; r++) {
+                        float2 &vv = mine[(t * RW + r) * T];
+                        df v = df{vv.x, vv.y};
+                        df_accumulate(v, f, Ea[r]);
+                        vv = make_float2(v.hi, v.lo);
+                    }
+                }
+            }
+        }
+
+        // The walkers' sums, added over the warp; lanes of walker 0 leave
+        // them in their slots: columns 0..R-1, then the total W signed by
+        // each of the LW columns that differ between walkers, then W.
+        if (!active) {
+#pragma unroll
+            for (int r = 0; r < RW; r++) V0[r] = WT[r] = df{0.f, 0.f};
+        }
+        auto total = [&](df v, float f) {
+            v = df{f * v.hi, f * v.lo};
+#pragma unroll
+            for (int o = P; o < 32; o <<= 1) v = df_add(v, df_shfl_xor(v, o));
+            return v;
+        };
+        const uint64_t gw = g0 ^ (g0 >> 1);
+#pragma unroll
+        for (int r = 0; r < RW; r++) {
+            for (int t = 0; t < R + LW + 1; t++) {
+                float2 &vv = mine[((t < R ? t : S::RMAX + t - R) * RW + r) * T];
+                const bool neg = t >= R && t < R + LW && ((gw >> t) & 1);
+                const df v = total(t == 0 && R > 0 ? V0[r] : t < R ? df{vv.x, vv.y} : WT[r],
+                                   neg ? -1.f : 1.f);
+                if (w == 0) vv = make_float2(v.hi, v.lo);
+            }
+        }
+        __syncwarp();
+        const uint64_t gt = (k << LW) << R, gtm = gt ^ (gt >> 1);
+        for (int e = lane; e < N * N; e += 32) {
+            const int i = e / N, j = e - i * N, rr = i % RW, ln = i / RW;
+            const int t = j == N - 1 || j >= R + LW ? S::RMAX + LW : j < R ? j : S::RMAX + j - R;
+            const float2 v = warp0[(t * RW + rr) * T + ln];
+            double x = (double)v.x + (double)v.y;
+            if (j < N - 1 && j >= R + LW && ((gtm >> j) & 1)) x = -x;
+            double sm = slot[2 + e], cp = slot[2 + N * N + e];
+            kahan(sm, cp, x);
+            slot[2 + e] = sm;
+            slot[2 + N * N + e] = cp;
+        }
+        __syncwarp();
+        kahan(fsum, fcomp, active ? df_to(ft) : 0.0);
+        fabs_sum += active ? (double)fa : 0.0;
+#pragma unroll
+        for (int r = 0; r < RW; r++) gabs[r] += active ? (double)ga[r] : 0.0;
+    }
+    fsum -= fcomp;
+#pragma unroll
+    for (int o = P; o < 32; o <<= 1) {
+        fsum += __shfl_xor_sync(0xffffffffu, fsum, o);
+        fabs_sum += __shfl_xor_sync(0xffffffffu, fabs_sum, o);
+#pragma unroll
+        for (int r = 0; r < RW; r++) gabs[r] += __shfl_xor_sync(0xffffffffu, gabs[r], o);
+    }
+    if (lane == 0) {
+        slot[0] = fsum;
+        slot[1] = fabs_sum;
+        if (aborted) atomicExch(a.status, 1);
+    }
+    if (w == 0)
+#pragma unroll
+        for (int r = 0; r < RW; r++)
+            if (p * RW + r < N) slot[2 + 2 * N * N + p * RW + r] = gabs[r];
+}
+
+template <int N>
+cudaError_t launch_glynn_gradient(const GradArgs &a, cudaStream_t s) {
+    constexpr size_t smem = GradShape<N>::smem;
+    if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(glynn_gradient_kernel<N>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    glynn_gradient_kernel<N><<<(unsigned)(a.batch * a.blocks_per), 32 * GRAD_WARPS, smem, s>>>(a);
+    return cudaGetLastError();
+}
+
+// log2 of a warp's walkers and of the longest range at order n
+void gradient_shape(int n, int *log_walkers, int *log_range_max);
+
+// Instantiated in f64_grad_{lo,mid,hi}.cu: orders 2..16, 17..24, 25..32.
+cudaError_t launch_gradient_lo(int n, const GradArgs &a, cudaStream_t s);
+cudaError_t launch_gradient_mid(int n, const GradArgs &a, cudaStream_t s);
+cudaError_t launch_gradient_hi(int n, const GradArgs &a, cudaStream_t s);
+
+}  // namespace pg

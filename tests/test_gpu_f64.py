@@ -279,3 +279,31 @@ def test_windows_at_large_orders(lib, n):
     G = rng.normal(0, 1 / np.sqrt(n), (n, n))
     got, s = glynn_window(G, 0, w)
     assert s > 0 and np.isfinite(got)
+
+
+@pytest.mark.parametrize("n", [6, 7, 9, 10, 12, 14, 15, 16, 18, 21, 22, 23, 25, 26, 32])
+def test_walk_shapes_against_exact_values(lib, n):
+    # every rows-per-lane split of the gradient kernel, walks shorter than a
+    # warp's ranges and longer, batches of 1 and 3: integer-valued matrices
+    # (exact in FP64) against exact permanents and minors, and the complex
+    # D A (rows multiplied by 1, i, -1, -i) against prod(d) per(A)
+    import torch
+    from permgpu.f64 import permanent_c64, permanent_f64
+    rng = np.random.default_rng(1200 + n)
+    batch = 1 if n > 18 else 3
+    A = rng.integers(-2, 3, (batch, n, n)).astype(np.int64)
+    exact = lib.batch_exact(list(A))
+    per, grad, s, gs = permanent_f64(_t(A))
+    fwd, _, sf, _ = permanent_f64(_t(A), want_grad=False)
+    d = np.array([1, 1j, -1, -1j])[rng.integers(0, 4, n)]
+    cplx, sc = permanent_c64(torch.as_tensor(d[:, None] * A.astype(complex)).cuda())
+    for b in range(batch):
+        assert abs(per[b].item() - exact[b]) <= TOL * s[b].item()
+        assert abs(fwd[b].item() - exact[b]) <= TOL * sf[b].item()
+        assert abs(cplx[b].item() - np.prod(d) * exact[b]) <= TOL * sc[b].item()
+        assert abs(s[b].item() - sf[b].item()) <= 1e-5 * s[b].item()
+        assert abs(sc[b].item() - sf[b].item()) <= 1e-5 * sf[b].item()
+        minors = [np.delete(np.delete(A[b], i, 0), j, 1) for i in range(n) for j in range(n)]
+        want = np.array([float(v) for v in lib.batch_exact(minors)]).reshape(n, n)
+        err = np.abs(grad[b].cpu().numpy() - want)
+        assert (err <= TOL * gs[b].cpu().numpy()[:, None]).all(), err.max()
