@@ -45,16 +45,12 @@ __global__ void glynn_forward_reduce(const double *Are, const double *Aim, const
     if (abs_sum) abs_sum[b] = ldexp(as, -e - (n - 1));
 }
 
-// per(A) of `batch` device matrices of order 2..32 (Aim null: real).
-static int glynn_forward_run(const double *Are, const double *Aim, int batch, int n, double *re,
-                             double *im, double *abs_sum, cudaStream_t stream) {
-    DeviceInfo dev;
-    int st = device_info(&dev);
-    if (st != PG_OK) return st;
-    volatile int *abort_dev;
-    st = abort_flag_device(&abort_dev);
-    if (st != PG_OK) return st;
-    FwdArgs a;
+// Launch shape of the forward walk of `batch` matrices of order 2..32 (Aim
+// null: real): fills a.batch, a.log_block, a.blocks_per; returns the slots'
+// bytes.
+static size_t forward_shape(const double *Are, const double *Aim, int batch, int n, int sms,
+                            FwdArgs *out) {
+    FwdArgs &a = *out;
     a.Are = Are;
     a.Aim = Aim;
     a.batch = batch;
@@ -63,17 +59,48 @@ static int glynn_forward_run(const double *Are, const double *Aim, int batch, in
     // waves of warps are busy; complex ones keep the length that fixes the
     // order of their |term| sums
     while (!Aim && a.log_block > 8 &&
-           ((uint64_t)batch << (n - 1 - a.log_block)) < (uint64_t)dev.sm_count * 64)
+           ((uint64_t)batch << (n - 1 - a.log_block)) < (uint64_t)sms * 64)
         a.log_block--;
     // thread blocks: a power of two per matrix, so that every warp takes the
     // same number of blocks of states
     const uint64_t tasks = 1ull << (n - 1 - a.log_block);
     a.blocks_per = 1;
     while ((uint64_t)a.blocks_per * FWD_WARPS < tasks &&
-           (uint64_t)batch * a.blocks_per * 2 <= (uint64_t)dev.sm_count * 64)
+           (uint64_t)batch * a.blocks_per * 2 <= (uint64_t)sms * 64)
         a.blocks_per *= 2;
-    const size_t warps = (size_t)a.blocks_per * FWD_WARPS;
-    const size_t bytes = (size_t)batch * warps * FWD_SLOT * sizeof(double) + 256;
+    return (size_t)batch * a.blocks_per * FWD_WARPS * FWD_SLOT * sizeof(double);
+}
+
+// The walk and its reduction, asynchronous on s.
+static int forward_launch(const FwdArgs &a, int n, double *re, double *im, double *abs_sum,
+                          cudaStream_t s) {
+    PG_CUDA(!a.Aim ? launch_forward_real(n, a, s)
+            : n <= 22 ? launch_forward_cplx_lo(n, a, s) : launch_forward_cplx_hi(n, a, s));
+    glynn_forward_reduce<<<a.batch, 32, 0, s>>>(a.Are, a.Aim, a.slots, n, a.blocks_per * FWD_WARPS,
+                                                re, im, abs_sum);
+    PG_CUDA(cudaGetLastError());
+    return PG_OK;
+}
+
+static int f64_finish(const int *status, cudaStream_t s) {
+    int hstatus = 0;
+    PG_CUDA(cudaMemcpyAsync(&hstatus, status, sizeof(int), cudaMemcpyDeviceToHost, s));
+    PG_CUDA(cudaStreamSynchronize(s));
+    if (hstatus) return fail(PG_EABORT, "FP64 launch aborted by pg_abort()");
+    return PG_OK;
+}
+
+// per(A) of `batch` device matrices of order 2..32 (Aim null: real).
+static int glynn_forward_run(const double *Are, const double *Aim, int batch, int n, double *re,
+                             double *im, double *abs_sum, cudaStream_t stream) {
+    DeviceInfo dev;
+    int st = device_info(&dev);
+    if (st != PG_OK) return st;
+    FwdArgs a;
+    volatile int *abort_dev;
+    st = abort_flag_device(&abort_dev);
+    if (st != PG_OK) return st;
+    const size_t bytes = forward_shape(Are, Aim, batch, n, dev.sm_count, &a) + 256;
     Workspace *ws;
     st = workspace(&ws, bytes, 64);
     if (st != PG_OK) return st;
@@ -82,49 +109,30 @@ static int glynn_forward_run(const double *Are, const double *Aim, int batch, in
     a.slots = (double *)((char *)ws->dev + 256);
     a.abort_flag = abort_dev;
     PG_CUDA(cudaMemsetAsync(a.status, 0, sizeof(int), s));
-    PG_CUDA(!Aim ? launch_forward_real(n, a, s)
-            : n <= 22 ? launch_forward_cplx_lo(n, a, s) : launch_forward_cplx_hi(n, a, s));
-    glynn_forward_reduce<<<batch, 32, 0, s>>>(Are, Aim, a.slots, n, (int)warps, re, im, abs_sum);
-    PG_CUDA(cudaGetLastError());
-    int hstatus = 0;
-    PG_CUDA(cudaMemcpyAsync(&hstatus, a.status, sizeof(int), cudaMemcpyDeviceToHost, s));
-    PG_CUDA(cudaStreamSynchronize(s));
-    if (hstatus) return fail(PG_EABORT, "FP64 launch aborted by pg_abort()");
-    return PG_OK;
+    if ((st = forward_launch(a, n, re, im, abs_sum, s)) != PG_OK) return st;
+    return f64_finish(a.status, s);
 }
 
 // One block per matrix and gradient row: warp v adds the slots v, v + 8, ...
 // (lane = column), the first warp adds the eight sums; all in a fixed order.
-// Row 0's block also reduces the permanent.
 __global__ void __launch_bounds__(256) glynn_gradient_reduce(
-    const double *A, const double *slots, int n, int per_matrix, double *per, double *grad,
-    double *abs_sum, double *grad_abs) {
+    const double *A, const double *slots, int n, int per_matrix, double *grad, double *grad_abs) {
     const int b = blockIdx.x, i = blockIdx.y, lane = threadIdx.x & 31, v = threadIdx.x >> 5;
     const int sd = grad_slot(n);
     const double *base = slots + (size_t)b * per_matrix * sd;
-    __shared__ double part[8][32], extra[8][3];
+    __shared__ double part[8][32], rows[8];
     __shared__ int ex[32];
-    double s = 0, c = 0, as = 0, ps = 0, pc = 0, pa = 0;
+    double s = 0, c = 0, as = 0;
     for (int w = v; w < per_matrix; w += 8) {
         const double *sl = base + (size_t)w * sd;
         if (lane < n) {
-            kahan(s, c, sl[2 + i * n + lane]);
-            kahan(s, c, -sl[2 + n * n + i * n + lane]);
+            kahan(s, c, sl[i * n + lane]);
+            kahan(s, c, -sl[n * n + i * n + lane]);
         }
-        if (lane == 0) {
-            as += sl[2 + 2 * n * n + i];
-            if (i == 0) {
-                kahan(ps, pc, sl[0]);
-                pa += sl[1];
-            }
-        }
+        if (lane == 0) as += sl[2 * n * n + i];
     }
     part[v][lane] = s - c;
-    if (lane == 0) {
-        extra[v][0] = as;
-        extra[v][1] = ps - pc;
-        extra[v][2] = pa;
-    }
+    if (lane == 0) rows[v] = as;
     if (threadIdx.x < 32)
         ex[lane] = lane < n ? fwd_row_exponent(A + ((size_t)b * n + lane) * n, nullptr, n,
                                                fwd_bound_log(false)) : 0;
@@ -137,20 +145,14 @@ __global__ void __launch_bounds__(256) glynn_gradient_reduce(
     double g = 0, gc = 0;
     for (int u = 0; u < 8; u++) kahan(g, gc, part[u][lane]);
     if (lane < n) grad[((size_t)b * n + i) * n + lane] = ldexp(g - gc, shift);
-    if (lane != 0) return;
-    double t = 0, tc = 0, ta = 0, tg = 0;
-    for (int u = 0; u < 8; u++) {
-        tg += extra[u][0];
-        kahan(t, tc, extra[u][1]);
-        ta += extra[u][2];
-    }
-    if (grad_abs) grad_abs[(size_t)b * n + i] = ldexp(tg, shift);
-    if (i == 0) {
-        per[b] = ldexp(t - tc, -total - (n - 1));
-        if (abs_sum) abs_sum[b] = ldexp(ta, -total - (n - 1));
-    }
+    if (lane != 0 || !grad_abs) return;
+    double tg = 0;
+    for (int u = 0; u < 8; u++) tg += rows[u];
+    grad_abs[(size_t)b * n + i] = ldexp(tg, shift);
 }
 
+// The permanents come from the forward walk, so that they do not depend on
+// whether the gradient is asked for (a tenth of the gradient's time).
 static int glynn_gradient_run(const double *A, int batch, int n, double *per, double *grad,
                               double *abs_sum, double *grad_abs, cudaStream_t stream) {
     DeviceInfo dev;
@@ -188,24 +190,23 @@ static int glynn_gradient_run(const double *A, int batch, int n, double *per, do
     }
     const size_t warps = (size_t)a.blocks_per * GRAD_WARPS;
     const size_t bytes = (size_t)batch * warps * grad_slot(n) * sizeof(double) + 256;
+    FwdArgs f;
+    const size_t fwd_bytes = forward_shape(A, nullptr, batch, n, dev.sm_count, &f);
     Workspace *ws;
-    st = workspace(&ws, bytes, 64);
+    st = workspace(&ws, bytes + fwd_bytes, 64);
     if (st != PG_OK) return st;
     cudaStream_t s = stream ? stream : ws->stream;
-    a.status = (int *)ws->dev;
+    a.status = f.status = (int *)ws->dev;
     a.slots = (double *)((char *)ws->dev + 256);
-    a.abort_flag = abort_dev;
+    f.slots = (double *)((char *)ws->dev + bytes);
+    a.abort_flag = f.abort_flag = abort_dev;
     PG_CUDA(cudaMemsetAsync(ws->dev, 0, bytes, s));
+    if ((st = forward_launch(f, n, per, nullptr, abs_sum, s)) != PG_OK) return st;
     PG_CUDA(n <= 16 ? launch_gradient_lo(n, a, s)
             : n <= 24 ? launch_gradient_mid(n, a, s) : launch_gradient_hi(n, a, s));
-    glynn_gradient_reduce<<<dim3(batch, n), 256, 0, s>>>(A, a.slots, n, (int)warps, per, grad,
-                                                         abs_sum, grad_abs);
+    glynn_gradient_reduce<<<dim3(batch, n), 256, 0, s>>>(A, a.slots, n, (int)warps, grad, grad_abs);
     PG_CUDA(cudaGetLastError());
-    int hstatus = 0;
-    PG_CUDA(cudaMemcpyAsync(&hstatus, a.status, sizeof(int), cudaMemcpyDeviceToHost, s));
-    PG_CUDA(cudaStreamSynchronize(s));
-    if (hstatus) return fail(PG_EABORT, "FP64 launch aborted by pg_abort()");
-    return PG_OK;
+    return f64_finish(a.status, s);
 }
 
 }  // namespace pg
