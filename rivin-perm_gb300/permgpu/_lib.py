@@ -308,13 +308,35 @@ def binary_residues(matrix: np.ndarray, primes) -> list[int]:
 
 def limbs_to_int(words: np.ndarray) -> int:
     """Two's-complement little-endian uint32 words -> Python int."""
-    v = 0
-    for i, w in enumerate(words.tolist()):
-        v |= int(w) << (32 * i)
-    bits = 32 * len(words)
-    if v >> (bits - 1):
-        v -= 1 << bits
-    return v
+    return int.from_bytes(np.asarray(words, dtype="<u4").tobytes(), "little", signed=True)
+
+
+def int64_matrix(matrix):
+    """The int64 array of a square matrix given as a list of rows of plain
+    ints or as a signed integer array; None for anything else (other types,
+    entries beyond int64, ragged rows), which needs entry-by-entry checks."""
+    if type(matrix) is np.ndarray:
+        if matrix.ndim != 2 or matrix.shape[0] != matrix.shape[1] or matrix.dtype.kind != "i":
+            return None
+        return np.ascontiguousarray(matrix, dtype=np.int64)
+    if type(matrix) not in (list, tuple):
+        return None
+    n = len(matrix)
+    for row in matrix:
+        if type(row) not in (list, tuple) or len(row) != n or set(map(type, row)) != {int}:
+            return None
+    try:
+        return np.array(matrix, dtype=np.int64).reshape(n, n)
+    except OverflowError:
+        return None
+
+
+def row_bounds_fit(largest: float, n: int) -> bool:
+    """True when every row-sum bound being at most ``largest`` is enough for
+    the exact engine at order n: the smallest compiled row groups (1 row to
+    order 16, 2 to 32, 3 to 48) then stay below 2^30.  The native check also
+    knows larger groups; it decides the other matrices."""
+    return n <= 48 and largest < (1 << 30 if n <= 16 else 1 << 15 if n <= 32 else 1 << 10)
 
 
 def exact_supported(matrix: np.ndarray) -> bool:
@@ -324,9 +346,11 @@ def exact_supported(matrix: np.ndarray) -> bool:
 
 def exact_limbs(matrix: np.ndarray) -> int:
     """Output words that hold any value within the row-sum bound."""
-    bits = 0.0
-    for row in np.abs(np.asarray(matrix, dtype=np.float64)):
-        bits += float(np.log2(max(1.0, float(row.sum()))))
+    sums = np.abs(np.asarray(matrix, dtype=np.float64)).sum(axis=-1)
+    return _limbs_of_bits(float(np.log2(np.maximum(1.0, sums)).sum()))
+
+
+def _limbs_of_bits(bits: float) -> int:
     return int(bits + 2) // 32 + 2
 
 
@@ -381,21 +405,37 @@ class ExactPlan:
 def pack_batch(matrices):
     """(A_packed int64, offsets int64, orders int32) for a list of square
     integer matrices."""
-    orders = np.array([np.asarray(m).shape[0] if np.asarray(m).ndim == 2 else 0
-                       for m in matrices], dtype=np.int32)
+    mats = [np.asarray(m, dtype=np.int64) for m in matrices]
+    orders = np.array([m.shape[0] if m.ndim == 2 else 0 for m in mats], dtype=np.int32)
     sizes = orders.astype(np.int64) ** 2
-    offsets = np.zeros(len(matrices), dtype=np.int64)
-    if len(matrices) > 1:
+    offsets = np.zeros(len(mats), dtype=np.int64)
+    if len(mats) > 1:
         offsets[1:] = np.cumsum(sizes)[:-1]
-    packed = np.zeros(int(sizes.sum()) or 1, dtype=np.int64)
-    for m, off, sz in zip(matrices, offsets, sizes):
-        if sz:
-            packed[off:off + sz] = np.asarray(m, dtype=np.int64).reshape(-1)
-    return packed, offsets, orders
+    flat = [m.reshape(-1) for m, sz in zip(mats, sizes) if sz]
+    return (np.concatenate(flat) if flat else np.zeros(1, dtype=np.int64)), offsets, orders
 
 
-def batch_limbs(matrices) -> int:
-    return max([exact_limbs(np.asarray(m)) for m in matrices if np.asarray(m).size] or [2])
+def batch_row_sums(packed: np.ndarray, orders: np.ndarray):
+    """(row sums of |a_ij| of every packed matrix in turn, first row of each
+    matrix of order >= 1)."""
+    widths = np.repeat(orders, orders).astype(np.int64)
+    if not widths.size:
+        return np.zeros(0), np.zeros(0, dtype=np.int64)
+    starts = np.concatenate(([0], np.cumsum(widths)[:-1]))
+    sums = np.add.reduceat(np.abs(packed.astype(np.float64)), starts)
+    rows = orders[orders > 0].astype(np.int64)
+    return sums, np.concatenate(([0], np.cumsum(rows)[:-1]))
+
+
+def batch_limbs(matrices, packed=None) -> int:
+    """Output words that hold any matrix's permanent; ``packed``: the
+    matrices' pack_batch, if at hand."""
+    packed, _, orders = packed or pack_batch(matrices)
+    sums, first = batch_row_sums(packed, orders)
+    if not first.size:
+        return 2
+    bits = np.add.reduceat(np.log2(np.maximum(1.0, sums)), first)
+    return _limbs_of_bits(float(bits.max()))
 
 
 class BatchPlan:
@@ -405,8 +445,8 @@ class BatchPlan:
 
     def __init__(self, matrices, tune: tuple | None = None):
         self.count = len(matrices)
-        self.limbs = batch_limbs(matrices)
         packed, offsets, orders = pack_batch(matrices)
+        self.limbs = batch_limbs(matrices, (packed, offsets, orders))
         self.orders = orders
         t = BatchTune(*(tune or (0, 0, 0)))
         h = ctypes.c_void_p()
@@ -442,8 +482,8 @@ class BatchPlan:
 
 def batch_exact(matrices) -> list[int]:
     """One-shot host-to-host batched evaluation (pg_batch_exact)."""
-    limbs = batch_limbs(matrices)
     packed, offsets, orders = pack_batch(matrices)
+    limbs = batch_limbs(matrices, (packed, offsets, orders))
     out = np.zeros(len(matrices) * limbs, dtype=np.uint32)
     check(load().pg_batch_exact(ptr(packed, ctypes.c_int64), ptr(offsets, ctypes.c_int64),
                                 ptr(orders, ctypes.c_int32), len(matrices),

@@ -39,7 +39,13 @@ def batch_permanents(matrices: Sequence, tune="auto", cache_path=None) -> List[i
     """
     mats = [np.asarray(m, dtype=np.int64).reshape(len(m), len(m)) if len(m) else
             np.zeros((0, 0), np.int64) for m in matrices]
-    ok = [i for i, m in enumerate(mats) if _exact_ok(m)]
+    packed, _, orders = _lib.pack_batch(mats)
+    sums, first = _lib.batch_row_sums(packed, orders)
+    top = np.zeros(len(mats))
+    if first.size:
+        top[orders > 0] = np.maximum.reduceat(sums, first)
+    ok = [i for i, m in enumerate(mats)
+          if _lib.row_bounds_fit(top[i], int(orders[i])) or _exact_ok(m)]
     out: List[int] = [0] * len(mats)
     if ok:
         sub = [mats[i] for i in ok]

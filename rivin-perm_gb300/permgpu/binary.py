@@ -44,6 +44,9 @@ def normalize_binary_matrix(matrix, *, strict: bool = True) -> Tuple[Tuple[int, 
             raise TypeError("matrix rows must be sequences") from exc
         if width != n:
             raise ValueError("matrix must be square")
+        if type(row) in (list, tuple) and set(map(type, row)) == {int} and set(row) <= {0, 1}:
+            rows.append(tuple(row))
+            continue
         out = []
         for j, entry in enumerate(row):
             if isinstance(entry, (bool, np.bool_)):

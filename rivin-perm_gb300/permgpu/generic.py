@@ -71,7 +71,8 @@ def matrix_permanent(matrix, verbose: bool = False, parallel: bool = True,
     engine, so 'low_rank' raises).  ``engine`` selects 'auto', 'exact' or
     'residue' for testing either GPU path directly.
     """
-    n = _validate_integer_matrix(matrix)
+    arr = _lib.int64_matrix(matrix)
+    n = _validate_integer_matrix(matrix) if arr is None else len(arr)
     _validate_threads(num_threads)
     if not isinstance(method, str):
         raise TypeError("method must be a string")
@@ -86,13 +87,18 @@ def matrix_permanent(matrix, verbose: bool = False, parallel: bool = True,
         return 1
     if n == 1:
         return int(matrix[0][0])
-    rows = [[int(x) for x in row] for row in matrix]
-    fits_int64 = all(-(1 << 63) <= x < (1 << 63) for row in rows for x in row)
-    arr = np.array(rows, dtype=np.int64) if fits_int64 else None
-    if engine != "residue" and arr is not None and _lib.exact_supported(arr):
-        if verbose:
-            print(f"exact GPU engine, order {n}")
-        return _lib.exact_permanent(arr, _lib.exact_limbs(arr))
+    if arr is None:
+        rows = [[int(x) for x in row] for row in matrix]
+        if all(-(1 << 63) <= x < (1 << 63) for row in rows for x in row):
+            arr = np.array(rows, dtype=np.int64)
+    else:
+        rows = arr.tolist()
+    if engine != "residue" and arr is not None:
+        top = float(np.abs(arr.astype(np.float64)).sum(axis=1).max())
+        if _lib.row_bounds_fit(top, n) or _lib.exact_supported(arr):
+            if verbose:
+                print(f"exact GPU engine, order {n}")
+            return _lib.exact_permanent(arr, _lib.exact_limbs(arr))
     if engine == "exact":
         raise ValueError("matrix is outside the exact engine's range")
     bound = matrix_permanent_bound(rows)

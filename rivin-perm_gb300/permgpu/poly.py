@@ -109,6 +109,9 @@ def _snapshot_integer_matrix(matrix, name: str) -> Matrix:
             raise TypeError(f"{name} rows must be sequences") from exc
         if width != order:
             raise ValueError(f"{name} must be square")
+        if type(row) in (list, tuple) and set(map(type, row)) == {int}:
+            rows.append(tuple(row))
+            continue
         out = []
         for j, entry in enumerate(row):
             try:
@@ -172,15 +175,12 @@ def _bounds(c: Matrix, l: Matrix) -> Tuple[int, ...]:
     n = len(c)
     if n == 0:
         return (1,)
-    cols = range(n)
-    rc = [sum(abs(v) for v in row) for row in c]
-    rl = [sum(abs(v) for v in row) for row in l]
-    cc = [sum(abs(c[i][j]) for i in cols) for j in cols]
-    cl = [sum(abs(l[i][j]) for i in cols) for j in cols]
-    mc = [max(abs(v) for v in row) for row in c]
-    ml = [max(abs(v) for v in row) for row in l]
-    kc = [max(abs(c[i][j]) for i in cols) for j in cols]
-    kl = [max(abs(l[i][j]) for i in cols) for j in cols]
+    c = [list(map(abs, row)) for row in c]
+    l = [list(map(abs, row)) for row in l]
+    rc, mc = list(map(sum, c)), list(map(max, c))
+    rl, ml = list(map(sum, l)), list(map(max, l))
+    cc, kc = list(map(sum, zip(*c))), list(map(max, zip(*c)))
+    cl, kl = list(map(sum, zip(*l))), list(map(max, zip(*l)))
     f = math.factorial(n)
     cands = (_affine_product(rc, rl), _affine_product(cc, cl),
              [f * v for v in _affine_product(mc, ml)], [f * v for v in _affine_product(kc, kl)])
@@ -210,7 +210,7 @@ def _gpu_primes(target: int) -> List[int]:
 
 
 def _fits_int64(m: Matrix) -> bool:
-    return all(-(1 << 63) <= v <= _INT64_MAX for row in m for v in row)
+    return all(-(1 << 63) <= min(row) and max(row) <= _INT64_MAX for row in m)
 
 
 def _residues(c: Matrix, l: Matrix, moduli: Sequence[int]) -> List[List[int]]:
@@ -238,7 +238,7 @@ def _exact(c: Matrix, l: Matrix) -> Tuple[int, ...]:
     top = max(bounds)
     if top == 0:
         return (0,) * (n + 1)
-    nonneg = all(v >= 0 for m in (c, l) for row in m for v in row)
+    nonneg = all(min(row) >= 0 for m in (c, l) for row in m)
     primes = _gpu_primes(top if nonneg else 2 * top)
     res = _residues(c, l, primes)
     vals, mod = list(res[0]), primes[0]
