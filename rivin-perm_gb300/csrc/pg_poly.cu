@@ -22,6 +22,7 @@
 #include "pg_internal.h"
 #include "glynn_m32.cuh"
 #include "poly_common.cuh"
+#include "poly_esym.cuh"
 
 // 1: matrices C with equal rows (rook polynomials) take the uniform kernel.
 #ifndef PG_POLY_UNIFORM
@@ -302,12 +303,141 @@ static int uniform_residues_impl(const int64_t *C, const int64_t *L, int n,
     return PG_OK;
 }
 
+// The exact kernel (poly_esym.cuh) takes constant C and row sums of |L| up
+// to 31 at orders 14..31; below, both kernels are launch-bound.  Its cost
+// does not depend on the number of moduli (order 25: 1.3 ms, the modular
+// kernel about 2 ms for each).
+static bool esym_shape(const int64_t *C, const int64_t *L, int n, EsymEntry *out) {
+    if (n < ESYM_MIN_N || n > ESYM_MAX_N) return false;
+    for (int i = 1; i < n * n; i++)
+        if (C[i] != C[0]) return false;
+    int64_t top = 0;
+    for (int i = 0; i < n; i++) {
+        int64_t sum = 0;
+        for (int j = 0; j < n; j++) {
+            const int64_t v = L[(size_t)i * n + j];
+            if (v > ESYM_MAX_L || v < -ESYM_MAX_L) return false;
+            sum += v < 0 ? -v : v;
+        }
+        top = std::max(top, sum);
+    }
+    if (top <= 15) return esym_entry_15(n, out);
+    if (top <= 20) return esym_entry_20(n, out);
+    return top <= ESYM_MAX_L && esym_entry_31(n, out);
+}
+
+// sets of k of the columns 0..n-1 in revolving-door order (neighbours differ
+// by one exchange), appended to out with the columns in `with`
+static void revolving_door(int n, int k, bool back, uint8_t with, std::vector<uint8_t> *out) {
+    if (k == 0 || k == n) {
+        out->push_back((uint8_t)(with | ((1u << k) - 1)));
+        return;
+    }
+    const uint8_t top = (uint8_t)(with | (1u << (n - 1)));
+    if (back) {
+        revolving_door(n - 1, k - 1, false, top, out);
+        revolving_door(n - 1, k, true, with, out);
+    } else {
+        revolving_door(n - 1, k, false, with, out);
+        revolving_door(n - 1, k - 1, true, top, out);
+    }
+}
+
+static int esym_residues_impl(const EsymEntry &entry, int64_t gamma, const int64_t *L, int n,
+                              const uint64_t *moduli, int k, uint64_t *out) {
+    const EsymLayout &S = entry.layout;
+    DeviceInfo dev;
+    int st = device_info(&dev);
+    if (st != PG_OK) return st;
+    volatile int *abort_dev;
+    st = abort_flag_device(&abort_dev);
+    if (st != PG_OK) return st;
+    const int high = n - 1 - ESYM_LOW;
+    const size_t off_init = poly_align((size_t)(n - 1) * S.words * 4);
+    const size_t off_binom = poly_align(off_init + (size_t)S.words * 4);
+    const size_t off_first = poly_align(off_binom + 32 * 32 * 4);
+    const size_t off_sets = poly_align(off_first + 32 * 4);
+    const size_t off_bins = poly_align(off_sets + 64);
+    const size_t off_status = poly_align(off_bins + (size_t)n * S.sums * 8);
+    const size_t total = poly_align(off_status + 16);
+    Workspace *ws;
+    st = workspace(&ws, total, total);
+    if (st != PG_OK) return st;
+    char *h = (char *)ws->host;
+    char *d = (char *)ws->dev;
+    std::memset(h, 0, off_bins);
+    uint32_t *cols = (uint32_t *)h, *init = (uint32_t *)(h + off_init);
+    uint32_t *binom = (uint32_t *)(h + off_binom), *first = (uint32_t *)(h + off_first);
+    for (int i = 0; i < n; i++) {
+        int64_t sum = 128;
+        for (int j = 0; j < n; j++) {
+            const int64_t v = L[(size_t)i * n + j];
+            sum += v;
+            if (j < n - 1) cols[j * S.words + i / 4] += (uint32_t)(2 * v) << (8 * (i & 3));
+        }
+        init[i / 4] += (uint32_t)sum << (8 * (i & 3));
+    }
+    for (int i = n; i < 4 * ((n + 3) / 4); i++) init[i / 4] += 128u << (8 * (i & 3));
+    for (int i = 0; i < 32; i++)
+        for (int q = 0; q <= i; q++)
+            binom[i * 32 + q] = q == 0 || q == i ? 1 : binom[(i - 1) * 32 + q - 1] + binom[(i - 1) * 32 + q];
+    for (int p = 0; p <= high; p++) first[p + 1] = first[p] + (binom[high * 32 + p] + 31) / 32;
+    std::vector<uint8_t> sets;
+    for (int w = 0; w <= ESYM_LOW; w++) revolving_door(ESYM_LOW, w, false, 0, &sets);
+    std::memcpy(h + off_sets, sets.data(), sets.size());
+    EsymArgs a;
+    a.cols = (const uint32_t *)d;
+    a.init = (const uint32_t *)(d + off_init);
+    a.binom = (const uint32_t *)(d + off_binom);
+    a.first = (const uint32_t *)(d + off_first);
+    a.sets = (const uint8_t *)(d + off_sets);
+    a.n = n;
+    a.high = high;
+    a.bins = (long long *)(d + off_bins);
+    a.status = (int *)(d + off_status);
+    a.abort_flag = abort_dev;
+    PG_CUDA(cudaMemcpyAsync(d, h, off_bins, cudaMemcpyHostToDevice, ws->stream));
+    PG_CUDA(cudaMemsetAsync(d + off_bins, 0, total - off_bins, ws->stream));
+    PG_CUDA(entry.launch(a, dev.sm_count, first[high + 1], ws->stream));
+    PG_CUDA(cudaMemcpyAsync(h + off_bins, d + off_bins, total - off_bins, cudaMemcpyDeviceToHost,
+                            ws->stream));
+    PG_CUDA(cudaStreamSynchronize(ws->stream));
+    if (*(int *)(h + off_status)) return fail(PG_EABORT, "launch aborted by pg_abort()");
+    const long long *bins = (const long long *)(h + off_bins);
+    for (int t = 0; t < k; t++) {
+        const int64_t p = (int64_t)moduli[t];
+        uint64_t *o = out + (size_t)t * (n + 1);
+        std::vector<int64_t> pow2(10, 1 % p);              // 2^(26 j) mod p
+        for (int j = 1; j < 10; j++) pow2[j] = (int64_t)(((uint64_t)pow2[j - 1] << ESYM_RADIX) % (uint64_t)p);
+        const int64_t half = (int64_t)powmod_u64((uint64_t)(p >> 1) + 1, (uint64_t)(n - 1), (uint64_t)p);
+        const int64_t g = (int64_t)normmod_i64(gamma, (uint64_t)p);
+        std::vector<int64_t> coef(n + 1, 0);
+        for (int m = 0; m < n; m++) {
+            const int64_t c = g * (int64_t)normmod_i64(n - 2 * m, (uint64_t)p) % p;
+            int64_t w = (m & 1) ? (p - half) % p : half;   // (-1)^m c^(n - kk) 2^(1-n)
+            for (int kk = n; kk >= 0; kk--, w = w * c % p) {
+                // T[m][0] counts the sign vectors with m minus signs
+                int64_t v = kk == 0 ? binom[(n - 1) * 32 + m] % p : 0;
+                for (int j = 0; kk > 0 && j < S.digits[kk]; j++)
+                    v += bins[(size_t)m * S.sums + S.sum_off[kk] + j] % p * pow2[j] % p;
+                v %= p;
+                if (v < 0) v += p;
+                coef[kk] = (coef[kk] + v * w) % p;
+            }
+        }
+        for (int kk = 0; kk <= n; kk++) o[kk] = (uint64_t)coef[kk];
+    }
+    return PG_OK;
+}
+
 // out[t*(n+1) + d] = coefficient d of per(C + x L) mod moduli[t], 2 <= n <= 63
 // (orders above 32 in pg_poly_wide.cu), odd moduli 3 <= m < 2^30, k <= 65535.
 static int affine_residues_impl(const int64_t *C, const int64_t *L, int n,
                                 const uint64_t *moduli, int k, uint64_t *out) {
     if (n > POLY_REG_MAX_N)
         return affine_wide_residues(C, L, n, 0, 1ull << (n - 1), true, moduli, k, out);
+    EsymEntry esym;
+    if (esym_shape(C, L, n, &esym)) return esym_residues_impl(esym, C[0], L, n, moduli, k, out);
 #if PG_POLY_UNIFORM
     if (rows_equal(C, n)) return uniform_residues_impl(C, L, n, moduli, k, out);
 #endif

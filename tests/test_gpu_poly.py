@@ -156,3 +156,49 @@ def test_rook_polynomial_order_34_whole_walk(lib):
         m = np.ones((n, n), dtype=np.int64) + t * a
         want = lib.exact_permanent(m, lib.exact_limbs(m))
         assert sum(rk * math.factorial(n - k) * t ** k for k, rk in enumerate(r)) == want
+
+
+def _small_rows(rng, n, top):
+    # integer rows with sum |a_ij| <= top, one row exactly at top
+    a = np.zeros((n, n), dtype=np.int64)
+    for i in range(n):
+        left = top if i == 1 else int(rng.integers(top // 2, top + 1))
+        while left:
+            v = int(rng.integers(1, min(left, 3) + 1))
+            a[i, rng.integers(0, n)] += v if i % 2 else -v
+            left -= v
+        a[i, rng.integers(0, n)] = 0
+    a[1] = 0
+    a[1, : min(n, top)] = 1
+    a[1, 0] += top - int(np.abs(a[1]).sum())
+    return a
+
+
+@pytest.mark.parametrize("top", [15, 20, 31])
+@pytest.mark.parametrize("n", [14, 15, 16, 17])
+def test_exact_symmetric_sums_vs_oracle(lib, n, top):
+    # constant C and small row sums: the exact kernel, every row-sum class,
+    # signed entries, prime and composite moduli from 3 to 2^30
+    rng = np.random.default_rng(100 * n + top)
+    L = _small_rows(rng, n, top)
+    moduli = [3, 1_000_003, 999_999_937, (1 << 30) - 35, 1_000_005]
+    for gamma in (1, -7):
+        C = np.full((n, n), gamma, dtype=np.int64)
+        got = lib.affine_residues(C, L, moduli)
+        for m, r in zip(moduli, got):
+            assert r == oracle.affine_mod_p(C, L, m)
+
+
+@pytest.mark.parametrize("n,top", [(20, 20), (21, 15), (25, 20), (25, 31), (28, 20), (29, 15),
+                                   (31, 31)])
+def test_exact_symmetric_sums_against_exact_permanents(lib, n, top):
+    # the polynomial at x = 1, -1, 2 against the exact engine's permanent of
+    # the matrix gamma + x a_ij
+    rng = np.random.default_rng(10 * n + top)
+    L = _small_rows(rng, n, top)
+    m = (1 << 30) - 35
+    coef = lib.affine_residues(np.full((n, n), 3, dtype=np.int64), L, [m])[0]
+    for x in (1, -1, 2):
+        a = 3 + x * L
+        want = lib.exact_permanent(a, lib.exact_limbs(a)) % m
+        assert sum(c * pow(x, d, m) for d, c in enumerate(coef)) % m == want
