@@ -305,8 +305,9 @@ static int uniform_residues_impl(const int64_t *C, const int64_t *L, int n,
 
 // The exact kernel (poly_esym.cuh) takes constant C and row sums of |L| up
 // to 31 at orders 14..31; below, both kernels are launch-bound.  Its cost
-// does not depend on the number of moduli (order 25: 1.3 ms, the modular
-// kernel about 2 ms for each).
+// hardly depends on the number of moduli (one / five moduli, whole call, at
+// order 14: 109 / 134 us against 178 / 199 with the modular kernel, 20: 168 /
+// 216 against 218 / 438, 25: 1.87 / 1.96 ms against 2.63 / 13.7).
 static bool esym_shape(const int64_t *C, const int64_t *L, int n, EsymEntry *out) {
     if (n < ESYM_MIN_N || n > ESYM_MAX_N) return false;
     for (int i = 1; i < n * n; i++)
