@@ -60,6 +60,23 @@ struct ChunkPlan {
 };
 ChunkPlan plan_chunks(int log_states, int min_log_len, uint64_t target_chunks);
 
+// Blocks per modulus of a launch that gives every one of k moduli the same
+// number of blocks, with equal work in every block and `slots` blocks
+// resident: the number whose whole waves waste least.  Rounding slots / k up
+// instead starts a second, nearly empty wave (476 blocks in 456 slots for 34
+// moduli: 24 x 24 3.23 -> 2.70 ms, 26 x 26 13.3 -> 10.5 ms).
+static inline uint64_t blocks_per_modulus(uint64_t slots, int k) {
+    uint64_t best = 1, best_waves = ((uint64_t)k + slots - 1) / slots;
+    for (uint64_t waves = 1; waves <= 4; waves++) {
+        const uint64_t b = waves * slots / (uint64_t)k;
+        if (b > 0 && waves * best < best_waves * b) {
+            best = b;
+            best_waves = waves;
+        }
+    }
+    return best;
+}
+
 // ---- host modular helpers (exact, 128-bit) -------------------------------
 static inline uint64_t mulmod_u64(uint64_t a, uint64_t b, uint64_t m) {
     return (uint64_t)(((unsigned __int128)a * b) % m);

@@ -187,7 +187,7 @@ static cudaError_t launch_affine_n(const PolyArgs &args, int k, int sm_count, cu
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
     // one resident wave shared by the k moduli, no more blocks than chunks
-    uint64_t bpm = ((uint64_t)per_sm * sm_count + k - 1) / k;
+    uint64_t bpm = blocks_per_modulus((uint64_t)per_sm * sm_count, k);
     const uint64_t max_blocks = (args.chunks + BT - 1) / BT;
     if (bpm > max_blocks) bpm = max_blocks;
     if (bpm < 1) bpm = 1;

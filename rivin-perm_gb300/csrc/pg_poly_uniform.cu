@@ -175,7 +175,7 @@ static cudaError_t launch_uniform_n(const PolyArgs &args, int k, int sm_count, c
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, uniform_m32_kernel<N>, BT, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
-    uint64_t bpm = ((uint64_t)per_sm * sm_count + k - 1) / k;
+    uint64_t bpm = blocks_per_modulus((uint64_t)per_sm * sm_count, k);
     const uint64_t max_blocks = (args.chunks + BT - 1) / BT;
     if (bpm > max_blocks) bpm = max_blocks;
     if (bpm < 1) bpm = 1;

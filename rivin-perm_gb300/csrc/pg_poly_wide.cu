@@ -205,7 +205,7 @@ int affine_wide_residues(const int64_t *C, const int64_t *L, int n, uint64_t lo,
     PG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, affine_wide_kernel,
                                                           POLY_WIDE_BT, smem));
     if (per_sm < 1) per_sm = 1;
-    uint64_t bpm = ((uint64_t)per_sm * dev.sm_count + k - 1) / k;
+    uint64_t bpm = blocks_per_modulus((uint64_t)per_sm * dev.sm_count, k);
     const uint64_t max_blocks = (a.chunks + POLY_WIDE_BT - 1) / POLY_WIDE_BT;
     if (bpm > max_blocks) bpm = max_blocks;
     if (bpm < 1) bpm = 1;

@@ -222,22 +222,23 @@ static int glynn_m32_batch(const uint64_t *mats, int n, const uint64_t *moduli,
         }
     }
 
-    // Launch shape: one resident wave of blocks shared by the k moduli; each
-    // thread owns a contiguous range of ~128 chunks of >= 64 states (small
-    // orders use fewer blocks so every thread keeps >= 512 states).
+    // Launch shape: whole waves of blocks shared by the k moduli; each thread
+    // owns a contiguous range of ~128 chunks of >= 64 states (small orders use
+    // fewer blocks so every thread keeps >= 128 states).
     const int occ = occupancy_m32_any(N, wide);
     const int log_states = n - 1;
     const bool partial = hi > 0;
     const uint64_t span = partial ? hi - lo : 1ull << log_states;
-    uint64_t bpm = ((uint64_t)occ * dev.sm_count + k - 1) / k;
-    while (bpm > 1 && (span >> 9) < bpm * 256) bpm >>= 1;
-    if (bpm < 1) bpm = 1;
+    uint64_t bpm = blocks_per_modulus((uint64_t)occ * dev.sm_count, k);
+    while (bpm > 1 && (span >> 7) < bpm * 256) bpm >>= 1;
     if (bpm > 65535) bpm = 65535;
     int log_T = 0;
     while ((2ull << log_T) <= bpm * 256) log_T++;
     ChunkPlan pl;
     pl.log_len = log_states - (log_T + 7);
-    const int min_len = log_states < 6 ? log_states : 6;
+    // chunks of 16 states where 64 would leave a thread less than eight
+    const int floor_len = (span >> 9) < bpm * 256 ? 4 : 6;
+    const int min_len = log_states < floor_len ? log_states : floor_len;
     if (pl.log_len < min_len) pl.log_len = min_len;
     if (pl.log_len > 30) pl.log_len = 30;
     if (pl.log_len < 1) pl.log_len = 1;
