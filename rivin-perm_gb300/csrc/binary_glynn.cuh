@@ -10,53 +10,58 @@
 // for every state (perm_binary_omp.c:236-347, perm_binary_cuda.cu:111-205);
 // this kernel only searches for the states without a zero row.
 //
-// Search.  A chunk is the 1024 states of one setting of the high columns'
-// signs: bit k of lane l's word is the state whose low ten signs are
-// k | l << 5 (aligned 2^10-state Gray windows, in another order).  The high
-// columns are common to the warp, so an even-degree row is zero exactly
-// where the low columns hold x = deg_r / 2 - (ones in high minus columns)
-// more, a word that depends only on the lane and on x in 0..dlow_r (any
-// other x: never zero).  Rows are packed into groups whose table of AND-ed
-// "no zero" words, one per combination of the rows' x, fits in shared
-// memory ([entry][32 lanes]: no bank conflicts); a chunk costs one load and
-// one AND per group, with a vote after every four groups.  The 32 lanes
-// prepare the table entries of 32 consecutive chunks (popcounts of the high
-// signs) and publish them through shared memory.
+// Search.  A chunk is the 1024 W states of one setting of the high columns'
+// signs (W words a lane): bit k of word h of lane l is the state whose low
+// signs are k | l << 5 | h << 10 (aligned Gray windows, in another order).
+// The high columns are common to the warp, so an even-degree row is zero
+// exactly where the low columns hold x = deg_r / 2 - (ones in high minus
+// columns) more, words that depend only on the lane and on x in 0..dlow_r
+// (any other x: never zero).  Rows are packed into groups whose table of
+// AND-ed "no zero" words, one entry per combination of the rows' x, fits in
+// shared memory ([entry][32 lanes][W]: no bank conflicts); a chunk costs one
+// load and W ANDs per group, with a vote after every eight groups.  The 32
+// lanes prepare the entries of 32 consecutive chunks, whose signs differ in
+// five columns: row counts are bytes, the warp's count minus a 32-row
+// table's, four rows per subtraction.  W = 2 where under 1/64 of the states
+// survive (grid40 34.9 ms, 58.6 with W = 1); else the evaluations need the
+// shared memory and W = 1 is faster (36 x 36 Bernoulli(1/2): 21.3 against
+// 26.7 ms).
 //
 // Evaluation.  Surviving states are appended to a per-warp queue; whenever
 // 32 are queued every lane evaluates one exactly.  The row sums come as
-// bytes: base bytes of the chunk minus low-column bytes of the state (two
-// shared tables, four rows per 32-bit subtraction) and one byte permute per
-// row, then the exact multi-word term of exact_glynn.cuh (row groups, signed
-// running product, 64-bit column accumulators).  Counting the signs by
-// popcount took 40 issues of the quarter-rate pipe per 32 states, two thirds
-// of the evaluation.
+// bytes: base bytes of the chunk (and of h) minus a table of the ten low
+// columns, four rows per subtraction, and one byte permute per row; then the
+// exact multi-word term of exact_glynn.cuh (row groups, signed running
+// product, 64-bit column accumulators).  Counting the signs by popcount took
+// 40 issues of the quarter-rate pipe per 32 states.
 //
 // Rows are padded to NPAD (pad rows: degree 1, no toggled column, s = 1) so
 // that one instantiation serves a range of orders; the walk itself runs the
 // true order's 2^(n-1) states.  Accumulation, the block reduction and the
 // per-block result slots are those of the exact kernel.
 //
-// Issue bound (82 % of the issue slots; 6 % quarter-rate pipe).  Whole calls
-// against the bit-sliced tracker that updated one state per lane and step
-// and evaluated by popcount: 4x4x5 grid (40 x 40, 0.08 % survive) 446 -> 59
-// ms, 36 x 36 Bernoulli(1/2) (6-13 % survive) 68 -> 32 ms.
+// Issue bound (65-80 % of the issue slots).  Whole calls against a
+// bit-sliced tracker that updated one state per lane and step and evaluated
+// by popcount: 4x4x5 grid (40 x 40, 0.08 % survive) 441 -> 34.9 ms, 36 x 36
+// Bernoulli(1/2) (6-13 % survive) 67-76 -> 22-28 ms.
 #pragma once
 
 #include "exact_glynn.cuh"
 
 namespace pg {
 
-constexpr int BIN_LOW = 10;        // columns spread over word bits (5) and lanes (5)
+// columns spread over word bits (5), lanes (5) and, with two words a lane, words
+__host__ __device__ constexpr int bin_low(int W) { return 9 + W; }
+constexpr int BIN_TAB = 10;        // low columns of the evaluation's table
 constexpr int BIN_QCAP = 320;      // queue entries per warp (31 pending + 32 lanes x 8 bits)
 constexpr size_t BIN_SMEM = 222 * 1024;   // dynamic shared memory of a block, at most
 
 // One even-degree row, in table-group order.
 struct BinTrack {
-    uint64_t high;      // the row's ones in toggled columns 10, 11, ... (bit 0: column 10)
-    uint16_t low;       // the row's ones in columns 0..9
+    uint64_t high;      // the row's ones in toggled columns bin_low, ... (bit 0 the first)
+    uint16_t low;       // the row's ones in the columns below
     uint8_t half;       // deg / 2
-    uint8_t cap;        // ones in columns 0..9, plus 1: the entry of "never zero"
+    uint8_t cap;        // ones in `low`, plus 1: the entry of "never zero"
     uint16_t stride;    // entries per unit of this row's x in its group's table
     uint16_t base;      // the group's first entry on its first row, else 0xffff
 };
@@ -69,6 +74,7 @@ struct BinaryArgs {
     int entries;               // table entries (entry 0: no row is zero)
     int list_words;            // words of a chunk's list: the byte offset of each group's
                                // entry, padded with entry 0 to a multiple of four
+    int words;                 // words a lane: 2 when few states survive, else 1
     int sparse;                // few states survive
     int warps;                 // warps of a block
     unsigned long long *acc;   // [NL] per-word sums (exact kernel layout)
@@ -82,28 +88,21 @@ struct BinaryArgs {
     int log_unit;              // batches of a work unit
 };
 
-#ifndef BIN_T32
-#define BIN_T32 768
-#endif
-#ifndef BIN_T40
-#define BIN_T40 768
-#endif
-#ifndef BIN_T48
-#define BIN_T48 512
-#endif
 // threads of a block, at most: as many warps as the registers allow
 // (fewer when the tables leave no room for their lists)
-__host__ __device__ constexpr int binary_max_threads(int NPAD) {
-    return NPAD > 40 ? BIN_T48 : NPAD > 32 ? BIN_T40 : BIN_T32;
+__host__ __device__ constexpr int binary_max_threads(int NPAD, int W) {
+    return NPAD > 40 ? 512 : W > 1 ? 640 : 768;
 }
-// words of a state's row bytes, padded for 16-byte loads
-__host__ __device__ constexpr int binary_row_words(int NPAD) { return (NPAD / 4 + 3) & ~3; }
-__host__ __device__ constexpr size_t binary_warp_bytes(int NPAD, int list_words) {
-    return (size_t)32 * binary_row_words(NPAD) * 4 + (size_t)32 * list_words * 4 + BIN_QCAP * 2;
+// words of a state's row bytes, padded for 8-byte loads
+__host__ __device__ constexpr int binary_row_words(int NPAD) { return (NPAD / 4 + 1) & ~1; }
+constexpr int BIN_TRACK_WORDS = 12;     // bytes of the even-degree rows (at most 48)
+__host__ __device__ constexpr size_t binary_warp_bytes(int NPAD, int W, int list_words) {
+    return (size_t)32 * W * binary_row_words(NPAD) * 4 + (size_t)32 * list_words * 4 + BIN_QCAP * 2 +
+           BIN_TRACK_WORDS * 4 + 48;
 }
-__host__ __device__ constexpr size_t binary_smem(int NPAD, int entries, int list_words, int warps) {
-    return (size_t)entries * 128 + (size_t)1024 * binary_row_words(NPAD) * 4 +
-           warps * binary_warp_bytes(NPAD, list_words);
+__host__ __device__ constexpr size_t binary_smem(int NPAD, int W, int entries, int list_words, int warps) {
+    return (size_t)entries * 128 * W + (size_t)(1024 + 32) * binary_row_words(NPAD) * 4 +
+           32 * BIN_TRACK_WORDS * 4 + warps * ((binary_warp_bytes(NPAD, W, list_words) + 15) & ~(size_t)15);
 }
 
 // byte K of x, sign-extended
@@ -114,21 +113,28 @@ __device__ __forceinline__ int32_t binary_byte(uint32_t x) {
     return r;
 }
 
-template <int NPAD, int G>
-__global__ void __launch_bounds__(binary_max_threads(NPAD), 1) binary_glynn_kernel(BinaryArgs a) {
+template <int NPAD, int G, int W>
+__global__ void __launch_bounds__(binary_max_threads(NPAD, W), 1) binary_glynn_kernel(BinaryArgs a) {
     using S = ExactShape<NPAD, G>;
     constexpr int NL = S::NL, NR = S::NR;
     constexpr int FOLD = 1 << EXACT_LOGU;   // terms the 64-bit columns hold between folds
-    constexpr int NW = NPAD / 4, LS = binary_row_words(NPAD);
+    constexpr int NW = NPAD / 4, LS = binary_row_words(NPAD), TW = BIN_TRACK_WORDS;
+    constexpr int LOW = bin_low(W), HI = LOW + 5;         // first column common to a batch of 32 chunks
     extern __shared__ uint4 bin_shared[];
-    uint32_t *ztab = reinterpret_cast<uint32_t *>(bin_shared);     // [entries][32]
-    uint32_t *ltab = ztab + (size_t)a.entries * 32;                 // [1024][LS]
+    uint32_t *ztab = reinterpret_cast<uint32_t *>(bin_shared);      // [entries][32][W]
+    uint32_t *ltab = ztab + (size_t)a.entries * 32 * W;             // [1024][LS]
+    uint32_t *ctab = ltab + 1024 * LS;                // [32][LS] bytes of the five chunk columns
+    uint32_t *xtab = ctab + 32 * LS;                  // [32][TW] the same of the even rows
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    char *mine = reinterpret_cast<char *>(ltab + 1024 * LS) + warp * binary_warp_bytes(NPAD, a.list_words);
-    uint32_t *base = reinterpret_cast<uint32_t *>(mine);            // [32][LS]
-    uint32_t *list = base + 32 * LS;                                // [32][list_words]
-    uint16_t *q = reinterpret_cast<uint16_t *>(list + 32 * a.list_words);
+    char *mine = reinterpret_cast<char *>(xtab + 32 * TW) +
+                 warp * ((binary_warp_bytes(NPAD, W, a.list_words) + 15) & ~(size_t)15);
+    uint32_t *list = reinterpret_cast<uint32_t *>(mine);            // [32][list_words]
+    uint32_t *base = list + 32 * a.list_words;                      // [32][W][LS]
+    uint32_t *ucnt = base + 32 * W * LS;                                // row bytes, then even rows'
+    uint32_t *xcnt = ucnt + 12;
+    uint16_t *q = reinterpret_cast<uint16_t *>(xcnt + TW);
     __shared__ BinTrack s_trk[48];
+    __shared__ uint4 s_rec[48];         // cap, stride bytes, group's first byte + 1 on its last row
     __shared__ uint64_t s_rm[NPAD];
     __shared__ int32_t s_deg[NPAD];
     __shared__ uint32_t s_eq[32][6];    // [mask][v]: the k in 0..31 with popc(k & mask) == v
@@ -144,30 +150,56 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD), 1) binary_glynn_kern
         s_eq[i / 6][i % 6] = w;
     }
     __syncthreads();
-    if (warp == 0) ztab[lane] = 0xffffffffu;
+    if (warp == 0)
+        for (int h = 0; h < W; h++) ztab[lane * W + h] = 0xffffffffu;
     for (int e0 = 0; e0 < a.ntracked;) {            // table groups
         int e1 = e0 + 1, size = s_trk[e0].cap + 1;
         for (; e1 < a.ntracked && s_trk[e1].base == 0xffff; e1++) size *= s_trk[e1].cap + 1;
+        if ((int)threadIdx.x >= e0 && (int)threadIdx.x < e1)
+            s_rec[threadIdx.x] = make_uint4(s_trk[threadIdx.x].cap, s_trk[threadIdx.x].stride * 128u * W,
+                                            (int)threadIdx.x == e1 - 1 ? s_trk[e0].base * 128u * W + 1 : 0, 0);
         for (int idx = warp; idx < size; idx += warps) {
-            uint32_t w = 0xffffffffu;
+            uint32_t w[W];
+#pragma unroll
+            for (int h = 0; h < W; h++) w[h] = 0xffffffffu;
             for (int e = e0, rem = idx; e < e1; e++) {
                 const int cap = s_trk[e].cap, low = s_trk[e].low;
                 const int x = rem % (cap + 1), v = x - __popc((low >> 5) & lane);
                 rem /= cap + 1;
-                if (x < cap && v >= 0 && v <= 5) w &= ~s_eq[low & 31][v];
+#pragma unroll
+                for (int h = 0; h < W; h++) {
+                    const int y = v - (h & (low >> 10));
+                    if (x < cap && y >= 0 && y <= 5) w[h] &= ~s_eq[low & 31][y];
+                }
             }
-            ztab[(s_trk[e0].base + idx) * 32 + lane] = w;
+#pragma unroll
+            for (int h = 0; h < W; h++) ztab[((s_trk[e0].base + idx) * 32 + lane) * W + h] = w[h];
         }
         e0 = e1;
     }
-    for (int i = threadIdx.x; i < 1024 * NW; i += blockDim.x) {
-        const int w = i & 1023, r = (i >> 10) * 4;
+    // twice the ones of four rows among the minus columns of `bits`
+    auto row_bytes = [&](int v, int shift, uint32_t bits) {
         uint32_t b = 0;
 #pragma unroll
         for (int t = 0; t < 4; t++)
-            b |= (uint32_t)(2 * __popc((uint32_t)s_rm[r + t] & (uint32_t)w)) << (8 * t);
-        ltab[w * LS + (i >> 10)] = b;
+            b |= (uint32_t)(2 * __popc((uint32_t)(s_rm[4 * v + t] >> shift) & bits)) << (8 * t);
+        return b;
+    };
+    for (int i = threadIdx.x; i < 1024 * NW; i += blockDim.x)
+        ltab[(i & 1023) * LS + (i >> 10)] = row_bytes(i >> 10, 0, (uint32_t)(i & 1023));
+    for (int i = threadIdx.x; i < 32 * NW; i += blockDim.x)
+        ctab[(i & 31) * LS + (i >> 5)] = row_bytes(i >> 5, LOW, (uint32_t)(i & 31));
+    for (int i = threadIdx.x; i < 32 * TW; i += blockDim.x) {
+        uint32_t b = 0;
+        for (int t = 0; t < 4; t++) {
+            const int e = 4 * (i >> 5) + t;
+            if (e < a.ntracked) b |= (uint32_t)__popc((uint32_t)s_trk[e].high & (uint32_t)(i & 31)) << (8 * t);
+        }
+        xtab[(i & 31) * TW + (i >> 5)] = b;
     }
+    uint32_t h_bytes[NW];               // column 10 (two words a lane)
+#pragma unroll
+    for (int v = 0; v < NW; v++) h_bytes[v] = W > 1 ? row_bytes(v, BIN_TAB, 1u) : 0;
     __syncthreads();
 
     uint32_t acc[NL];
@@ -178,23 +210,21 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD), 1) binary_glynn_kern
     int terms = 0;       // terms in the columns since the last fold (warp-uniform)
     int qn = 0;          // queued states (warp-uniform)
     uint32_t c_odd = 0;  // parity of the batch's first chunk
-
     // evaluates the last `count` (<= 32) queued states
     auto evaluate = [&](int count) {
         __syncwarp();
         qn -= count;
         const bool live = lane < count;
-        const uint32_t e = live ? q[qn + lane] : 0, w = e & 1023u, k = e >> 10;
+        // low signs, chunk of the batch (5 bits); the chunk and h pick the base row
+        const uint32_t e = live ? q[qn + lane] : 0, k = e >> LOW;
         uint32_t d[LS];
 #pragma unroll
-        for (int v = 0; v < LS / 4; v++) {
-            const uint4 x = reinterpret_cast<const uint4 *>(base + k * LS)[v];
-            const uint4 y = reinterpret_cast<const uint4 *>(ltab + w * LS)[v];
+        for (int v = 0; v < LS / 2; v++) {
+            const uint2 x = reinterpret_cast<const uint2 *>(base + (e >> BIN_TAB) * LS)[v];
+            const uint2 y = reinterpret_cast<const uint2 *>(ltab + (e & 1023u) * LS)[v];
             // bytes 128 + s_r, no borrow between them; then two's complement
-            d[4 * v + 0] = (x.x - y.x) ^ 0x80808080u;
-            d[4 * v + 1] = (x.y - y.y) ^ 0x80808080u;
-            d[4 * v + 2] = (x.z - y.z) ^ 0x80808080u;
-            d[4 * v + 3] = (x.w - y.w) ^ 0x80808080u;
+            d[2 * v + 0] = (x.x - y.x) ^ 0x80808080u;
+            d[2 * v + 1] = (x.y - y.y) ^ 0x80808080u;
         }
         int32_t s[NPAD];
 #pragma unroll
@@ -205,26 +235,18 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD), 1) binary_glynn_kern
             s[4 * v + 3] = binary_byte<3>(d[v]);
         }
         if (!live) s[0] = 0;
-        exact_term_col<NPAD, G, 0>(s, col, colt, (__popc(w) ^ k ^ c_odd) & 1u, terms == 0);
+        // batches start at even chunks or hold one
+        exact_term_col<NPAD, G, 0>(s, col, colt, (__popc(e & ((1u << LOW) - 1)) ^ k ^ c_odd) & 1u,
+                                   terms == 0);
         if (++terms == FOLD) {
             FoldCols<NR, NL>::apply(acc, col, colt);
             terms = 0;
         }
         __syncwarp();
     };
-
-    // appends the states `part` of chunk k at queue positions given by a scan
-    // over the lanes (inc: inclusive count), then evaluates full rounds
-    auto push = [&](uint32_t part, int k, int inc, int total) {
-        int pos = qn + inc - __popc(part);
-        while (part) {
-            const uint32_t rest = part & (part - 1);
-            q[pos++] = (uint16_t)((k << 10) | (lane << 5) | __popc((part ^ rest) - 1));
-            part = rest;
-        }
-        qn += total;
-        while (qn >= 32) evaluate(32);
-    };
+    // Appends the states of `alive` (tag: chunk and h).  Few survivors: one of
+    // each lane at a time, placed by a ballot.  Many: placed by a scan over the
+    // lanes' counts, all at once while they fit the queue, else 256 at most.
     auto scan = [&](uint32_t part) {
         int inc = __popc(part);
 #pragma unroll
@@ -234,121 +256,172 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD), 1) binary_glynn_kern
         }
         return inc;
     };
-    auto append = [&](uint32_t alive, int k) {
-        if (a.sparse) {                              // one state of each lane at a time
-            for (uint32_t mask = __ballot_sync(0xffffffffu, alive != 0); mask;
-                 mask = __ballot_sync(0xffffffffu, alive != 0)) {
-                if (alive) {
-                    const uint32_t rest = alive & (alive - 1);
-                    q[qn + __popc(mask & ((1u << lane) - 1u))] =
-                        (uint16_t)((k << 10) | (lane << 5) | __popc((alive ^ rest) - 1));
-                    alive = rest;
+    auto push = [&](uint32_t part, uint32_t tag, int inc, int total) {
+        int pos = qn + inc - __popc(part);
+        while (part) {
+            const uint32_t rest = part & (part - 1);
+            q[pos++] = (uint16_t)(tag | (lane << 5) | __popc((part ^ rest) - 1));
+            part = rest;
+        }
+        qn += total;
+        while (qn >= 32) evaluate(32);
+    };
+    auto append = [&](uint32_t alive, uint32_t tag) {
+        uint32_t mask = __ballot_sync(0xffffffffu, alive != 0);
+        if (!mask) return;
+        if (!a.sparse) {
+            const int inc = scan(alive), total = __shfl_sync(0xffffffffu, inc, 31);
+            if (qn + total <= BIN_QCAP) {
+                push(alive, tag, inc, total);
+            } else {
+                for (int o = 0; o < 32; o += 8) {
+                    const uint32_t part = alive & (0xffu << o);
+                    const int pi = scan(part);
+                    push(part, tag, pi, __shfl_sync(0xffffffffu, pi, 31));
                 }
-                qn += __popc(mask);
-                if (qn >= 32) evaluate(32);
             }
             return;
         }
-        const int inc = scan(alive), total = __shfl_sync(0xffffffffu, inc, 31);
-        if (qn + total <= BIN_QCAP) {
-            push(alive, k, inc, total);
-        } else {                                     // at most 256 states at a time
-            for (int o = 0; o < 32; o += 8) {
-                const uint32_t part = alive & (0xffu << o);
-                const int pi = scan(part);
-                push(part, k, pi, __shfl_sync(0xffffffffu, pi, 31));
+        for (; mask; mask = __ballot_sync(0xffffffffu, alive != 0)) {
+            if (alive) {
+                const uint32_t rest = alive & (alive - 1);
+                q[qn + __popc(mask & ((1u << lane) - 1u))] =
+                    (uint16_t)(tag | (lane << 5) | __popc((alive ^ rest) - 1));
+                alive = rest;
             }
+            qn += __popc(mask);
+            if (qn >= 32) evaluate(32);
         }
     };
 
     // Work units go to warps from a counter (the share of surviving states
     // varies strongly along the walk with the signs of the columns), one
-    // ahead, so that the atomic's round trip overlaps the work.
-    const uint64_t chunk0 = a.state_lo >> BIN_LOW;
-    const uint64_t chunks = ((a.state_hi + (1u << BIN_LOW) - 1) >> BIN_LOW) - chunk0;
-    const uint64_t units = (chunks + (1ull << (a.log_steps + a.log_unit)) - 1) >> (a.log_steps + a.log_unit);
-    const char *zl = reinterpret_cast<const char *>(ztab + lane);
+    // ahead, so that the atomic's round trip overlaps the work.  A unit is
+    // 2^log_unit batches of 2^log_steps chunks, aligned.
+    const uint64_t c_lo = a.state_lo >> LOW;
+    const uint64_t c_hi = (a.state_hi + (1u << LOW) - 1) >> LOW;
+    const int log_all = a.log_steps + a.log_unit;
+    const uint64_t units = ((c_hi - 1) >> log_all) - (c_lo >> log_all) + 1;
+    const char *zl = reinterpret_cast<const char *>(ztab + lane * W);
     bool aborted = false;
     uint32_t polls = 0;
     for (uint64_t unit = (uint64_t)warp * gridDim.x + blockIdx.x; unit < units && !aborted;) {
         unsigned long long nx = 0;
         if (lane == 0) nx = (uint64_t)gridDim.x * warps + atomicAdd(a.next, 1ull);
         for (uint32_t bb = 0; bb < (1u << a.log_unit); bb++) {
-            const uint64_t ci = ((unit << a.log_unit) + bb) << a.log_steps;
-            if (ci >= chunks) break;
+            // chunks c0 + k0 .. c0 + k1 - 1 of the batch lie in the window
+            const uint64_t c0 = (((c_lo >> log_all) + unit) << log_all) + ((uint64_t)bb << a.log_steps);
+            const int k1 = c_hi <= c0 ? 0 : c_hi - c0 < (1ull << a.log_steps) ? (int)(c_hi - c0)
+                                                                             : 1 << a.log_steps;
+            const int kfirst = c_lo > c0 ? (c_lo - c0 < (uint64_t)k1 ? (int)(c_lo - c0) : k1) : 0;
+            if (kfirst >= k1) continue;
             // the host-mapped abort word is read once per 128 batches, from
             // the warp's second period on
             if ((++polls & 127) == 0 && __any_sync(0xffffffffu, *a.abort_flag != 0)) {
                 aborted = true;
                 break;
             }
-            const int steps = chunks - ci < (1ull << a.log_steps) ? (int)(chunks - ci) : 1 << a.log_steps;
-            const uint64_t c0 = chunk0 + ci;
             c_odd = (uint32_t)c0;
-            // this lane's chunk: row bytes and table entries of its high signs
-            const uint64_t hw = (c0 + lane) ^ ((c0 + lane) >> 1);
-            auto ones = [&](uint64_t m) {
-                return NPAD > 40 ? __popcll(m & hw) : __popc((uint32_t)m & (uint32_t)hw);
-            };
-            if (lane < steps) {
+            const bool edge = ((c0 + kfirst) << LOW) < a.state_lo || ((c0 + k1) << LOW) > a.state_hi;
+            // the batch's common high signs: gray(c0 >> 5) in columns HI and up
+            const uint64_t b5 = c0 >> 5;
+            const uint32_t hw = (uint32_t)(b5 ^ (b5 >> 1));
+            auto ones = [&](uint64_t m) { return __popc((uint32_t)m & hw); };
+            for (int r = lane; r < NPAD; r += 32)
+                reinterpret_cast<uint8_t *>(ucnt)[r] = (uint8_t)(128 + s_deg[r] - 2 * ones(s_rm[r] >> HI));
+            for (int r = lane; r < a.ntracked; r += 32)
+                reinterpret_cast<uint8_t *>(xcnt)[r] = (uint8_t)(128 + s_trk[r].half - ones(s_trk[r].high >> 5));
+            __syncwarp();
+            // this lane's chunk: the signs of the five columns below those
+            const uint32_t l5 = ((uint32_t)c0 + lane) & 31u;
+            const uint32_t x5 = l5 ^ (l5 >> 1) ^ (((uint32_t)b5 & 1u) << 4);
+            {
+                const uint32_t *cb = ctab + x5 * LS;
+                uint32_t *o = base + lane * W * LS;
 #pragma unroll
                 for (int v = 0; v < NW; v++) {
-                    uint32_t b = 0;
-#pragma unroll
-                    for (int t = 0; t < 4; t++)
-                        b |= (uint32_t)(128 + s_deg[4 * v + t] - 2 * ones(s_rm[4 * v + t] >> BIN_LOW))
-                             << (8 * t);
-                    base[lane * LS + v] = b;
+                    const uint32_t b = ucnt[v] - cb[v];
+                    o[v] = b;
+                    if (W > 1) o[LS + v] = b - h_bytes[v];
                 }
             }
             {
                 uint32_t *ll = list + lane * a.list_words;
-                int g = -1;
+                int g = 0;
                 uint32_t off = 0;
-                for (int e = 0; e < a.ntracked; e++) {
-                    const BinTrack t = s_trk[e];
-                    if (t.base != 0xffff) {
-                        if (g >= 0) ll[g] = off * 128;
-                        g++;
-                        off = t.base;
+                for (int e = 0; e < a.ntracked; e += 4) {
+                    // bytes of x in two's complement: negative ones exceed every cap
+                    const uint32_t x = (xcnt[e >> 2] - xtab[x5 * TW + (e >> 2)]) ^ 0x80808080u;
+#pragma unroll
+                    for (int t = 0; t < 4; t++) {
+                        if (e + t >= a.ntracked) break;
+                        const uint4 rec = s_rec[e + t];
+                        off += min(__byte_perm(x, 0, 0x4440 + t), rec.x) * rec.y;
+                        if (rec.z) {
+                            ll[g++] = off + rec.z - 1;
+                            off = 0;
+                        }
                     }
-                    off += min((uint32_t)(t.half - ones(t.high)), (uint32_t)t.cap) * t.stride;
                 }
-                for (; g < a.list_words; off = 0, g++) ll[g] = off * 128;
+                for (; g < a.list_words; g++) ll[g] = 0;
             }
             __syncwarp();
-            for (int k0 = 0; k0 < steps; k0 += 2) {
-                uint32_t alive[2] = {0xffffffffu, k0 + 1 < steps ? 0xffffffffu : 0u};
+            for (int k0 = kfirst; k0 < k1; k0 += 2) {
+                uint32_t alive[2][W];
+#pragma unroll
+                for (int t = 0; t < 2; t++)
+#pragma unroll
+                    for (int h = 0; h < W; h++) alive[t][h] = k0 + t < k1 ? 0xffffffffu : 0u;
                 for (int v = 0; v < a.list_words; v += 4) {
+                    uint32_t any = 0;
 #pragma unroll
                     for (int t = 0; t < 2; t++) {
-                        const uint4 o = *reinterpret_cast<const uint4 *>(list + (k0 + t) * a.list_words + v);
-                        const auto at = [&](uint32_t off) {
-                            return *reinterpret_cast<const uint32_t *>(zl + off);
-                        };
-                        alive[t] &= at(o.x) & at(o.y) & at(o.z) & at(o.w);
+                        // (beyond the batch: row 31, whose words are not used)
+                        const int row = k0 + t < 32 ? k0 + t : 31;
+                        const uint4 o = *reinterpret_cast<const uint4 *>(list + row * a.list_words + v);
+                        if constexpr (W > 1) {
+                            const auto at = [&](uint32_t off) {
+                                return *reinterpret_cast<const uint2 *>(zl + off);
+                            };
+                            const uint2 z0 = at(o.x), z1 = at(o.y), z2 = at(o.z), z3 = at(o.w);
+                            alive[t][0] &= z0.x & z1.x & z2.x & z3.x;
+                            alive[t][W - 1] &= z0.y & z1.y & z2.y & z3.y;
+                        } else {
+                            const auto at = [&](uint32_t off) {
+                                return *reinterpret_cast<const uint32_t *>(zl + off);
+                            };
+                            alive[t][0] &= at(o.x) & at(o.y) & at(o.z) & at(o.w);
+                        }
+#pragma unroll
+                        for (int h = 0; h < W; h++) any |= alive[t][h];
                     }
-                    if ((v & 4) && !__any_sync(0xffffffffu, (alive[0] | alive[1]) != 0)) break;
+                    if ((v & 4) && !__any_sync(0xffffffffu, any != 0)) break;
+                }
+                if (edge) {             // a window that starts or ends inside a chunk
+#pragma unroll
+                    for (int t = 0; t < 2; t++)
+#pragma unroll
+                        for (int h = 0; h < W; h++) {
+                            const uint64_t c = c0 + k0 + t;
+                            uint32_t in = 0;
+                            for (int k = 0; k < 32; k++) {
+                                uint32_t i = (uint32_t)(k | (lane << 5) | (h << 10)) ^
+                                             (uint32_t)((c & 1) << (LOW - 1));
+                                i ^= i >> 1;
+                                i ^= i >> 2;
+                                i ^= i >> 4;
+                                i ^= i >> 8;
+                                const uint64_t g = (c << LOW) | i;
+                                in |= (uint32_t)(g >= a.state_lo && g < a.state_hi) << k;
+                            }
+                            alive[t][h] &= in;
+                        }
                 }
 #pragma unroll
-                for (int t = 0; t < 2; t++) {
-                    const uint64_t c = c0 + k0 + t;
-                    if ((c << BIN_LOW) < a.state_lo || ((c + 1) << BIN_LOW) > a.state_hi) {
-                        // a window that starts or ends inside this chunk
-                        uint32_t in = 0;
-                        for (int k = 0; k < 32; k++) {
-                            uint32_t i = (uint32_t)(k | (lane << 5)) ^ (uint32_t)((c & 1) << (BIN_LOW - 1));
-                            i ^= i >> 1;
-                            i ^= i >> 2;
-                            i ^= i >> 4;
-                            i ^= i >> 8;
-                            const uint64_t g = (c << BIN_LOW) | i;
-                            in |= (uint32_t)(g >= a.state_lo && g < a.state_hi) << k;
-                        }
-                        alive[t] &= in;
-                    }
-                    if (__any_sync(0xffffffffu, alive[t] != 0)) append(alive[t], k0 + t);
-                }
+                for (int t = 0; t < 2; t++)
+#pragma unroll
+                    for (int h = 0; h < W; h++)
+                        append(alive[t][h], (uint32_t)((k0 + t) << LOW) | (uint32_t)(h << BIN_TAB));
             }
             if (qn > 0) evaluate(qn);       // the next batch has other base bytes
             __syncwarp();
@@ -358,7 +431,7 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD), 1) binary_glynn_kern
     if (terms > 0) FoldCols<NR, NL>::apply(acc, col, colt);
 
     // block reduction and result words: as the exact kernel
-    __shared__ long long red[binary_max_threads(NPAD) / 32][NL];
+    __shared__ long long red[binary_max_threads(NPAD, W) / 32][NL];
     __shared__ int any_abort;
     if (threadIdx.x == 0) any_abort = 0;
     __syncthreads();
@@ -374,18 +447,23 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD), 1) binary_glynn_kern
     exact_epilogue<NL>(red, any_abort, a.acc, a.part, a.status);
 }
 
-template <int NPAD, int G>
-cudaError_t launch_binary_glynn(const BinaryArgs &args, int blocks, cudaStream_t stream) {
-    const size_t smem = binary_smem(NPAD, args.entries, args.list_words, args.warps);
-    cudaError_t e = cudaFuncSetAttribute(binary_glynn_kernel<NPAD, G>,
+template <int NPAD, int G, int W>
+cudaError_t launch_binary_words(const BinaryArgs &args, int blocks, cudaStream_t stream) {
+    const size_t smem = binary_smem(NPAD, W, args.entries, args.list_words, args.warps);
+    cudaError_t e = cudaFuncSetAttribute(binary_glynn_kernel<NPAD, G, W>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    binary_glynn_kernel<NPAD, G><<<blocks, 32 * args.warps, smem, stream>>>(args);
+    binary_glynn_kernel<NPAD, G, W><<<blocks, 32 * args.warps, smem, stream>>>(args);
     return cudaGetLastError();
 }
+template <int NPAD, int G>
+cudaError_t launch_binary_glynn(const BinaryArgs &args, int blocks, cudaStream_t stream) {
+    return args.words == 2 ? launch_binary_words<NPAD, G, 2>(args, blocks, stream)
+                           : launch_binary_words<NPAD, G, 1>(args, blocks, stream);
+}
 
-// Compiled shapes (binary_inst_*.cu): NPAD in {32, 40, 48}, G in {5, 6, 7,
-// 8, 10}.  Orders below BINARY_MIN_N, and matrices whose sampled share of
+// Compiled shapes (binary_inst_*.cu): NPAD in {24, 28, ..., 48}, G in {5, 6,
+// 7, 8, 10}.  Orders below BINARY_MIN_N, and matrices whose sampled share of
 // states without a zero row exceeds BINARY_MAX_SURVIVORS, use the exact
 // kernel.  EXACT_BINARY=0 sends every 0/1 matrix to the exact kernel (for
 // comparisons).
@@ -404,6 +482,6 @@ cudaError_t launch_binary_any(int NPAD, int G, const BinaryArgs &args, int block
 // tables to fit beside the NPAD kernel's other shared memory, with the most
 // warps that allow it; group[e] = the row's group.  Returns the number of
 // groups, 0 if there is no such packing.
-int binary_pack_groups(int NPAD, const int *caps, int rows, int *group, int *warps);
+int binary_pack_groups(int NPAD, int W, const int *caps, int rows, int *group, int *warps);
 
 }  // namespace pg

@@ -194,8 +194,8 @@ struct ExactPlan {
     // 0/1 kernel (binary_glynn.cuh): bits of the largest even row's half
     // degree (0: the general kernel), tracked (even-degree) rows, padded
     // rows, table entries and list words, Gray window
-    int planes = 0, ntracked = 0, npad = 0, entries = 0, list_words = 0, sparse = 0,
-        warps = 0;
+    int planes = 0, ntracked = 0, npad = 0, entries = 0, list_words = 0, warps = 0,
+        words = 1, sparse = 0;
     size_t off_deg = 0, off_trk = 0;
     uint64_t lo = 0, hi = 0;
     ChunkPlan chunks{};
@@ -212,7 +212,9 @@ struct ExactPlan {
     volatile int *abort_dev = nullptr;
 };
 
-int binary_pack_groups(int NPAD, const int *caps, int rows, int *group, int *warps) {
+// Sixteen warps keep the kernel within 2 % of its best (12..24 measured).
+constexpr int BIN_WARPS_MIN = 16;
+int binary_pack_groups(int NPAD, int W, const int *caps, int rows, int *group, int *warps) {
     std::vector<int> by(rows);
     for (int e = 0; e < rows; e++) by[e] = e;
     std::stable_sort(by.begin(), by.end(), [&](int x, int y) { return caps[x] > caps[y]; });
@@ -228,19 +230,21 @@ int binary_pack_groups(int NPAD, const int *caps, int rows, int *group, int *war
         for (double v : size) total += v;
         return total < 65536 ? (size_t)total : 65536;
     };
-    const int most = binary_max_threads(NPAD) / 32;
-    for (int w = most; w >= most / 4; w -= most / 4)
-        for (int T = 1; T <= rows; T++) {
-            const int words = (T + 3) / 4 * 4;
-            if (binary_smem(NPAD, (int)pack(T), words, w) > BIN_SMEM) continue;
-            // the lookups run in fours: use all of them, with smaller tables
-            const int T4 = words < rows ? words : rows;
+    // the fewest lookups (a multiple of four) with at least BIN_WARPS_MIN
+    // warps, then the most warps for them; fewer warps only where nothing fits
+    const int most = binary_max_threads(NPAD, W) / 32;
+    int best = 0;
+    for (int w = most; w >= 2 && (w >= BIN_WARPS_MIN || !best); w -= 2)
+        for (int T = 4; T < rows + 4 && (!best || T < best); T += 4) {
+            const int groups = T < rows ? T : rows;
+            if (binary_smem(NPAD, W, (int)pack(groups), T, w) > BIN_SMEM) continue;
+            best = T;
             *warps = w;
-            if (T4 == T || binary_smem(NPAD, (int)pack(T4), words, w) <= BIN_SMEM) return T4;
-            pack(T);
-            return T;
         }
-    return 0;
+    if (!best) return 0;
+    const int groups = best < rows ? best : rows;
+    pack(groups);
+    return groups;
 }
 
 // The 0/1 kernel for a 0/1 matrix of order BINARY_MIN_N..48: the even-degree
@@ -249,45 +253,64 @@ int binary_pack_groups(int NPAD, const int *caps, int rows, int *group, int *war
 // keeps the fixed sign.  The share of states with no zero row is estimated
 // from 1024 sampled states: above BINARY_MAX_SURVIVORS the exact evaluations
 // would cost more than the general kernel, which then runs (as it does when
-// the matrix is not 0/1 or no compiled shape fits).
-static bool plan_build_binary(const int64_t *A, int n, ExactPlan *P) {
+// the matrix is not 0/1 or no compiled shape fits).  A whole walk takes the
+// transpose when fewer of its sampled states survive (36 x 36
+// Bernoulli(1/2): 6..13 % either way); windows keep the rows' own states.
+struct BinaryRows {
+    std::vector<uint64_t> deg, rows;     // padded to NPAD
+    std::vector<int> tracked;            // even-degree rows
+    int maxh = 0, survive = 0;           // largest half degree, survivors of 1024 samples
+};
+constexpr int BINARY_SAMPLES = 1024;
+static void binary_rows(const int64_t *A, int n, bool transposed, BinaryRows *B) {
+    const int NPAD = binary_npad(n);
+    B->deg.assign(NPAD, 1);
+    B->rows.assign(NPAD, 0);
+    for (int i = 0; i < n; i++) {
+        uint64_t d = 0, m = 0;
+        for (int j = 0; j < n; j++) {
+            const uint64_t v = (uint64_t)(transposed ? A[(size_t)j * n + i] : A[(size_t)i * n + j]);
+            d += v;
+            if (j < n - 1) m |= v << j;
+        }
+        B->deg[i] = d;
+        B->rows[i] = m;
+        if (d % 2 == 0) {
+            B->tracked.push_back(i);
+            B->maxh = std::max(B->maxh, (int)(d / 2));
+        }
+    }
+    // sampled share of states with no zero row (fixed LCG, Gray words)
+    uint64_t x = 0x9e3779b97f4a7c15ull;
+    const uint64_t state_mask = (1ull << (n - 1)) - 1;
+    for (int t = 0; t < BINARY_SAMPLES; t++) {
+        x = x * 6364136223846793005ull + 1442695040888963407ull;
+        const uint64_t g = (x >> 11) & state_mask, gm = g ^ (g >> 1);
+        bool zero = false;
+        for (int r : B->tracked)
+            if (2 * (uint64_t)__builtin_popcountll(B->rows[r] & gm) == B->deg[r]) { zero = true; break; }
+        B->survive += !zero;
+    }
+}
+
+static bool plan_build_binary(const int64_t *A, int n, bool whole, ExactPlan *P) {
     if (!EXACT_BINARY || n < BINARY_MIN_N || n > 48) return false;
     for (size_t i = 0; i < (size_t)n * n; i++)
         if (A[i] != 0 && A[i] != 1) return false;
     const int NPAD = binary_npad(n);
-    std::vector<uint64_t> deg(NPAD, 1), rows(NPAD, 0);
-    std::vector<int> tracked;
-    int maxh = 0;
-    for (int i = 0; i < n; i++) {
-        uint64_t d = 0, m = 0;
-        for (int j = 0; j < n; j++) {
-            d += (uint64_t)A[(size_t)i * n + j];
-            if (j < n - 1 && A[(size_t)i * n + j]) m |= 1ull << j;
-        }
-        deg[i] = d;
-        rows[i] = m;
-        if (d % 2 == 0) {
-            tracked.push_back(i);
-            maxh = std::max(maxh, (int)(d / 2));
-        }
-    }
-    if (tracked.empty()) return false;          // no row can vanish: every state counts
+    BinaryRows B;
+    binary_rows(A, n, false, &B);
+    if (B.tracked.empty()) return false;        // no row can vanish: every state counts
+    if (B.survive > BINARY_MAX_SURVIVORS * BINARY_SAMPLES) return false;
     int K = 2;
-    while ((1 << K) <= maxh) K++;
-    // sampled share of states with no zero row (fixed LCG, Gray words)
-    uint64_t x = 0x9e3779b97f4a7c15ull;
-    int survive = 0;
-    const int samples = 1024;
-    const uint64_t state_mask = (1ull << (n - 1)) - 1;
-    for (int t = 0; t < samples; t++) {
-        x = x * 6364136223846793005ull + 1442695040888963407ull;
-        const uint64_t g = (x >> 11) & state_mask, gm = g ^ (g >> 1);
-        bool zero = false;
-        for (int r : tracked)
-            if (2 * (uint64_t)__builtin_popcountll(rows[r] & gm) == deg[r]) { zero = true; break; }
-        survive += !zero;
+    while ((1 << K) <= B.maxh) K++;
+    if (whole) {
+        BinaryRows T;
+        binary_rows(A, n, true, &T);
+        if (!T.tracked.empty() && T.survive < B.survive) B = std::move(T);
     }
-    if (survive > BINARY_MAX_SURVIVORS * samples) return false;
+    const std::vector<uint64_t> &deg = B.deg, &rows = B.rows;
+    const std::vector<int> &tracked = B.tracked;
     std::vector<int> order(NPAD);
     int G = 0;
     for (int g : {10, 8, 7, 6, 5}) {
@@ -296,10 +319,13 @@ static bool plan_build_binary(const int64_t *A, int n, ExactPlan *P) {
     }
     if (!G) return false;
     const int nt = (int)tracked.size();
-    constexpr uint64_t low_mask = (1ull << BIN_LOW) - 1;
+    P->sparse = B.survive * 64 < BINARY_SAMPLES;
+    P->words = P->sparse ? 2 : 1;
+    const int low = bin_low(P->words);
+    const uint64_t low_mask = (1ull << low) - 1;
     std::vector<int> caps(nt), group(nt);
     for (int e = 0; e < nt; e++) caps[e] = __builtin_popcountll(rows[tracked[e]] & low_mask) + 1;
-    const int groups = binary_pack_groups(NPAD, caps.data(), nt, group.data(), &P->warps);
+    const int groups = binary_pack_groups(NPAD, P->words, caps.data(), nt, group.data(), &P->warps);
     if (!groups) return false;
     P->planes = K;
     P->ntracked = nt;
@@ -324,7 +350,7 @@ static bool plan_build_binary(const int64_t *A, int n, ExactPlan *P) {
         for (int e = 0; e < nt; e++) {
             if (group[e] != g) continue;
             BinTrack &t = trk[w++];
-            t.high = rows[tracked[e]] >> BIN_LOW;
+            t.high = rows[tracked[e]] >> low;
             t.low = (uint16_t)(rows[tracked[e]] & low_mask);
             t.half = (uint8_t)(deg[tracked[e]] / 2);
             t.cap = (uint8_t)caps[e];
@@ -335,7 +361,6 @@ static bool plan_build_binary(const int64_t *A, int n, ExactPlan *P) {
         entries += stride;
     }
     P->entries = entries;
-    P->sparse = survive * 64 < samples;
     P->list_words = (groups + 3) / 4 * 4;
     P->lo = 0;
     P->hi = 1ull << (n - 1);
@@ -409,8 +434,8 @@ static void add_block_slots(ExactPlan *P) {
     P->image.resize(P->total, 0);
 }
 
-static int plan_build(const int64_t *A, int n, ExactPlan *P) {
-    if (plan_build_binary(A, n, P)) {
+static int plan_build(const int64_t *A, int n, ExactPlan *P, bool whole = true) {
+    if (plan_build_binary(A, n, whole, P)) {
         DeviceInfo dev;
         int st = device_info(&dev);
         if (st != PG_OK) return st;
@@ -423,8 +448,8 @@ static int plan_build(const int64_t *A, int n, ExactPlan *P) {
         P->total = align_up(P->off_out + (size_t)(P->NL + 1) * 8, 256);
         P->image.resize(P->total, 0);
         // one block per SM: the warps share its tables
-        P->chunks.log_len = BIN_LOW;
-        P->chunks.chunks = 1ull << (n - 1 - BIN_LOW);
+        P->chunks.log_len = bin_low(P->words);
+        P->chunks.chunks = 1ull << (n - 1 - P->chunks.log_len);
         P->blocks = (uint64_t)dev.sm_count;
         add_block_slots(P);
         return PG_OK;
@@ -501,8 +526,9 @@ static int plan_launch(ExactPlan *P, cudaStream_t stream) {
         b.ntracked = P->ntracked;
         b.entries = P->entries;
         b.list_words = P->list_words;
-        b.sparse = P->sparse;
         b.warps = P->warps;
+        b.sparse = P->sparse;
+        b.words = P->words;
         b.acc = (unsigned long long *)(P->dev + P->off_acc);
         b.status = (int *)(P->dev + P->off_status);
         b.part = (unsigned long long *)(P->dev + P->off_part);
@@ -514,10 +540,10 @@ static int plan_launch(ExactPlan *P, cudaStream_t stream) {
         // batches of 32 chunks (one per lane) while every warp gets two of
         // them, shorter ones below; several batches to a unit on long walks,
         // so that the counter's atomics stay rare
-        const uint64_t chunks = ((P->hi - P->lo) >> BIN_LOW) + 1;
+        const uint64_t chunks = ((P->hi - P->lo) >> bin_low(P->words)) + 1;
         const uint64_t warps = P->blocks * (uint64_t)P->warps;
         b.log_steps = 5;
-        while (b.log_steps > 2 && (chunks >> b.log_steps) < 2 * warps) b.log_steps--;
+        while (b.log_steps > 1 && (chunks >> b.log_steps) < 2 * warps) b.log_steps--;
         b.log_unit = 0;
         while (b.log_unit < 3 && (chunks >> (6 + b.log_unit)) >= 32 * warps) b.log_unit++;
         PG_CUDA(launch_binary_any(P->npad, P->G, b, (int)P->blocks, stream));
@@ -642,7 +668,7 @@ int pg_exact_partial(const int64_t *A, int n, uint64_t state_lo, uint64_t state_
     using namespace pg;
     if (!A || !words || !nwords || n < 2 || n >= 64) return fail(PG_EINVAL, "bad arguments");
     ExactPlan P;
-    int st = plan_build(A, n, &P);
+    int st = plan_build(A, n, &P, false);
     if (st != PG_OK) return st;
     if ((st = plan_restrict(&P, state_lo, state_hi)) != PG_OK) return st;
     if (max_words < P.NL) return fail(PG_ERANGE, "words buffer too small");
