@@ -62,7 +62,7 @@ struct GradShape {
     // two blocks of 128 threads per SM: (RMAX + waiting slots) rows of 8
     // bytes per thread and the table in 113 KB
     static constexpr int RCAP = RW == 8 ? 8 : 10;
-    static constexpr int RMAX = N - 1 - LW < 0 ? 0 : N - 1 - LW < RCAP ? N - 1 - LW : RCAP;
+    static constexpr int RMAX = N - 1 - LW < 1 ? 1 : N - 1 - LW < RCAP ? N - 1 - LW : RCAP;
     static constexpr int WAIT = LW + 1 > GRAD_TREE - 1 ? LW + 1 : GRAD_TREE - 1;
     static constexpr int SLOTS = RMAX + WAIT;
     static constexpr size_t smem =
@@ -83,24 +83,76 @@ __device__ __forceinline__ df df_sum(df a, float f, df b) {
     return a;
 }
 
+// Two FP32 values in a register pair: one issue slot does both (the FP32
+// pipes take the same time, but two warps per scheduler cannot issue enough
+// single operations to fill them).
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 f2_pack(float x, float y) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 f2_unpack(f2 a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+    return r;
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f2 f2_neg(f2 a) { return a ^ 0x8000000080000000ull; }
+__device__ __forceinline__ f2 f2_sub(f2 a, f2 b) { return f2_fma(b, f2_pack(-1.f, -1.f), a); }
+
+struct df2 { f2 hi, lo; };       // two double-floats
+__device__ __forceinline__ void df2_chain(df2 &p, df2 s) {
+    const f2 q = f2_mul(p.hi, s.hi);
+    f2 e = f2_fma(p.hi, s.hi, f2_neg(q));
+    e = f2_fma(p.hi, s.lo, e);
+    p.lo = f2_fma(p.lo, s.hi, e);
+    p.hi = q;
+}
+__device__ __forceinline__ df2 df2_renorm(df2 a) {
+    const f2 h = f2_add(a.hi, a.lo);
+    return df2{h, f2_sub(a.lo, f2_sub(h, a.hi))};
+}
+__device__ __forceinline__ f2 f2_shfl_xor(f2 a, int off) {
+    const float2 v = f2_unpack(a);
+    return f2_pack(__shfl_xor_sync(0xffffffffu, v.x, off), __shfl_xor_sync(0xffffffffu, v.y, off));
+}
+__device__ __forceinline__ df2 df2_shfl_xor(df2 a, int off) {
+    return df2{f2_shfl_xor(a.hi, off), f2_shfl_xor(a.lo, off)};
+}
+
 template <int N>
 __global__ void __launch_bounds__(32 * GRAD_WARPS, 2) glynn_gradient_kernel(GradArgs a) {
     using S = GradShape<N>;
     constexpr int P = S::P, RW = S::RW, RP = S::RP, COL = S::COL, WK = S::WK, LW = S::LW;
-    constexpr int BL = fwd_bound_log(false), T = 32 * GRAD_WARPS;
+    constexpr int BL = fwd_bound_log(false), BT = 32 * GRAD_WARPS;
     extern __shared__ float4 grad_smem[];
     float *tab = reinterpret_cast<float *>(grad_smem);   // [N][P][3][RP]; column N-1: all-plus sums
     __shared__ int row_exp[N];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int p = lane & (P - 1), w = lane >> S::LP;
-    // this thread's column of the slots: slot t, row r at [(t RW + r) T]
+    // this thread's column of the slots: slot t, row r at [(t RW + r) BT]
     float2 *mine = reinterpret_cast<float2 *>(tab + N * COL) + threadIdx.x;
     const float2 *warp0 = mine - lane;
     const int b = blockIdx.x / a.blocks_per, part = blockIdx.x - b * a.blocks_per;
     const double *A = a.A + (size_t)b * N * N;
-    for (int r = threadIdx.x; r < N; r += T) row_exp[r] = fwd_row_exponent(A + r * N, nullptr, N, BL);
+    for (int r = threadIdx.x; r < N; r += BT) row_exp[r] = fwd_row_exponent(A + r * N, nullptr, N, BL);
     __syncthreads();
-    for (int idx = threadIdx.x; idx < N * P * RP; idx += T) {
+    for (int idx = threadIdx.x; idx < N * P * RP; idx += BT) {
         const int j = idx / (P * RP), q = idx - j * (P * RP), lp = q / RP, r = q - lp * RP;
         float *t = tab + j * COL + lp * 3 * RP + r;
         const int row = lp * RW + r;
@@ -113,7 +165,7 @@ __global__ void __launch_bounds__(32 * GRAD_WARPS, 2) glynn_gradient_kernel(Grad
         }
     }
     __syncthreads();
-    for (int idx = threadIdx.x; idx < COL; idx += T) {
+    for (int idx = threadIdx.x; idx < COL; idx += BT) {
         float sum = tab[(N - 1) * COL + idx];
         for (int j = 0; j < N - 1; j++) {
             const float v = tab[j * COL + idx];
@@ -125,8 +177,8 @@ __global__ void __launch_bounds__(32 * GRAD_WARPS, 2) glynn_gradient_kernel(Grad
     __syncthreads();
 
     const int R = a.log_range, M = R < GRAD_TREE ? R : GRAD_TREE;
-    // below 2^LW states (N - 1 < LW) the walkers beyond them are idle
-    const bool active = N - 1 >= LW || w < (1 << (N - 1));
+    // where there are fewer ranges than walkers the others are idle
+    const bool active = N - 1 - R >= LW || w < (1 << (N - 1 - R));
     const uint64_t states = 1ull << (N - 1);
     const uint64_t tasks = states >> R >> LW ? states >> R >> LW : 1;
     double *slot = a.slots + ((size_t)blockIdx.x * GRAD_WARPS + warp) * grad_slot(N);
@@ -139,34 +191,42 @@ __global__ void __launch_bounds__(32 * GRAD_WARPS, 2) glynn_gradient_kernel(Grad
     for (uint64_t k = first; k < tasks; k += (uint64_t)a.blocks_per * GRAD_WARPS) {
         if (k != first && *a.abort_flag) { aborted = true; break; }
         const uint64_t g0 = active ? ((k << LW) + w) << R : 0;
-        float s[3][RW];
-        auto load = [&](const float *col, int c, int v) {
-            return reinterpret_cast<const float4 *>(col + c * RP)[v];
-        };
-#pragma unroll
-        for (int c = 0; c < 3; c++)
-#pragma unroll
-            for (int v = 0; v < RP / 4; v++) {
-                const float4 x = load(own + (N - 1) * COL, c, v);
-                s[c][4 * v] = x.x;
-                if (4 * v + 1 < RW) s[c][4 * v + 1] = x.y;
-                if (4 * v + 2 < RW) s[c][4 * v + 2] = x.z;
-                if (4 * v + 3 < RW) s[c][4 * v + 3] = x.w;
-            }
-        auto step = [&](int j, float f) {
+        // row sums of two states: u (column 0 plus) and v (column 0 minus)
+        f2 s[3][RW];
+        auto column = [&](int j, float (&x)[3][RW]) {
 #pragma unroll
             for (int c = 0; c < 3; c++)
 #pragma unroll
                 for (int v = 0; v < RP / 4; v++) {
-                    const float4 x = load(own + j * COL, c, v);
-                    s[c][4 * v] = fmaf(f, x.x, s[c][4 * v]);
-                    if (4 * v + 1 < RW) s[c][4 * v + 1] = fmaf(f, x.y, s[c][4 * v + 1]);
-                    if (4 * v + 2 < RW) s[c][4 * v + 2] = fmaf(f, x.z, s[c][4 * v + 2]);
-                    if (4 * v + 3 < RW) s[c][4 * v + 3] = fmaf(f, x.w, s[c][4 * v + 3]);
+                    const float4 q = reinterpret_cast<const float4 *>(own + j * COL + c * RP)[v];
+                    x[c][4 * v] = q.x;
+                    if (4 * v + 1 < RW) x[c][4 * v + 1] = q.y;
+                    if (4 * v + 2 < RW) x[c][4 * v + 2] = q.z;
+                    if (4 * v + 3 < RW) x[c][4 * v + 3] = q.w;
                 }
         };
+        auto step = [&](int j, float f) {
+            float x[3][RW];
+            column(j, x);
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+#pragma unroll
+                for (int r = 0; r < RW; r++) {
+                    const float2 t = f2_unpack(s[c][r]);
+                    s[c][r] = f2_pack(fmaf(f, x[c][r], t.x), fmaf(f, x[c][r], t.y));
+                }
+        };
+        {
+            float x[3][RW], y[3][RW];
+            column(N - 1, x);
+            column(0, y);
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+#pragma unroll
+                for (int r = 0; r < RW; r++) s[c][r] = f2_pack(x[c][r], x[c][r] - y[c][r]);
+        }
         const uint64_t gr = g0 ^ (g0 >> 1);
-        for (int j = 0; j < N - 1; j++)
+        for (int j = 1; j < N - 1; j++)
             if (__any_sync(0xffffffffu, (gr >> j) & 1)) step(j, ((gr >> j) & 1) ? -1.f : 0.f);
 
         df V0[RW], WT[RW];
@@ -178,101 +238,91 @@ __global__ void __launch_bounds__(32 * GRAD_WARPS, 2) glynn_gradient_kernel(Grad
         }
         for (int t = 1; t < R; t++)
 #pragma unroll
-            for (int r = 0; r < RW; r++) mine[(t * RW + r) * T] = make_float2(0.f, 0.f);
+            for (int r = 0; r < RW; r++) mine[(t * RW + r) * BT] = make_float2(0.f, 0.f);
 
-        // E[r] of the current state
-        auto products = [&](df *E) {
-            df x[RW], pre[RW];          // pre[r] = x[0] ... x[r]
-#pragma unroll
-            for (int r = 0; r < RW; r++) {
-                const float h = s[0][r] + s[1][r];
-                x[r] = df{h, (s[1][r] - (h - s[0][r])) + s[2][r]};
-                pre[r] = x[r];
-                if (r > 0) {
-                    pre[r] = pre[r - 1];
-                    df_chain(pre[r], x[r]);
-                }
-            }
-            // q: the other lanes' product
-            df q = df{1.f, 0.f};
-            if constexpr (P > 1) {
-                df own = df_renorm(pre[RW - 1]);
-                q = df_shfl_xor(own, 1);
-                if constexpr (P > 2) {
-                    df_chain(own, q);
-                    df_chain(q, df_shfl_xor(df_renorm(own), 2));
-                    q = df_renorm(q);
-                }
-            }
-#pragma unroll
-            for (int r = RW - 1; r > 0; r--) {
-                if (P == 1 && r == RW - 1) {
-                    E[r] = pre[r - 1];
-                    q = x[r];
-                } else {
-                    E[r] = pre[r - 1];
-                    df_chain(E[r], q);
-                    df_chain(q, x[r]);
-                }
-            }
-            E[0] = q;
-#pragma unroll
-            for (int r = 0; r < RW; r++) ga[r] += fabsf(E[r].hi);
-        };
-
-        df Ea[RW];
-        if (R == 0) {
-            const float f = (g0 & 1) ? -1.f : 1.f;
-            products(Ea);
-#pragma unroll
-            for (int r = 0; r < RW; r++) df_accumulate(WT[r], f, Ea[r]);
-        }
-        for (uint32_t i = 0; i < (1u << R) >> 1 << 1; i += 2) {
+        // states g0 + i and g0 + i + 1 together: u and v share every sign but
+        // column 0's, which costs no update
+        for (uint32_t i = 0; i < (1u << R); i += 2) {
             const uint64_t g = g0 + i;
             if (i) {
                 const int j = __ffs(i) - 1;
                 step(j, ((g >> (j + 1)) & 1) ? 1.f : -1.f);
             }
-            products(Ea);
-            step(0, ((g >> 1) & 1) ? 1.f : -1.f);
-            df Eb[RW];
-            products(Eb);
-            const float f0 = ((g >> 1) & 1) ? -1.f : 1.f;
+            // E_r of both: prefix products, the other lanes' product, suffix pass
+            df2 x[RW], pre[RW];
 #pragma unroll
             for (int r = 0; r < RW; r++) {
-                df_accumulate(V0[r], f0, df_sum(Ea[r], 1.f, Eb[r]));
-                Ea[r] = df_sum(Ea[r], -1.f, Eb[r]);
+                const f2 h = f2_add(s[0][r], s[1][r]);
+                x[r] = df2{h, f2_add(f2_sub(s[1][r], f2_sub(h, s[0][r])), s[2][r])};
+                pre[r] = x[r];
+                if (r > 0) {
+                    pre[r] = pre[r - 1];
+                    df2_chain(pre[r], x[r]);
+                }
             }
-            // Ea: the sum of this pair; join it with the waiting sums
+            df2 q = x[RW - 1];
+            if constexpr (P > 1) {
+                df2 mine2 = df2_renorm(pre[RW - 1]);
+                q = df2_shfl_xor(mine2, 1);
+                if constexpr (P > 2) {
+                    df2_chain(mine2, q);
+                    df2_chain(q, df2_shfl_xor(df2_renorm(mine2), 2));
+                    q = df2_renorm(q);
+                }
+            }
+            // with p = (-1)^(minus signs but column 0's): w is p E_u and -p E_v,
+            // so column 0 takes p (E_u + E_v); T = E_u - E_v goes up the tree
+            const float p0 = ((g >> 1) & 1) ? -1.f : 1.f;
+            df T[RW];
+#pragma unroll
+            for (int r = RW - 1; r >= 0; r--) {
+                df2 E;
+                if (r == 0) {
+                    E = q;
+                } else if (P == 1 && r == RW - 1) {
+                    E = pre[r - 1];
+                } else {
+                    E = pre[r - 1];
+                    df2_chain(E, q);
+                    df2_chain(q, x[r]);
+                }
+                const float2 h = f2_unpack(E.hi), l = f2_unpack(E.lo);
+                const df u = df{h.x, l.x}, v = df{h.y, l.y};
+                ga[r] += fabsf(u.hi) + fabsf(v.hi);
+                df_accumulate(V0[r], p0, df_sum(u, 1.f, v));
+                T[r] = df_sum(u, -1.f, v);
+            }
+            // Join T with the waiting sums.  On the first level the two pairs
+            // have opposite p (the earlier one +), above it sums are signed.
             int t = 1;
             for (; t < M && ((i >> t) & 1); t++) {
-                const float f = ((g >> (t + 1)) & 1) ? -1.f : 1.f;
+                const float f = ((g >> (t + 1)) & 1) ? -1.f : 1.f, e = t == 1 ? -1.f : 1.f;
 #pragma unroll
                 for (int r = 0; r < RW; r++) {
-                    const float2 hv = mine[((S::RMAX + t - 1) * RW + r) * T];
-                    float2 &vv = mine[(t * RW + r) * T];
+                    const float2 hv = mine[((S::RMAX + t - 1) * RW + r) * BT];
+                    float2 &vv = mine[(t * RW + r) * BT];
                     const df h = df{hv.x, hv.y};
                     df v = df{vv.x, vv.y};
-                    df_accumulate(v, f, df_sum(h, -1.f, Ea[r]));
+                    df_accumulate(v, f, df_sum(h, -e, T[r]));
                     vv = make_float2(v.hi, v.lo);
-                    Ea[r] = df_sum(h, 1.f, Ea[r]);
+                    T[r] = df_sum(h, e, T[r]);
                 }
             }
             if (t < M) {
 #pragma unroll
                 for (int r = 0; r < RW; r++)
-                    mine[((S::RMAX + t - 1) * RW + r) * T] = make_float2(Ea[r].hi, Ea[r].lo);
+                    mine[((S::RMAX + t - 1) * RW + r) * BT] = make_float2(T[r].hi, T[r].lo);
             } else {
 #pragma unroll
-                for (int r = 0; r < RW; r++) df_accumulate(WT[r], 1.f, Ea[r]);
+                for (int r = 0; r < RW; r++) df_accumulate(WT[r], M == 1 ? p0 : 1.f, T[r]);
                 const uint64_t gm = g ^ (g >> 1);
                 for (t = M; t < R; t++) {
                     const float f = ((gm >> t) & 1) ? -1.f : 1.f;
 #pragma unroll
                     for (int r = 0; r < RW; r++) {
-                        float2 &vv = mine[(t * RW + r) * T];
+                        float2 &vv = mine[(t * RW + r) * BT];
                         df v = df{vv.x, vv.y};
-                        df_accumulate(v, f, Ea[r]);
+                        df_accumulate(v, f, T[r]);
                         vv = make_float2(v.hi, v.lo);
                     }
                 }
@@ -296,9 +346,9 @@ __global__ void __launch_bounds__(32 * GRAD_WARPS, 2) glynn_gradient_kernel(Grad
 #pragma unroll
         for (int r = 0; r < RW; r++) {
             for (int t = 0; t < R + LW + 1; t++) {
-                float2 &vv = mine[((t < R ? t : S::RMAX + t - R) * RW + r) * T];
+                float2 &vv = mine[((t < R ? t : S::RMAX + t - R) * RW + r) * BT];
                 const bool neg = t >= R && t < R + LW && ((gw >> t) & 1);
-                const df v = total(t == 0 && R > 0 ? V0[r] : t < R ? df{vv.x, vv.y} : WT[r],
+                const df v = total(t == 0 ? V0[r] : t < R ? df{vv.x, vv.y} : WT[r],
                                    neg ? -1.f : 1.f);
                 if (w == 0) vv = make_float2(v.hi, v.lo);
             }
@@ -308,7 +358,7 @@ __global__ void __launch_bounds__(32 * GRAD_WARPS, 2) glynn_gradient_kernel(Grad
         for (int e = lane; e < N * N; e += 32) {
             const int i = e / N, j = e - i * N, rr = i % RW, ln = i / RW;
             const int t = j == N - 1 || j >= R + LW ? S::RMAX + LW : j < R ? j : S::RMAX + j - R;
-            const float2 v = warp0[(t * RW + rr) * T + ln];
+            const float2 v = warp0[(t * RW + rr) * BT + ln];
             double x = (double)v.x + (double)v.y;
             if (j < N - 1 && j >= R + LW && ((gtm >> j) & 1)) x = -x;
             double sm = slot[e], cp = slot[N * N + e];
