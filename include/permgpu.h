@@ -147,7 +147,7 @@ int pg_affine_residues_partial(const int64_t *C, const int64_t *L, int n,
 
 /*
  * Permanent modulo 3 (*out in {0, 1, 2}) by Glynn's formula over F_3 with
- * table lookups over 1024 states, 0 <= n < 64, any int64 entries.  Replaces
+ * table lookups over 2048 states, 0 <= n < 64, any int64 entries.  Replaces
  * permanent_mod3_matrix (perm_mod3_cuda.cu:300-349) and the OpenMP
  * perm_mod3_omp.permanent_mod3 behind perm_mod3.permanent_mod3_fast
  * (perm_mod3.py:355-383).

@@ -1,4 +1,4 @@
-// Permanent modulo 3 by Glynn's formula with table lookups over 1024 states.
+// Permanent modulo 3 by Glynn's formula with table lookups over 2048 states.
 //
 //   per(A) = 2^(1-n) sum_d (prod_k d_k) prod_i s_i(d)   over F_3,
 // s_i(d) = sum_j d_j a_ij, last sign fixed: 2^(n-1) sign vectors (2 is a unit
@@ -12,25 +12,26 @@
 //
 // A term counts only when no row sum is zero, about (2/3)^n of the states
 // for random entries, so the walk is a search for states without a zero row.
-// The low ten columns' signs are spread over a warp: bit k of lane l's word is
-// the state with low signs (k | l << 5).  The high columns are common to the
-// warp, so row i's sum is h_i + low_i(lane, bit), and "row i is nonzero" is a
-// word that depends only on the lane and on h_i in {0, 1, 2}.  For groups of
-// four rows the 81 AND-ed words per lane sit in shared memory ([81][32] words,
-// lane-minor: no bank conflicts).  One high state (1024 sign vectors) is five
-// loads and ANDs for the first 20 rows; (2/3)^20 of the states, about one in
-// four warps, go on to the next groups, and only states with every row
-// nonzero read the rows' sign words.  The 32 lanes hold the high row sums of
-// 32 consecutive high states (row-sliced, one column update per 32 of them)
-// and publish their table offsets through shared memory.
+// The low eleven columns' signs are spread over a warp: bit k of word h of
+// lane l is the state with low signs (k | l << 5 | h << 10).  The high
+// columns are common to the warp, so row i's sum is h_i + low_i(lane, h, bit),
+// and "row i is nonzero" is a pair of words that depends only on the lane and
+// on h_i in {0, 1, 2}.  For the first six groups of four rows (five up to
+// order 20 and above 52) the 81 AND-ed pairs per lane sit in shared memory
+// ([81][32] pairs, lane-minor: no bank conflicts): one high state (2048 sign
+// vectors) is six 8-byte loads and ANDs for the first 24 rows.  (2/3)^24 of
+// the states, in one of eight high states, go on row by row, and only states
+// with every row nonzero read the rows' sign words.  The 32 lanes hold the
+// high row sums of 32 consecutive high states (row-sliced, one column update
+// per 32 of them) and publish their table offsets through shared memory.
 //
-// Bound by shared-memory loads: 6 loads and ~20 instructions per 1024 states.
-// 35 x 35 random: 22.9 ms a call with the row-sliced Ryser walk (17.5 instructions
-// per subset, ALU pipe 91 % busy), 0.67 ms now (whole call).  Groups of five rows (243
-// words per lane) need 31 KB each and do not fit from order 36 on.  A matrix
-// whose states all survive (equal rows) reads every row's sign word for
-// every high state: ~10 instructions per row and 1024 states, still well
-// below the row-sliced walk, so no other path is kept.
+// Bound by shared-memory loads (95 % of their rate): 17 wavefronts per 2048
+// states.  35 x 35 random, a call: 22.9 ms with the row-sliced Ryser walk
+// (17.5 instructions per subset, ALU pipe 91 % busy), 0.67 ms with single
+// words and tables for every row group, 0.66 with five groups, 0.52 now.  A
+// matrix whose states all survive (equal rows) reads every row's words for
+// every high state, ~14 instructions per row and 2048 states, still well below
+// the row-sliced walk, so no other path is kept.
 #include "pg_internal.h"
 
 #include <cstring>
@@ -38,8 +39,7 @@
 namespace pg {
 
 constexpr int MOD3_THREADS = 1024;   // one block per SM: the tables take up to 212 KB
-constexpr int MOD3_LOW = 10;         // columns spread over word bits (5) and lanes (5)
-constexpr int MOD3_FIRST = 5;        // row groups looked up before the first vote
+constexpr int MOD3_LOW = 11;         // columns over word bits (5), lanes (5) and words (1)
 constexpr int MOD3_DIGITS = 81;      // states of a group of four rows' high sums
 
 struct Mod3Args {
@@ -52,17 +52,12 @@ struct Mod3Args {
     volatile const int *abort_flag;
 };
 
-__host__ __device__ constexpr int mod3_groups(int n) {
-    return (n + 3) / 4 < MOD3_FIRST ? MOD3_FIRST : (n + 3) / 4;
-}
-// per-row words [n][3][32]; the magnitude words' space later holds the warps'
-// offset lists (one uint4 per high state)
-__host__ __device__ constexpr size_t mod3_row_bytes(int n) { return (size_t)n * 3 * 32 * 4; }
-__host__ __device__ constexpr size_t mod3_list_bytes(int n) {
-    return mod3_row_bytes(n) > MOD3_THREADS * 16 ? mod3_row_bytes(n) : MOD3_THREADS * 16;
-}
+// row groups with tables: six (24 rows) where rows and memory allow, else five
+__host__ __device__ constexpr int mod3_tables(int n) { return n > 20 && n <= 52 ? 6 : 5; }
+// per-row words [n][3][32] pairs; the lists hold six offsets a high state
+__host__ __device__ constexpr size_t mod3_row_bytes(int n) { return (size_t)n * 3 * 32 * 8; }
 __host__ __device__ constexpr size_t mod3_smem(int n) {
-    return (size_t)mod3_groups(n) * MOD3_DIGITS * 128 + mod3_row_bytes(n) + mod3_list_bytes(n);
+    return (size_t)mod3_tables(n) * MOD3_DIGITS * 256 + 2 * mod3_row_bytes(n) + MOD3_THREADS * 24;
 }
 
 // row sums (m, s) += or -= column (cm, cs) over F_3, bitwise per row
@@ -87,14 +82,15 @@ __device__ __forceinline__ uint32_t mod3_pattern(int j) {
          : j == 3 ? 0xff00ff00u : 0xffff0000u;
 }
 
-template <typename W>
+template <typename W, int GT>
 __global__ void __launch_bounds__(MOD3_THREADS, 1) mod3_kernel(Mod3Args a) {
     extern __shared__ uint4 mod3_shared[];
-    const int n = a.n, G = mod3_groups(n);
-    uint32_t *gtab = reinterpret_cast<uint32_t *>(mod3_shared);      // [G][81][32]
-    uint32_t *rsgn = gtab + (size_t)G * MOD3_DIGITS * 32;             // [n][3][32]
-    uint32_t *rmag = rsgn + (size_t)n * 96;                           // [n][3][32], build only
-    uint4 *lists = reinterpret_cast<uint4 *>(rmag);                   // [warps][32]
+    const int n = a.n;
+    uint2 *gtab = reinterpret_cast<uint2 *>(mod3_shared);            // [GT][81][32]
+    uint2 *rsgn = gtab + GT * MOD3_DIGITS * 32;              // [n][3][32]
+    uint2 *rmag = rsgn + (size_t)n * 96;                             // [n][3][32]
+    uint4 *lists = reinterpret_cast<uint4 *>(rmag + (size_t)n * 96); // [warps][32]
+    uint2 *lists2 = reinterpret_cast<uint2 *>(lists + MOD3_THREADS);
     __shared__ uint16_t dmap[256];      // (magnitudes | signs << 4) -> byte offset in a group
     __shared__ uint64_t cm_s[64], cs_s[64];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = MOD3_THREADS / 32;
@@ -106,41 +102,54 @@ __global__ void __launch_bounds__(MOD3_THREADS, 1) mod3_kernel(Mod3Args a) {
         int idx = 0, p3 = 1;
         for (int t = 0; t < 4; t++, p3 *= 3)
             if ((threadIdx.x >> t) & 1) idx += p3 * (1 + ((threadIdx.x >> (t + 4)) & 1));
-        dmap[threadIdx.x] = (uint16_t)(idx * 128);
+        dmap[threadIdx.x] = (uint16_t)(idx * 256);
     }
     __syncthreads();
     const int low = n - 1 < MOD3_LOW ? n - 1 : MOD3_LOW;
     for (int r = warp; r < n; r += warps) {
         uint32_t m = 0, s = 0;
-        for (int j = 0; j < low; j++) {
+        for (int j = 0; j < low && j < 10; j++) {
             if (!((cm_s[j] >> r) & 1)) continue;
             const uint32_t minus = j < 5 ? mod3_pattern(j) : 0u - ((lane >> (j - 5)) & 1u);
             f3_add(m, s, 0xffffffffu, ((cs_s[j] >> r) & 1) ? ~minus : minus);
         }
+        // word 0: column 10 plus, word 1: minus
+        const uint32_t cm = low > 10 && ((cm_s[10] >> r) & 1) ? 0xffffffffu : 0u;
+        const uint32_t cs = cm && ((cs_s[10] >> r) & 1) ? 0xffffffffu : 0u;
+        uint32_t m1 = m, s1 = s;
+        f3_add(m, s, cm, cs);
+        f3_sub(m1, s1, cm, cs);
         for (int d = 0; d < 3; d++) {
-            uint32_t md = m, sd = s;
-            if (d) f3_add(md, sd, 0xffffffffu, d == 2 ? 0xffffffffu : 0u);
-            rmag[(r * 3 + d) * 32 + lane] = md;
-            rsgn[(r * 3 + d) * 32 + lane] = sd;
+            uint32_t a0 = m, b0 = s, a1 = m1, b1 = s1;
+            if (d) {
+                f3_add(a0, b0, 0xffffffffu, d == 2 ? 0xffffffffu : 0u);
+                f3_add(a1, b1, 0xffffffffu, d == 2 ? 0xffffffffu : 0u);
+            }
+            rmag[(r * 3 + d) * 32 + lane] = make_uint2(a0, a1);
+            rsgn[(r * 3 + d) * 32 + lane] = make_uint2(b0, b1);
         }
     }
     __syncthreads();
-    for (int e = warp; e < G * MOD3_DIGITS; e += warps) {
+    for (int e = warp; e < GT * MOD3_DIGITS; e += warps) {
         const int g = e / MOD3_DIGITS;
         int d = e - g * MOD3_DIGITS;
-        uint32_t w = 0xffffffffu;
+        uint2 w = make_uint2(0xffffffffu, 0xffffffffu);
         for (int t = 0; t < 4; t++, d /= 3) {
             const int r = 4 * g + t;
-            if (r < n) w &= rmag[(r * 3 + d % 3) * 32 + lane];
+            if (r >= n) continue;
+            const uint2 x = rmag[(r * 3 + d % 3) * 32 + lane];
+            w.x &= x.x;
+            w.y &= x.y;
         }
         gtab[e * 32 + lane] = w;
     }
     __syncthreads();
 
-    // low states that exist (n - 1 < 10: fewer lanes or word bits) and those
-    // with an odd number of minus signs
+    // low states that exist (n - 1 < 11: fewer words, lanes or word bits) and
+    // those with an odd number of minus signs in word 0
     const uint32_t exist = low < 5 ? (lane == 0 ? (1u << (1 << low)) - 1u : 0u)
-                                   : (lane < (1 << (low - 5)) ? 0xffffffffu : 0u);
+                           : low < 10 ? (lane < (1 << (low - 5)) ? 0xffffffffu : 0u) : 0xffffffffu;
+    const uint32_t exist1 = low > 10 ? 0xffffffffu : 0u;
     const uint32_t odd = 0x96696996u ^ (0u - (__popc(lane) & 1u));
 
     // one contiguous, balanced range of batches per warp
@@ -148,12 +157,13 @@ __global__ void __launch_bounds__(MOD3_THREADS, 1) mod3_kernel(Mod3Args a) {
     const uint64_t wid = (uint64_t)blockIdx.x * warps + warp;
     const uint64_t b_begin = wid * a.batches / TW, b_end = (wid + 1) * a.batches / TW;
     const char *tab = reinterpret_cast<const char *>(gtab + lane);
-    constexpr int GB = MOD3_DIGITS * 128;
+    constexpr int GB = MOD3_DIGITS * 256;
     uint4 *list = lists + warp * 32;
+    uint2 *list2 = lists2 + warp * 32;
     unsigned long long count = 0;   // sum of 1 (term +1) or 2 (term -1)
     bool aborted = false;
     // high signs of lane l in batch b: l | gray(b) << 5, bit t the sign of
-    // column 10 + t; the last column's sign is +
+    // column 11 + t; the last column's sign is +
     W m = 0, s = 0;
     if (b_begin < b_end) {
         m = (W)cm_s[n - 1];
@@ -165,21 +175,28 @@ __global__ void __launch_bounds__(MOD3_THREADS, 1) mod3_kernel(Mod3Args a) {
         }
     }
 
-    // The states `alive` of high state k after the first groups: the other
-    // groups, then the signs.  Everything but the words is warp-uniform.
-    auto finish = [&](int k, uint32_t alive, uint32_t flip) {
+    // The states `alive` of high state k after the first 20 rows: the other
+    // rows, then the signs.  Everything but the words is warp-uniform.
+    auto finish = [&](int k, uint2 alive, uint32_t flip) {
         const W km = __shfl_sync(0xffffffffu, m, k), ks = __shfl_sync(0xffffffffu, s, k);
-        for (int g = MOD3_FIRST; g < G; g++) {
-            const uint32_t e = (uint32_t)((km >> (4 * g)) & 15) | (uint32_t)((ks >> (4 * g)) & 15) << 4;
-            alive &= *reinterpret_cast<const uint32_t *>(tab + g * GB + dmap[e]);
-            if (!__any_sync(0xffffffffu, alive != 0)) return;
+        const auto digit = [&](int r) { return ((km >> r) & 1) ? 1 + (int)((ks >> r) & 1) : 0; };
+        for (int r = 4 * GT; r < n; r += 2) {
+            const int q = r + 1 < n ? r + 1 : r;
+            const uint2 x = rmag[(r * 3 + digit(r)) * 32 + lane], y = rmag[(q * 3 + digit(q)) * 32 + lane];
+            alive.x &= x.x & y.x;
+            alive.y &= x.y & y.y;
+            if (!__any_sync(0xffffffffu, (alive.x | alive.y) != 0)) return;
         }
-        uint32_t neg = odd ^ flip ^ (0u - (__popc(k) & 1u));
+        uint2 neg;
+        neg.x = odd ^ flip ^ (0u - (__popc(k) & 1u));
+        neg.y = ~neg.x;
         for (int r = 0; r < n; r++) {
-            const int d = ((km >> r) & 1) ? 1 + (int)((ks >> r) & 1) : 0;
-            neg ^= rsgn[(r * 3 + d) * 32 + lane];
+            const uint2 x = rsgn[(r * 3 + digit(r)) * 32 + lane];
+            neg.x ^= x.x;
+            neg.y ^= x.y;
         }
-        count += (unsigned long long)(__popc(alive) + __popc(alive & neg));
+        count += (unsigned long long)(__popc(alive.x) + __popc(alive.x & neg.x) + __popc(alive.y) +
+                                      __popc(alive.y & neg.y));
     };
 
     for (uint64_t b = b_begin; b < b_end; b++) {
@@ -195,29 +212,35 @@ __global__ void __launch_bounds__(MOD3_THREADS, 1) mod3_kernel(Mod3Args a) {
             if (((b >> (z + 1)) & 1) == 0) f3_add(m, s, (W)cm_s[j], (W)cs_s[j]);
             else f3_sub(m, s, (W)cm_s[j], (W)cs_s[j]);
         }
-        uint32_t off[MOD3_FIRST];
+        uint32_t off[GT];
 #pragma unroll
-        for (int g = 0; g < MOD3_FIRST; g++)
+        for (int g = 0; g < GT; g++)
             off[g] = dmap[(uint32_t)((m >> (4 * g)) & 15) | (uint32_t)((s >> (4 * g)) & 15) << 4];
-        list[lane] = make_uint4(off[0] | off[1] << 16, off[2] | off[3] << 16, off[4], 0);
+        list[lane] = make_uint4(off[0], off[1] + GB, off[2] + 2 * GB, off[3] + 3 * GB);
+        list2[lane] = make_uint2(off[4] + 4 * GB, GT > 5 ? off[GT - 1] + (GT - 1) * GB : 0);
         __syncwarp();
         const uint32_t flip = 0u - (uint32_t)(b & 1);     // parity of gray(b)
         for (int k0 = 0; k0 < a.steps; k0 += 4) {
-            uint32_t alive[4];
+            uint2 alive[4];
 #pragma unroll
             for (int t = 0; t < 4; t++) {
-                // beyond a.steps (below order 13) the list still holds valid offsets
+                // beyond a.steps (below order 14) the list still holds valid offsets
                 const uint4 o = list[k0 + t];
-                const auto at = [&](int g, uint32_t off) {
-                    return *reinterpret_cast<const uint32_t *>(tab + g * GB + off);
-                };
-                alive[t] = at(0, o.x & 0xffffu) & at(1, o.x >> 16) & at(2, o.y & 0xffffu) &
-                           at(3, o.y >> 16) & at(4, o.z);
+                const auto at = [&](uint32_t off) { return *reinterpret_cast<const uint2 *>(tab + off); };
+                const uint2 z0 = at(o.x), z1 = at(o.y), z2 = at(o.z), z3 = at(o.w);
+                const uint2 p = list2[k0 + t], z4 = at(p.x);
+                alive[t].x = z0.x & z1.x & z2.x & z3.x & z4.x & exist;
+                alive[t].y = z0.y & z1.y & z2.y & z3.y & z4.y & exist1;
+                if constexpr (GT > 5) {
+                    const uint2 z5 = at(p.y);
+                    alive[t].x &= z5.x;
+                    alive[t].y &= z5.y;
+                }
             }
 #pragma unroll
             for (int t = 0; t < 4; t++)
-                if (k0 + t < a.steps && __any_sync(0xffffffffu, (alive[t] & exist) != 0))
-                    finish(k0 + t, alive[t] & exist, flip);
+                if (k0 + t < a.steps && __any_sync(0xffffffffu, (alive[t].x | alive[t].y) != 0))
+                    finish(k0 + t, alive[t], flip);
         }
         __syncwarp();
     }
@@ -238,14 +261,14 @@ __global__ void __launch_bounds__(MOD3_THREADS, 1) mod3_kernel(Mod3Args a) {
     }
 }
 
-template <typename W>
+template <typename W, int GT>
 static cudaError_t launch_mod3(const Mod3Args &a, int sm_count, cudaStream_t s) {
     const size_t smem = mod3_smem(a.n);
-    cudaError_t e = cudaFuncSetAttribute(mod3_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(mod3_kernel<W, GT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
     const uint64_t blocks = a.batches < (uint64_t)sm_count ? a.batches : (uint64_t)sm_count;
-    mod3_kernel<W><<<(unsigned)blocks, MOD3_THREADS, smem, s>>>(a);
+    mod3_kernel<W, GT><<<(unsigned)blocks, MOD3_THREADS, smem, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -276,8 +299,11 @@ static int mod3_impl(const uint64_t *mags, const uint64_t *sgns, int n, int *out
     a.status = (int *)(d + off_status);
     a.abort_flag = abort_dev;
     PG_CUDA(cudaMemcpyAsync(d, h, total, cudaMemcpyHostToDevice, ws->stream));
-    if (n <= 32) PG_CUDA((launch_mod3<uint32_t>(a, dev.sm_count, ws->stream)));
-    else PG_CUDA((launch_mod3<uint64_t>(a, dev.sm_count, ws->stream)));
+    const bool six = mod3_tables(n) == 6;
+    if (n <= 32 && six) PG_CUDA((launch_mod3<uint32_t, 6>(a, dev.sm_count, ws->stream)));
+    else if (n <= 32) PG_CUDA((launch_mod3<uint32_t, 5>(a, dev.sm_count, ws->stream)));
+    else if (six) PG_CUDA((launch_mod3<uint64_t, 6>(a, dev.sm_count, ws->stream)));
+    else PG_CUDA((launch_mod3<uint64_t, 5>(a, dev.sm_count, ws->stream)));
     PG_CUDA(cudaMemcpyAsync(h + off_acc, d + off_acc, total - off_acc, cudaMemcpyDeviceToHost,
                             ws->stream));
     PG_CUDA(cudaStreamSynchronize(ws->stream));
