@@ -183,6 +183,15 @@ int pg_binary_residues(const uint8_t *A, int n, const uint64_t *primes, int k,
  */
 int pg_exact_permanent(const int64_t *A, int n, uint32_t *out, int limbs);
 
+/*
+ * The same for 2 <= n <= 32 and row bounds sum_j |a_ij| < 2^48 (64-bit row
+ * sums; PG_EOVERFLOW beyond).  It takes every such matrix, but those that
+ * pg_exact_permanent accepts run faster there.  Replaces the residue loop of
+ * perm.matrix_permanent(A, method="generic") (perm.py:1076-1212) for entries
+ * beyond 32-bit row sums.
+ */
+int pg_exact_wide(const int64_t *A, int n, uint32_t *out, int limbs);
+
 /* 1 if pg_exact_permanent accepts this matrix (bound fits), else 0. */
 int pg_exact_supported(const int64_t *A, int n);
 

@@ -70,6 +70,7 @@ SIGNATURES = {
                                    ctypes.c_int),
     "pg_binary_residues": ([_c_u8p, ctypes.c_int, _c_u64p, ctypes.c_int, _c_u64p], ctypes.c_int),
     "pg_exact_permanent": ([_c_i64p, ctypes.c_int, _c_u32p, ctypes.c_int], ctypes.c_int),
+    "pg_exact_wide": ([_c_i64p, ctypes.c_int, _c_u32p, ctypes.c_int], ctypes.c_int),
     "pg_exact_supported": ([_c_i64p, ctypes.c_int], ctypes.c_int),
     "pg_exact_plan_create": ([_c_i64p, ctypes.c_int, ctypes.POINTER(ctypes.c_void_p)], ctypes.c_int),
     "pg_exact_plan_launch": ([ctypes.c_void_p, ctypes.c_void_p], ctypes.c_int),
@@ -359,6 +360,14 @@ def exact_permanent(matrix: np.ndarray, limbs: int) -> int:
     out = np.zeros(limbs, dtype=np.uint32)
     check(load().pg_exact_permanent(ptr(a, ctypes.c_int64), a.shape[0],
                                     ptr(out, ctypes.c_uint32), limbs))
+    return limbs_to_int(out)
+
+
+def exact_wide_permanent(matrix: np.ndarray, limbs: int) -> int:
+    """per(matrix) for orders 2..32 and row bounds below 2^48 (pg_exact_wide)."""
+    a = np.ascontiguousarray(matrix, dtype=np.int64)
+    out = np.zeros(limbs, dtype=np.uint32)
+    check(load().pg_exact_wide(ptr(a, ctypes.c_int64), a.shape[0], ptr(out, ctypes.c_uint32), limbs))
     return limbs_to_int(out)
 
 

@@ -8,6 +8,8 @@ Engine choice for integer matrices:
   * exact engine (pg_exact_permanent) whenever every row-sum bound
     sum_j |a_ij| < 2^30 and the order is <= 48: one traversal, exact integer
     row sums, exact multi-word Glynn terms, no CRT;
+  * the 64-bit exact engine (pg_exact_wide) for row-sum bounds < 2^48 and
+    orders <= 32;
   * otherwise residues modulo descending primes below 2^31 (one launch for
     all primes) and the signed CRT lift of perm.py:1207-1210.
 """
@@ -101,6 +103,11 @@ def matrix_permanent(matrix, verbose: bool = False, parallel: bool = True,
             return _lib.exact_permanent(arr, _lib.exact_limbs(arr))
     if engine == "exact":
         raise ValueError("matrix is outside the exact engine's range")
+    if engine == "auto" and arr is not None and n <= 32 and top < float(1 << 48) - 1024:
+        # rows beyond 32 bits: 64-bit row sums, still one traversal
+        if verbose:
+            print(f"64-bit exact GPU engine, order {n}")
+        return _lib.exact_wide_permanent(arr, _lib.exact_limbs(arr))
     bound = matrix_permanent_bound(rows)
     primes = residue_plan(bound)
     if verbose:

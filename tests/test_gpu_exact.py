@@ -160,3 +160,49 @@ def test_exact_partial_windows_at_the_largest_orders(lib, n, kind):
         v = shard.words_value(shard.exact_partial_words(a, lo, lo + w))
         for p in (2_147_483_647, 1_000_000_007):
             assert v % p == oracle.glynn_range_mod_p(a, p, lo, lo + w), (n, kind, lo, p)
+
+
+@pytest.mark.parametrize("n", [2, 3, 5, 12, 13, 16, 17, 18, 19, 20, 21, 22, 23, 24, 25, 26, 27])
+def test_wide_engine_against_residues(lib, n):
+    # 64-bit row sums: every compiled order and row class (bounds just below
+    # 2^36, 2^40, 2^44, 2^48 and below 2^30) against the residue engine's
+    # CRT value, with zero rows, all-positive rows (the largest products) and
+    # mixed signs
+    import permgpu
+    rng = np.random.default_rng(2200 + n)
+    for bits in (30, 36, 40, 44, 48):
+        top = (1 << bits) - 1
+        a = rng.integers(-(top // n), top // n + 1, (n, n))
+        a[0] = np.abs(a[0])
+        if bits == 40:
+            a = np.full((n, n), top // n)            # every row at its bound
+        want = permgpu.matrix_permanent(a.tolist(), engine="residue")
+        assert lib.exact_wide_permanent(a, lib.exact_limbs(a)) == want, bits
+        if n > 23:
+            break
+    z = rng.integers(-(1 << 40), 1 << 40, (n, n))
+    z[n // 2] = 0
+    assert lib.exact_wide_permanent(z, lib.exact_limbs(z)) == 0
+
+
+@pytest.mark.parametrize("n,bits", [(28, 36), (28, 48), (30, 44), (30, 48), (32, 40), (32, 48)])
+def test_wide_engine_large_orders(lib, n, bits):
+    # per is multilinear in the rows: a small-entry matrix with its rows
+    # multiplied up to the class bound, against the 32-bit engine's value
+    rng = np.random.default_rng(40 * n + bits)
+    a = rng.integers(-8, 9, (n, n))
+    f = ((1 << bits) - 1) // np.maximum(1, np.abs(a).sum(1))
+    want = lib.exact_permanent(a, lib.exact_limbs(a))
+    for v in f:
+        want *= int(v)
+    w = a * f[:, None]
+    assert lib.exact_wide_permanent(w, lib.exact_limbs(w)) == want
+
+
+def test_wide_engine_refuses_wider_rows(lib):
+    a = np.full((4, 4), 1 << 46, dtype=np.int64)
+    with pytest.raises(lib.PermGpuError) as err:
+        lib.exact_wide_permanent(a, 40)
+    assert err.value.status == lib.PG_EOVERFLOW
+    with pytest.raises(lib.PermGpuError):
+        lib.exact_wide_permanent(np.ones((33, 33), np.int64), 40)
