@@ -207,6 +207,9 @@ struct ExactPlan {
     // device side (owned by a plan object, or borrowed from a workspace)
     char *dev = nullptr;
     char *host = nullptr;        // pinned staging, >= total bytes
+    // result words of the finishing kernel: in dev, or (one-shot calls) in
+    // the pinned staging itself, which saves the copy back
+    unsigned long long *out = nullptr;
     bool owns = false;
     cudaStream_t stream = nullptr;
     volatile int *abort_dev = nullptr;
@@ -505,13 +508,13 @@ static int plan_build(const int64_t *A, int n, ExactPlan *P, bool whole = true) 
     return PG_OK;
 }
 
-// Upload tables and zero the accumulators, status and result words
-// (async on P->stream).  Launches re-zero what they use, so this runs once
-// per plan.
+// Upload the tables with the zeroed accumulators, status and result words
+// behind them in one copy (async on P->stream).  The per-block slots need no
+// zeroing: every launch writes them in full.
 static int plan_upload(ExactPlan *P) {
-    std::memcpy(P->host, P->image.data(), P->total);
-    PG_CUDA(cudaMemcpyAsync(P->dev, P->host, P->off_acc, cudaMemcpyHostToDevice, P->stream));
-    PG_CUDA(cudaMemsetAsync(P->dev + P->off_acc, 0, P->total - P->off_acc, P->stream));
+    std::memcpy(P->host, P->image.data(), P->off_part);
+    if (!P->out) P->out = (unsigned long long *)(P->dev + P->off_out);
+    PG_CUDA(cudaMemcpyAsync(P->dev, P->host, P->off_part, cudaMemcpyHostToDevice, P->stream));
     return PG_OK;
 }
 
@@ -548,7 +551,7 @@ static int plan_launch(ExactPlan *P, cudaStream_t stream) {
         while (b.log_unit < 3 && (chunks >> (6 + b.log_unit)) >= 32 * warps) b.log_unit++;
         PG_CUDA(launch_binary_any(P->npad, P->G, b, (int)P->blocks, stream));
         PG_CUDA(exact_finish(b.part, (int)P->blocks, P->NL, b.acc, b.status,
-                             (unsigned long long *)(P->dev + P->off_out), stream, b.next));
+                             P->out, stream, b.next));
         return PG_OK;
     }
     ExactArgs args;
@@ -565,7 +568,7 @@ static int plan_launch(ExactPlan *P, cudaStream_t stream) {
     PG_CUDA(P->fr ? launch_exact_frows(P->n, P->G, P->fr, args, (int)P->blocks, stream)
                   : launch_exact_any(P->n, P->G, args, (int)P->blocks, stream));
     PG_CUDA(exact_finish(args.part, (int)P->blocks, P->NL, args.acc, args.status,
-                         (unsigned long long *)(P->dev + P->off_out), stream));
+                         P->out, stream));
     return PG_OK;
 }
 
@@ -592,8 +595,9 @@ static int plan_finish(ExactPlan *P, cudaStream_t stream, uint32_t *out, int lim
     if (32 * limbs < P->need_bits)
         return fail(PG_ERANGE, "output limb count too small for the permanent bound");
     const int NL = P->NL, W = NL + 3;
-    PG_CUDA(cudaMemcpyAsync(P->host + P->off_out, P->dev + P->off_out, (size_t)(NL + 1) * 8,
-                            cudaMemcpyDeviceToHost, stream));
+    if ((char *)P->out == P->dev + P->off_out)
+        PG_CUDA(cudaMemcpyAsync(P->host + P->off_out, P->out, (size_t)(NL + 1) * 8,
+                                cudaMemcpyDeviceToHost, stream));
     PG_CUDA(cudaStreamSynchronize(stream));
     const long long *acc = (const long long *)(P->host + P->off_out);
     if (acc[NL]) return fail(PG_EABORT, "exact launch aborted by pg_abort()");
@@ -626,6 +630,9 @@ int exact_run(const int64_t *A, int n, uint32_t *out, int limbs) {
     P.dev = (char *)ws->dev;
     P.host = (char *)ws->host;
     P.stream = ws->stream;
+    void *out_dev = nullptr;
+    PG_CUDA(cudaHostGetDevicePointer(&out_dev, P.host + P.off_out, 0));
+    P.out = (unsigned long long *)out_dev;
     if ((st = plan_upload(&P)) != PG_OK) return st;
     if ((st = plan_launch(&P, P.stream)) != PG_OK) return st;
     return plan_finish(&P, P.stream, out, limbs);
