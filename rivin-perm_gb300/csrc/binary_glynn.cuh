@@ -23,9 +23,18 @@
 // lanes prepare the entries of 32 consecutive chunks, whose signs differ in
 // five columns: row counts are bytes, the warp's count minus a 32-row
 // table's, four rows per subtraction.  W = 2 where under 1/64 of the states
-// survive (grid40 34.9 ms, 58.6 with W = 1); else the evaluations need the
+// survive (4x4x5 grid, before the next paragraph's shortcut: 34.9 ms, 58.6
+// with W = 1); else the evaluations need the
 // shared memory and W = 1 is faster (36 x 36 Bernoulli(1/2): 21.3 against
 // 26.7 ms).
+//
+// Rows without ones in the low columns need no table.  Such a row is zero in
+// all of a chunk or none of it, one without ones in the five chunk columns
+// either in all of a batch of 32 chunks or none: they are tested first, one
+// lane a row for the batch and by bytes for the chunk, and a batch or chunk
+// with a zero row is left.  4x4x5 grid 33.5 -> 11.6 ms (with a few bonds
+// removed 34.9 -> 25.7), 6x4x3 5.4 -> 4.2, 8x8 0.17 -> 0.05; dense matrices
+// have no such row and run as before within 1 %.
 //
 // Evaluation.  Surviving states are appended to a per-warp queue; whenever
 // 32 are queued every lane evaluates one exactly.  The row sums come as
@@ -42,7 +51,7 @@
 //
 // Issue bound (65-80 % of the issue slots).  Whole calls against a
 // bit-sliced tracker that updated one state per lane and step and evaluated
-// by popcount: 4x4x5 grid (40 x 40, 0.08 % survive) 441 -> 34.9 ms, 36 x 36
+// by popcount: 4x4x5 grid (40 x 40, 0.08 % survive) 441 -> 11.6 ms, 36 x 36
 // Bernoulli(1/2) (6-13 % survive) 67-76 -> 22-28 ms.
 #pragma once
 
@@ -69,8 +78,11 @@ struct BinTrack {
 struct BinaryArgs {
     const uint64_t *rmask;     // [NPAD] toggled-column bits of each row (group order)
     const int32_t *deg;        // [NPAD] row degrees (pad rows 1)
+    // Even-degree rows: batch rows (no ones below the columns common to a
+    // batch of 32 chunks), then chunk rows (none in the low columns), then
+    // table rows; the first two padded to a multiple of four
     const BinTrack *trk;       // [ntracked]
-    int ntracked;              // even-degree rows, 1..48
+    int batch_rows, uniform_rows, ntracked;   // ends of the three, ntracked <= BIN_TRACK
     int entries;               // table entries (entry 0: no row is zero)
     int list_words;            // words of a chunk's list: the byte offset of each group's
                                // entry, padded with entry 0 to a multiple of four
@@ -95,7 +107,8 @@ __host__ __device__ constexpr int binary_max_threads(int NPAD, int W) {
 }
 // words of a state's row bytes, padded for 8-byte loads
 __host__ __device__ constexpr int binary_row_words(int NPAD) { return (NPAD / 4 + 1) & ~1; }
-constexpr int BIN_TRACK_WORDS = 12;     // bytes of the even-degree rows (at most 48)
+constexpr int BIN_TRACK = 56;           // even-degree rows (at most 48) with their padding
+constexpr int BIN_TRACK_WORDS = BIN_TRACK / 4;
 __host__ __device__ constexpr size_t binary_warp_bytes(int NPAD, int W, int list_words) {
     return (size_t)32 * W * binary_row_words(NPAD) * 4 + (size_t)32 * list_words * 4 + BIN_QCAP * 2 +
            BIN_TRACK_WORDS * 4 + 48;
@@ -133,8 +146,8 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD, W), 1) binary_glynn_k
     uint32_t *ucnt = base + 32 * W * LS;                                // row bytes, then even rows'
     uint32_t *xcnt = ucnt + 12;
     uint16_t *q = reinterpret_cast<uint16_t *>(xcnt + TW);
-    __shared__ BinTrack s_trk[48];
-    __shared__ uint4 s_rec[48];         // cap, stride bytes, group's first byte + 1 on its last row
+    __shared__ BinTrack s_trk[BIN_TRACK];
+    __shared__ uint4 s_rec[BIN_TRACK];         // cap, stride bytes, group's first byte + 1 on its last row
     __shared__ uint64_t s_rm[NPAD];
     __shared__ int32_t s_deg[NPAD];
     __shared__ uint32_t s_eq[32][6];    // [mask][v]: the k in 0..31 with popc(k & mask) == v
@@ -152,7 +165,7 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD, W), 1) binary_glynn_k
     __syncthreads();
     if (warp == 0)
         for (int h = 0; h < W; h++) ztab[lane * W + h] = 0xffffffffu;
-    for (int e0 = 0; e0 < a.ntracked;) {            // table groups
+    for (int e0 = a.uniform_rows; e0 < a.ntracked;) {            // table groups
         int e1 = e0 + 1, size = s_trk[e0].cap + 1;
         for (; e1 < a.ntracked && s_trk[e1].base == 0xffff; e1++) size *= s_trk[e1].cap + 1;
         if ((int)threadIdx.x >= e0 && (int)threadIdx.x < e1)
@@ -315,26 +328,45 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD, W), 1) binary_glynn_k
                                                                              : 1 << a.log_steps;
             const int kfirst = c_lo > c0 ? (c_lo - c0 < (uint64_t)k1 ? (int)(c_lo - c0) : k1) : 0;
             if (kfirst >= k1) continue;
-            // the host-mapped abort word is read once per 128 batches, from
-            // the warp's second period on
-            if ((++polls & 127) == 0 && __any_sync(0xffffffffu, *a.abort_flag != 0)) {
-                aborted = true;
-                break;
+            // the host-mapped abort word is read once per 128 batches that are
+            // searched (4096 that are not), from the warp's second period on
+            if (++polls >= 4096) {
+                polls = 0;
+                if (__any_sync(0xffffffffu, *a.abort_flag != 0)) {
+                    aborted = true;
+                    break;
+                }
             }
-            c_odd = (uint32_t)c0;
-            const bool edge = ((c0 + kfirst) << LOW) < a.state_lo || ((c0 + k1) << LOW) > a.state_hi;
             // the batch's common high signs: gray(c0 >> 5) in columns HI and up
             const uint64_t b5 = c0 >> 5;
             const uint32_t hw = (uint32_t)(b5 ^ (b5 >> 1));
             auto ones = [&](uint64_t m) { return __popc((uint32_t)m & hw); };
-            for (int r = lane; r < NPAD; r += 32)
-                reinterpret_cast<uint8_t *>(ucnt)[r] = (uint8_t)(128 + s_deg[r] - 2 * ones(s_rm[r] >> HI));
-            for (int r = lane; r < a.ntracked; r += 32)
+            // a batch row that is zero now is zero in the whole batch
+            bool dead = false;
+            for (int r = lane; r < a.batch_rows; r += 32)
+                dead |= (int)s_trk[r].half == ones(s_trk[r].high >> 5);
+            if (__any_sync(0xffffffffu, dead)) continue;
+            for (int r = a.batch_rows + lane; r < a.ntracked; r += 32)
                 reinterpret_cast<uint8_t *>(xcnt)[r] = (uint8_t)(128 + s_trk[r].half - ones(s_trk[r].high >> 5));
             __syncwarp();
-            // this lane's chunk: the signs of the five columns below those
+            // this lane's chunk: the signs of the five columns below those; a
+            // chunk row with x = 0 (a zero byte) is zero in the whole chunk
             const uint32_t l5 = ((uint32_t)c0 + lane) & 31u;
             const uint32_t x5 = l5 ^ (l5 >> 1) ^ (((uint32_t)b5 & 1u) << 4);
+            uint32_t zero = 0;
+            for (int e = a.batch_rows >> 2; e < a.uniform_rows >> 2; e++) {
+                const uint32_t x = (xcnt[e] - xtab[x5 * TW + e]) ^ 0x80808080u;
+                zero |= (x - 0x01010101u) & ~x & 0x80808080u;
+            }
+            uint32_t chunks = __ballot_sync(0xffffffffu, zero == 0 && lane >= kfirst && lane < k1);
+            __syncwarp();               // xcnt is read
+            if (!chunks) continue;
+            polls += 31;
+            c_odd = (uint32_t)c0;
+            const bool edge = ((c0 + kfirst) << LOW) < a.state_lo || ((c0 + k1) << LOW) > a.state_hi;
+            for (int r = lane; r < NPAD; r += 32)
+                reinterpret_cast<uint8_t *>(ucnt)[r] = (uint8_t)(128 + s_deg[r] - 2 * ones(s_rm[r] >> HI));
+            __syncwarp();
             {
                 const uint32_t *cb = ctab + x5 * LS;
                 uint32_t *o = base + lane * W * LS;
@@ -349,7 +381,7 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD, W), 1) binary_glynn_k
                 uint32_t *ll = list + lane * a.list_words;
                 int g = 0;
                 uint32_t off = 0;
-                for (int e = 0; e < a.ntracked; e += 4) {
+                for (int e = a.uniform_rows; e < a.ntracked; e += 4) {
                     // bytes of x in two's complement: negative ones exceed every cap
                     const uint32_t x = (xcnt[e >> 2] - xtab[x5 * TW + (e >> 2)]) ^ 0x80808080u;
 #pragma unroll
@@ -366,19 +398,24 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD, W), 1) binary_glynn_k
                 for (; g < a.list_words; g++) ll[g] = 0;
             }
             __syncwarp();
-            for (int k0 = kfirst; k0 < k1; k0 += 2) {
+            while (chunks) {            // two chunks at a time
+                int kk[2];
+                kk[0] = __ffs(chunks) - 1;
+                chunks &= chunks - 1;
+                const bool pair = chunks != 0;
+                kk[1] = pair ? __ffs(chunks) - 1 : kk[0];
+                chunks &= chunks - 1;
                 uint32_t alive[2][W];
 #pragma unroll
-                for (int t = 0; t < 2; t++)
-#pragma unroll
-                    for (int h = 0; h < W; h++) alive[t][h] = k0 + t < k1 ? 0xffffffffu : 0u;
+                for (int h = 0; h < W; h++) {
+                    alive[0][h] = 0xffffffffu;
+                    alive[1][h] = pair ? 0xffffffffu : 0u;
+                }
                 for (int v = 0; v < a.list_words; v += 4) {
                     uint32_t any = 0;
 #pragma unroll
                     for (int t = 0; t < 2; t++) {
-                        // (beyond the batch: row 31, whose words are not used)
-                        const int row = k0 + t < 32 ? k0 + t : 31;
-                        const uint4 o = *reinterpret_cast<const uint4 *>(list + row * a.list_words + v);
+                        const uint4 o = *reinterpret_cast<const uint4 *>(list + kk[t] * a.list_words + v);
                         if constexpr (W > 1) {
                             const auto at = [&](uint32_t off) {
                                 return *reinterpret_cast<const uint2 *>(zl + off);
@@ -402,7 +439,7 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD, W), 1) binary_glynn_k
                     for (int t = 0; t < 2; t++)
 #pragma unroll
                         for (int h = 0; h < W; h++) {
-                            const uint64_t c = c0 + k0 + t;
+                            const uint64_t c = c0 + kk[t];
                             uint32_t in = 0;
                             for (int k = 0; k < 32; k++) {
                                 uint32_t i = (uint32_t)(k | (lane << 5) | (h << 10)) ^
@@ -421,7 +458,7 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD, W), 1) binary_glynn_k
                 for (int t = 0; t < 2; t++)
 #pragma unroll
                     for (int h = 0; h < W; h++)
-                        append(alive[t][h], (uint32_t)((k0 + t) << LOW) | (uint32_t)(h << BIN_TAB));
+                        append(alive[t][h], (uint32_t)(kk[t] << LOW) | (uint32_t)(h << BIN_TAB));
             }
             if (qn > 0) evaluate(qn);       // the next batch has other base bytes
             __syncwarp();
@@ -481,7 +518,7 @@ cudaError_t launch_binary_any(int NPAD, int G, const BinaryArgs &args, int block
 // table groups (a multiple of four where that takes no more lookups) for the
 // tables to fit beside the NPAD kernel's other shared memory, with the most
 // warps that allow it; group[e] = the row's group.  Returns the number of
-// groups, 0 if there is no such packing.
+// groups, -1 if there is no such packing.
 int binary_pack_groups(int NPAD, int W, const int *caps, int rows, int *group, int *warps);
 
 }  // namespace pg

@@ -194,7 +194,7 @@ struct ExactPlan {
     // 0/1 kernel (binary_glynn.cuh): bits of the largest even row's half
     // degree (0: the general kernel), tracked (even-degree) rows, padded
     // rows, table entries and list words, Gray window
-    int planes = 0, ntracked = 0, npad = 0, entries = 0, list_words = 0, warps = 0,
+    int planes = 0, batch_rows = 0, uniform_rows = 0, ntracked = 0, npad = 0, entries = 0, list_words = 0, warps = 0,
         words = 1, sparse = 0;
     size_t off_deg = 0, off_trk = 0;
     uint64_t lo = 0, hi = 0;
@@ -237,6 +237,8 @@ int binary_pack_groups(int NPAD, int W, const int *caps, int rows, int *group, i
     // warps, then the most warps for them; fewer warps only where nothing fits
     const int most = binary_max_threads(NPAD, W) / 32;
     int best = 0;
+    *warps = most;
+    if (rows == 0) return 0;
     for (int w = most; w >= 2 && (w >= BIN_WARPS_MIN || !best); w -= 2)
         for (int T = 4; T < rows + 4 && (!best || T < best); T += 4) {
             const int groups = T < rows ? T : rows;
@@ -244,7 +246,7 @@ int binary_pack_groups(int NPAD, int W, const int *caps, int rows, int *group, i
             best = T;
             *warps = w;
         }
-    if (!best) return 0;
+    if (!best) return -1;
     const int groups = best < rows ? best : rows;
     pack(groups);
     return groups;
@@ -321,24 +323,27 @@ static bool plan_build_binary(const int64_t *A, int n, bool whole, ExactPlan *P)
         if (exact_group_rows(deg.data(), NPAD, g, order.data())) { G = g; break; }
     }
     if (!G) return false;
-    const int nt = (int)tracked.size();
     P->sparse = B.survive * 64 < BINARY_SAMPLES;
     P->words = P->sparse ? 2 : 1;
     const int low = bin_low(P->words);
-    const uint64_t low_mask = (1ull << low) - 1;
+    const uint64_t low_mask = (1ull << low) - 1, batch_mask = (1ull << (low + 5)) - 1;
+    // rows without ones in the low columns need no table (binary_glynn.cuh)
+    std::vector<int> batch, chunk, table;
+    for (int r : tracked)
+        (!(rows[r] & batch_mask) ? batch : !(rows[r] & low_mask) ? chunk : table).push_back(r);
+    const int nt = (int)table.size();
     std::vector<int> caps(nt), group(nt);
-    for (int e = 0; e < nt; e++) caps[e] = __builtin_popcountll(rows[tracked[e]] & low_mask) + 1;
+    for (int e = 0; e < nt; e++) caps[e] = __builtin_popcountll(rows[table[e]] & low_mask) + 1;
     const int groups = binary_pack_groups(NPAD, P->words, caps.data(), nt, group.data(), &P->warps);
-    if (!groups) return false;
+    if (groups < 0) return false;
     P->planes = K;
-    P->ntracked = nt;
     P->npad = NPAD;
     P->G = G;
     P->NG = (NPAD + G - 1) / G;
     P->NL = P->NG + (NPAD > 32 ? 2 : 1);
     P->off_deg = align_up((size_t)NPAD * 8, 16);
     P->off_trk = align_up(P->off_deg + (size_t)NPAD * 4, 256);
-    P->off_acc = align_up(P->off_trk + 48 * sizeof(BinTrack), 256);
+    P->off_acc = align_up(P->off_trk + BIN_TRACK * sizeof(BinTrack), 256);
     P->image.assign(P->off_acc, 0);
     uint64_t *rm = (uint64_t *)P->image.data();
     int32_t *dg = (int32_t *)(P->image.data() + P->off_deg);
@@ -348,23 +353,32 @@ static bool plan_build_binary(const int64_t *A, int n, bool whole, ExactPlan *P)
         dg[i] = (int32_t)deg[order[i]];
     }
     int w = 0, entries = 1;                      // entry 0: all ones
+    const auto record = [&](int row, int cap, int stride, int base) {
+        BinTrack &t = trk[w++];
+        t.high = rows[row] >> low;
+        t.low = (uint16_t)(rows[row] & low_mask);
+        t.half = (uint8_t)(deg[row] / 2);
+        t.cap = (uint8_t)cap;
+        t.stride = (uint16_t)stride;
+        t.base = (uint16_t)base;
+    };
+    for (const std::vector<int> *list : {&batch, &chunk}) {
+        for (int row : *list) record(row, 0, 0, 0xffff);
+        for (; w & 3; w++) trk[w] = BinTrack{0, 0, 1, 0, 0, 0xffff};     // never zero
+        (list == &batch ? P->batch_rows : P->uniform_rows) = w;
+    }
     for (int g = 0; g < groups; g++) {
         int stride = 1;
         for (int e = 0; e < nt; e++) {
             if (group[e] != g) continue;
-            BinTrack &t = trk[w++];
-            t.high = rows[tracked[e]] >> low;
-            t.low = (uint16_t)(rows[tracked[e]] & low_mask);
-            t.half = (uint8_t)(deg[tracked[e]] / 2);
-            t.cap = (uint8_t)caps[e];
-            t.stride = (uint16_t)stride;
-            t.base = stride == 1 ? (uint16_t)entries : 0xffff;
+            record(table[e], caps[e], stride, stride == 1 ? entries : 0xffff);
             stride *= caps[e] + 1;
         }
         entries += stride;
     }
+    P->ntracked = w;
     P->entries = entries;
-    P->list_words = (groups + 3) / 4 * 4;
+    P->list_words = groups ? (groups + 3) / 4 * 4 : 4;
     P->lo = 0;
     P->hi = 1ull << (n - 1);
     return true;
@@ -526,6 +540,8 @@ static int plan_launch(ExactPlan *P, cudaStream_t stream) {
         b.rmask = (const uint64_t *)P->dev;
         b.deg = (const int32_t *)(P->dev + P->off_deg);
         b.trk = (const BinTrack *)(P->dev + P->off_trk);
+        b.batch_rows = P->batch_rows;
+        b.uniform_rows = P->uniform_rows;
         b.ntracked = P->ntracked;
         b.entries = P->entries;
         b.list_words = P->list_words;

@@ -145,3 +145,30 @@ def test_whole_chunks_survive(lib):
             a[i, first + 2 * i: first + 2 * i + 2] = 1
         assert _planes(lib, a) >= 2
         assert _exact(lib, a) == _via_general_kernel(lib, a)
+
+
+@pytest.mark.parametrize("n,degree", [(24, 5), (24, 4), (33, 3), (33, 4)])
+def test_rows_outside_the_low_columns(lib, n, degree):
+    # even rows with no ones in the low 10/11 columns (no table) and none in
+    # the low 15/16 (decided for 32 chunks at once), beside rows with ones
+    # anywhere; odd `degree`: no row has a table.  Windows, so that the
+    # transpose is not taken, and the whole walk.
+    from permgpu import shard
+    rng = np.random.default_rng(n * degree)
+    a = np.zeros((n, n), dtype=np.int64)
+    for i in range(n):
+        first, d = ((0, degree), (11, 4), (16, 2))[(i > n // 2) + (i > n // 2 + 4)]
+        a[i, rng.choice(np.arange(first, n), size=d, replace=False)] = 1
+    a[:n // 2 + 1] |= np.eye(n, dtype=np.int64)[:n // 2 + 1]
+    for i in range(n // 2 + 1):
+        if a[i].sum() % 2 != degree % 2:
+            a[i, rng.choice(np.flatnonzero(a[i] == 0))] = 1
+    assert _planes(lib, a) >= 2
+    b = a.copy()
+    b[0] *= 2
+    top = 1 << (n - 1)
+    for lo, hi in ((0, 1 << 20), (3 * 2048 + 4, (1 << 20) + 7 * 1024), (top - (1 << 21), top)):
+        v = shard.words_value(shard.exact_partial_words(a, lo, hi))
+        w = shard.words_value(shard.exact_partial_words(b, lo, hi))
+        assert 2 * v == w, (lo, hi)
+    assert _exact(lib, a) == _via_general_kernel(lib, a)
