@@ -34,7 +34,9 @@
 // lane a row for the batch and by bytes for the chunk, and a batch or chunk
 // with a zero row is left.  4x4x5 grid 33.5 -> 11.6 ms (with a few bonds
 // removed 34.9 -> 25.7), 6x4x3 5.4 -> 4.2, 8x8 0.17 -> 0.05; dense matrices
-// have no such row and run as before within 1 %.
+// have no such row and run as before within 1 %.  A whole walk also orders
+// its columns so that such rows exist (binary_order_columns): with bonds
+// removed and columns shuffled 6.8 ms.
 //
 // Evaluation.  Surviving states are appended to a per-warp queue; whenever
 // 32 are queued every lane evaluates one exactly.  The row sums come as
@@ -51,8 +53,8 @@
 //
 // Issue bound (65-80 % of the issue slots).  Whole calls against a
 // bit-sliced tracker that updated one state per lane and step and evaluated
-// by popcount: 4x4x5 grid (40 x 40, 0.08 % survive) 441 -> 11.6 ms, 36 x 36
-// Bernoulli(1/2) (6-13 % survive) 67-76 -> 22-28 ms.
+// by popcount: 4x4x5 grid (40 x 40, 0.08 % survive) 441 -> 6.8 ms, 36 x 36
+// Bernoulli(1/2) (6-13 % survive) 67-76 -> 18-22 ms.
 #pragma once
 
 #include "exact_glynn.cuh"

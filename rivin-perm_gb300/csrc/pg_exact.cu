@@ -260,9 +260,10 @@ int binary_pack_groups(int NPAD, int W, const int *caps, int rows, int *group, i
 // would cost more than the general kernel, which then runs (as it does when
 // the matrix is not 0/1 or no compiled shape fits).  A whole walk takes the
 // transpose when fewer of its sampled states survive (36 x 36
-// Bernoulli(1/2): 6..13 % either way); windows keep the rows' own states.
+// Bernoulli(1/2): 6..13 % either way) and orders the columns so that even
+// rows lie in the high ones; windows keep the rows' own states.
 struct BinaryRows {
-    std::vector<uint64_t> deg, rows;     // padded to NPAD
+    std::vector<uint64_t> deg, rows;     // padded to NPAD; bit j: column j
     std::vector<int> tracked;            // even-degree rows
     int maxh = 0, survive = 0;           // largest half degree, survivors of 1024 samples
 };
@@ -276,7 +277,7 @@ static void binary_rows(const int64_t *A, int n, bool transposed, BinaryRows *B)
         for (int j = 0; j < n; j++) {
             const uint64_t v = (uint64_t)(transposed ? A[(size_t)j * n + i] : A[(size_t)i * n + j]);
             d += v;
-            if (j < n - 1) m |= v << j;
+            m |= v << j;
         }
         B->deg[i] = d;
         B->rows[i] = m;
@@ -298,6 +299,51 @@ static void binary_rows(const int64_t *A, int n, bool transposed, BinaryRows *B)
     }
 }
 
+// Reorders the columns, from the last down: the columns of the even row that
+// has the fewest left (of equals, the one whose columns other even rows share
+// most), the most shared first, until `low` are left.  Each row that ends
+// above `low` decides whole chunks (binary_glynn.cuh).  The batches that are
+// left take longer and are fewer: from 2^15 batches on they still fill every
+// warp evenly.  4x4x5 grid with shuffled columns 25.7 -> 6.8 ms, 5x7x2
+// 0.66 -> 0.21, 36 x 36 Bernoulli(1/2) 25.0/21.2/21.0 -> 22.2/19.3/18.0;
+// Bernoulli(1/2) at order 31, with 2^15 batches, 1.02/0.95/0.88 ->
+// 1.03/0.92/0.86, at order 29 0.34 -> 0.40 (so not below).
+constexpr int BINARY_ORDER_LOG = 15;
+static void binary_order_columns(int n, int low, BinaryRows *B) {
+    uint64_t left = (1ull << n) - 1;
+    int order[48], at = n;               // order[new column] = old column
+    while (at > low) {
+        int count[48] = {0}, best = 0, best_columns = 49, best_shared = -1;
+        for (int r : B->tracked)
+            for (uint64_t m = B->rows[r] & left; m; m &= m - 1) count[__builtin_ctzll(m)]++;
+        for (int r : B->tracked) {
+            const int columns = __builtin_popcountll(B->rows[r] & left);
+            if (columns == 0 || columns > best_columns) continue;
+            int shared = 0;
+            for (uint64_t m = B->rows[r] & left; m; m &= m - 1) shared += count[__builtin_ctzll(m)];
+            if (columns == best_columns && shared <= best_shared) continue;
+            best = r;
+            best_columns = columns;
+            best_shared = shared;
+        }
+        if (best_shared < 0) break;
+        for (uint64_t m = B->rows[best] & left; m;) {
+            int top = __builtin_ctzll(m);
+            for (uint64_t t = m; t; t &= t - 1)
+                if (count[__builtin_ctzll(t)] > count[top]) top = __builtin_ctzll(t);
+            m &= ~(1ull << top);
+            left &= ~(1ull << top);
+            order[--at] = top;
+        }
+    }
+    for (; left; left &= left - 1) order[--at] = __builtin_ctzll(left);
+    for (uint64_t &m : B->rows) {
+        uint64_t v = 0;
+        for (int j = 0; j < n; j++) v |= (m >> order[j] & 1) << j;
+        m = v;
+    }
+}
+
 static bool plan_build_binary(const int64_t *A, int n, bool whole, ExactPlan *P) {
     if (!EXACT_BINARY || n < BINARY_MIN_N || n > 48) return false;
     for (size_t i = 0; i < (size_t)n * n; i++)
@@ -314,6 +360,11 @@ static bool plan_build_binary(const int64_t *A, int n, bool whole, ExactPlan *P)
         binary_rows(A, n, true, &T);
         if (!T.tracked.empty() && T.survive < B.survive) B = std::move(T);
     }
+    P->sparse = B.survive * 64 < BINARY_SAMPLES;
+    P->words = P->sparse ? 2 : 1;
+    const int low = bin_low(P->words);
+    if (whole && n - 1 >= low + 5 + BINARY_ORDER_LOG) binary_order_columns(n, low, &B);
+    for (uint64_t &m : B.rows) m &= (1ull << (n - 1)) - 1;       // the last column's sign is fixed
     const std::vector<uint64_t> &deg = B.deg, &rows = B.rows;
     const std::vector<int> &tracked = B.tracked;
     std::vector<int> order(NPAD);
@@ -323,9 +374,6 @@ static bool plan_build_binary(const int64_t *A, int n, bool whole, ExactPlan *P)
         if (exact_group_rows(deg.data(), NPAD, g, order.data())) { G = g; break; }
     }
     if (!G) return false;
-    P->sparse = B.survive * 64 < BINARY_SAMPLES;
-    P->words = P->sparse ? 2 : 1;
-    const int low = bin_low(P->words);
     const uint64_t low_mask = (1ull << low) - 1, batch_mask = (1ull << (low + 5)) - 1;
     // rows without ones in the low columns need no table (binary_glynn.cuh)
     std::vector<int> batch, chunk, table;
