@@ -10,37 +10,32 @@
 // for every state (perm_binary_omp.c:236-347, perm_binary_cuda.cu:111-205);
 // this kernel only searches for the states without a zero row.
 //
-// Search.  A chunk is the 1024 W states of one setting of the high columns'
-// signs (W words a lane): bit k of word h of lane l is the state whose low
-// signs are k | l << 5 | h << 10 (aligned Gray windows, in another order).
-// The high columns are common to the warp, so an even-degree row is zero
-// exactly where the low columns hold x = deg_r / 2 - (ones in high minus
-// columns) more, words that depend only on the lane and on x in 0..dlow_r
-// (any other x: never zero).  Rows are packed into groups whose table of
-// AND-ed "no zero" words, one entry per combination of the rows' x, fits in
-// shared memory ([entry][32 lanes][W]: no bank conflicts); a chunk costs one
-// load and W ANDs per group, with a vote after every eight groups.  The 32
-// lanes prepare the entries of 32 consecutive chunks, whose signs differ in
-// five columns: row counts are bytes, the warp's count minus a 32-row
-// table's, four rows per subtraction.  W = 2 where under 1/64 of the states
-// survive (4x4x5 grid, before the next paragraph's shortcut: 34.9 ms, 58.6
-// with W = 1); else the evaluations need the
-// shared memory and W = 1 is faster (36 x 36 Bernoulli(1/2): 21.3 against
-// 26.7 ms).
+// Search.  A chunk is the 1024 states of one setting of the high columns'
+// signs: bit k of lane l's word is the state whose low signs are k | l << 5
+// (an aligned Gray window, in another order).  The high columns are common to
+// the warp, so an even-degree row is zero exactly where the low columns hold
+// x = deg_r / 2 - (ones in high minus columns) more, words that depend only
+// on the lane and on x in 0..dlow_r (any other x: never zero).  Rows are
+// packed into groups whose table of AND-ed "no zero" words, one entry per
+// combination of the rows' x, fits in shared memory ([entry][32 lanes]: no
+// bank conflicts); a chunk costs one load and AND per group, with a vote
+// after every eight groups.  The 32 lanes prepare the entries of the 32
+// chunks of a batch, whose signs differ in five columns: row counts are
+// bytes, the warp's count minus a 32-row table's, four rows per subtraction.
 //
 // Rows without ones in the low columns need no table.  Such a row is zero in
 // all of a chunk or none of it, one without ones in the five chunk columns
-// either in all of a batch of 32 chunks or none: they are tested first, one
-// lane a row for the batch and by bytes for the chunk, and a batch or chunk
-// with a zero row is left.  4x4x5 grid 33.5 -> 11.6 ms (with a few bonds
-// removed 34.9 -> 25.7), 6x4x3 5.4 -> 4.2, 8x8 0.17 -> 0.05; dense matrices
-// have no such row and run as before within 1 %.  A whole walk also orders
-// its columns so that such rows exist (binary_order_columns): with bonds
-// removed and columns shuffled 6.8 ms.
+// either in all of a batch or none.  Batch rows are tested first, for 32
+// batches at once, one a lane; then the chunk rows, by bytes.  A whole walk
+// orders its columns so that such rows exist (binary_order_columns).  4x4x5
+// grid with a few bonds removed and columns shuffled: 34.9 ms without these
+// tests, 25.7 with them (one batch at a time), 6.2 with ordered columns; 2-3
+// with the batches of a unit tested together and taken from all over the
+// walk (neighbours are zero together, and warps ran dry).
 //
 // Evaluation.  Surviving states are appended to a per-warp queue; whenever
 // 32 are queued every lane evaluates one exactly.  The row sums come as
-// bytes: base bytes of the chunk (and of h) minus a table of the ten low
+// bytes: base bytes of the chunk minus a table of the ten low
 // columns, four rows per subtraction, and one byte permute per row; then the
 // exact multi-word term of exact_glynn.cuh (row groups, signed running
 // product, 64-bit column accumulators).  Counting the signs by popcount took
@@ -53,7 +48,7 @@
 //
 // Issue bound (65-80 % of the issue slots).  Whole calls against a
 // bit-sliced tracker that updated one state per lane and step and evaluated
-// by popcount: 4x4x5 grid (40 x 40, 0.08 % survive) 441 -> 6.8 ms, 36 x 36
+// by popcount: 4x4x5 grid (40 x 40, 0.08 % survive) 441 -> 3.0 ms, 36 x 36
 // Bernoulli(1/2) (6-13 % survive) 67-76 -> 18-22 ms.
 #pragma once
 
@@ -61,15 +56,13 @@
 
 namespace pg {
 
-// columns spread over word bits (5), lanes (5) and, with two words a lane, words
-__host__ __device__ constexpr int bin_low(int W) { return 9 + W; }
-constexpr int BIN_TAB = 10;        // low columns of the evaluation's table
+constexpr int BIN_LOW = 10;        // columns spread over word bits (5) and lanes (5)
 constexpr int BIN_QCAP = 320;      // queue entries per warp (31 pending + 32 lanes x 8 bits)
 constexpr size_t BIN_SMEM = 222 * 1024;   // dynamic shared memory of a block, at most
 
 // One even-degree row, in table-group order.
 struct BinTrack {
-    uint64_t high;      // the row's ones in toggled columns bin_low, ... (bit 0 the first)
+    uint64_t high;      // the row's ones in toggled columns BIN_LOW, ... (bit 0 the first)
     uint16_t low;       // the row's ones in the columns below
     uint8_t half;       // deg / 2
     uint8_t cap;        // ones in `low`, plus 1: the entry of "never zero"
@@ -88,8 +81,6 @@ struct BinaryArgs {
     int entries;               // table entries (entry 0: no row is zero)
     int list_words;            // words of a chunk's list: the byte offset of each group's
                                // entry, padded with entry 0 to a multiple of four
-    int words;                 // words a lane: 2 when few states survive, else 1
-    int sparse;                // few states survive
     int warps;                 // warps of a block
     unsigned long long *acc;   // [NL] per-word sums (exact kernel layout)
     int *status;
@@ -99,25 +90,24 @@ struct BinaryArgs {
     volatile const int *abort_flag;
     uint64_t state_lo, state_hi;   // Gray states to walk
     int log_steps;             // chunks of a batch (<= 5)
-    int log_unit;              // batches of a work unit
+    int log_batches;           // batches of the window, rounded up
+    int log_unit;              // batches of a work unit (<= 5, <= log_batches)
 };
 
 // threads of a block, at most: as many warps as the registers allow
 // (fewer when the tables leave no room for their lists)
-__host__ __device__ constexpr int binary_max_threads(int NPAD, int W) {
-    return NPAD > 40 ? 512 : W > 1 ? 640 : 768;
-}
+__host__ __device__ constexpr int binary_max_threads(int NPAD) { return NPAD > 40 ? 512 : 768; }
 // words of a state's row bytes, padded for 8-byte loads
 __host__ __device__ constexpr int binary_row_words(int NPAD) { return (NPAD / 4 + 1) & ~1; }
 constexpr int BIN_TRACK = 56;           // even-degree rows (at most 48) with their padding
 constexpr int BIN_TRACK_WORDS = BIN_TRACK / 4;
-__host__ __device__ constexpr size_t binary_warp_bytes(int NPAD, int W, int list_words) {
-    return (size_t)32 * W * binary_row_words(NPAD) * 4 + (size_t)32 * list_words * 4 + BIN_QCAP * 2 +
+__host__ __device__ constexpr size_t binary_warp_bytes(int NPAD, int list_words) {
+    return (size_t)32 * binary_row_words(NPAD) * 4 + (size_t)32 * list_words * 4 + BIN_QCAP * 2 +
            BIN_TRACK_WORDS * 4 + 48;
 }
-__host__ __device__ constexpr size_t binary_smem(int NPAD, int W, int entries, int list_words, int warps) {
-    return (size_t)entries * 128 * W + (size_t)(1024 + 32) * binary_row_words(NPAD) * 4 +
-           32 * BIN_TRACK_WORDS * 4 + warps * ((binary_warp_bytes(NPAD, W, list_words) + 15) & ~(size_t)15);
+__host__ __device__ constexpr size_t binary_smem(int NPAD, int entries, int list_words, int warps) {
+    return (size_t)entries * 128 + (size_t)(1024 + 32) * binary_row_words(NPAD) * 4 +
+           32 * BIN_TRACK_WORDS * 4 + warps * ((binary_warp_bytes(NPAD, list_words) + 15) & ~(size_t)15);
 }
 
 // byte K of x, sign-extended
@@ -128,24 +118,24 @@ __device__ __forceinline__ int32_t binary_byte(uint32_t x) {
     return r;
 }
 
-template <int NPAD, int G, int W>
-__global__ void __launch_bounds__(binary_max_threads(NPAD, W), 1) binary_glynn_kernel(BinaryArgs a) {
+template <int NPAD, int G>
+__global__ void __launch_bounds__(binary_max_threads(NPAD), 1) binary_glynn_kernel(BinaryArgs a) {
     using S = ExactShape<NPAD, G>;
     constexpr int NL = S::NL, NR = S::NR;
     constexpr int FOLD = 1 << EXACT_LOGU;   // terms the 64-bit columns hold between folds
     constexpr int NW = NPAD / 4, LS = binary_row_words(NPAD), TW = BIN_TRACK_WORDS;
-    constexpr int LOW = bin_low(W), HI = LOW + 5;         // first column common to a batch of 32 chunks
+    constexpr int LOW = BIN_LOW, HI = LOW + 5;         // first column common to a batch of 32 chunks
     extern __shared__ uint4 bin_shared[];
-    uint32_t *ztab = reinterpret_cast<uint32_t *>(bin_shared);      // [entries][32][W]
-    uint32_t *ltab = ztab + (size_t)a.entries * 32 * W;             // [1024][LS]
+    uint32_t *ztab = reinterpret_cast<uint32_t *>(bin_shared);      // [entries][32]
+    uint32_t *ltab = ztab + (size_t)a.entries * 32;             // [1024][LS]
     uint32_t *ctab = ltab + 1024 * LS;                // [32][LS] bytes of the five chunk columns
     uint32_t *xtab = ctab + 32 * LS;                  // [32][TW] the same of the even rows
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     char *mine = reinterpret_cast<char *>(xtab + 32 * TW) +
-                 warp * ((binary_warp_bytes(NPAD, W, a.list_words) + 15) & ~(size_t)15);
+                 warp * ((binary_warp_bytes(NPAD, a.list_words) + 15) & ~(size_t)15);
     uint32_t *list = reinterpret_cast<uint32_t *>(mine);            // [32][list_words]
-    uint32_t *base = list + 32 * a.list_words;                      // [32][W][LS]
-    uint32_t *ucnt = base + 32 * W * LS;                                // row bytes, then even rows'
+    uint32_t *base = list + 32 * a.list_words;                      // [32][LS]
+    uint32_t *ucnt = base + 32 * LS;                                    // row bytes, then even rows'
     uint32_t *xcnt = ucnt + 12;
     uint16_t *q = reinterpret_cast<uint16_t *>(xcnt + TW);
     __shared__ BinTrack s_trk[BIN_TRACK];
@@ -165,30 +155,22 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD, W), 1) binary_glynn_k
         s_eq[i / 6][i % 6] = w;
     }
     __syncthreads();
-    if (warp == 0)
-        for (int h = 0; h < W; h++) ztab[lane * W + h] = 0xffffffffu;
+    if (warp == 0) ztab[lane] = 0xffffffffu;
     for (int e0 = a.uniform_rows; e0 < a.ntracked;) {            // table groups
         int e1 = e0 + 1, size = s_trk[e0].cap + 1;
         for (; e1 < a.ntracked && s_trk[e1].base == 0xffff; e1++) size *= s_trk[e1].cap + 1;
         if ((int)threadIdx.x >= e0 && (int)threadIdx.x < e1)
-            s_rec[threadIdx.x] = make_uint4(s_trk[threadIdx.x].cap, s_trk[threadIdx.x].stride * 128u * W,
-                                            (int)threadIdx.x == e1 - 1 ? s_trk[e0].base * 128u * W + 1 : 0, 0);
+            s_rec[threadIdx.x] = make_uint4(s_trk[threadIdx.x].cap, s_trk[threadIdx.x].stride * 128u,
+                                            (int)threadIdx.x == e1 - 1 ? s_trk[e0].base * 128u + 1 : 0, 0);
         for (int idx = warp; idx < size; idx += warps) {
-            uint32_t w[W];
-#pragma unroll
-            for (int h = 0; h < W; h++) w[h] = 0xffffffffu;
+            uint32_t w = 0xffffffffu;
             for (int e = e0, rem = idx; e < e1; e++) {
                 const int cap = s_trk[e].cap, low = s_trk[e].low;
-                const int x = rem % (cap + 1), v = x - __popc((low >> 5) & lane);
+                const int x = rem % (cap + 1), y = x - __popc((low >> 5) & lane);
                 rem /= cap + 1;
-#pragma unroll
-                for (int h = 0; h < W; h++) {
-                    const int y = v - (h & (low >> 10));
-                    if (x < cap && y >= 0 && y <= 5) w[h] &= ~s_eq[low & 31][y];
-                }
+                if (x < cap && y >= 0 && y <= 5) w &= ~s_eq[low & 31][y];
             }
-#pragma unroll
-            for (int h = 0; h < W; h++) ztab[((s_trk[e0].base + idx) * 32 + lane) * W + h] = w[h];
+            ztab[(s_trk[e0].base + idx) * 32 + lane] = w;
         }
         e0 = e1;
     }
@@ -212,9 +194,6 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD, W), 1) binary_glynn_k
         }
         xtab[(i & 31) * TW + (i >> 5)] = b;
     }
-    uint32_t h_bytes[NW];               // column 10 (two words a lane)
-#pragma unroll
-    for (int v = 0; v < NW; v++) h_bytes[v] = W > 1 ? row_bytes(v, BIN_TAB, 1u) : 0;
     __syncthreads();
 
     uint32_t acc[NL];
@@ -230,12 +209,12 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD, W), 1) binary_glynn_k
         __syncwarp();
         qn -= count;
         const bool live = lane < count;
-        // low signs, chunk of the batch (5 bits); the chunk and h pick the base row
+        // low signs, chunk of the batch (5 bits)
         const uint32_t e = live ? q[qn + lane] : 0, k = e >> LOW;
         uint32_t d[LS];
 #pragma unroll
         for (int v = 0; v < LS / 2; v++) {
-            const uint2 x = reinterpret_cast<const uint2 *>(base + (e >> BIN_TAB) * LS)[v];
+            const uint2 x = reinterpret_cast<const uint2 *>(base + k * LS)[v];
             const uint2 y = reinterpret_cast<const uint2 *>(ltab + (e & 1023u) * LS)[v];
             // bytes 128 + s_r, no borrow between them; then two's complement
             d[2 * v + 0] = (x.x - y.x) ^ 0x80808080u;
@@ -259,9 +238,8 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD, W), 1) binary_glynn_k
         }
         __syncwarp();
     };
-    // Appends the states of `alive` (tag: chunk and h).  Few survivors: one of
-    // each lane at a time, placed by a ballot.  Many: placed by a scan over the
-    // lanes' counts, all at once while they fit the queue, else 256 at most.
+    // Appends the states of `alive` (tag: chunk), placed by a scan over the
+    // lanes' counts: all at once while they fit the queue, else 256 at most.
     auto scan = [&](uint32_t part) {
         int inc = __popc(part);
 #pragma unroll
@@ -282,72 +260,60 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD, W), 1) binary_glynn_k
         while (qn >= 32) evaluate(32);
     };
     auto append = [&](uint32_t alive, uint32_t tag) {
-        uint32_t mask = __ballot_sync(0xffffffffu, alive != 0);
-        if (!mask) return;
-        if (!a.sparse) {
-            const int inc = scan(alive), total = __shfl_sync(0xffffffffu, inc, 31);
-            if (qn + total <= BIN_QCAP) {
-                push(alive, tag, inc, total);
-            } else {
-                for (int o = 0; o < 32; o += 8) {
-                    const uint32_t part = alive & (0xffu << o);
-                    const int pi = scan(part);
-                    push(part, tag, pi, __shfl_sync(0xffffffffu, pi, 31));
-                }
+        if (!__any_sync(0xffffffffu, alive != 0)) return;
+        const int inc = scan(alive), total = __shfl_sync(0xffffffffu, inc, 31);
+        if (qn + total <= BIN_QCAP) {
+            push(alive, tag, inc, total);
+        } else {
+            for (int o = 0; o < 32; o += 8) {
+                const uint32_t part = alive & (0xffu << o);
+                const int pi = scan(part);
+                push(part, tag, pi, __shfl_sync(0xffffffffu, pi, 31));
             }
-            return;
-        }
-        for (; mask; mask = __ballot_sync(0xffffffffu, alive != 0)) {
-            if (alive) {
-                const uint32_t rest = alive & (alive - 1);
-                q[qn + __popc(mask & ((1u << lane) - 1u))] =
-                    (uint16_t)(tag | (lane << 5) | __popc((alive ^ rest) - 1));
-                alive = rest;
-            }
-            qn += __popc(mask);
-            if (qn >= 32) evaluate(32);
         }
     };
 
     // Work units go to warps from a counter (the share of surviving states
     // varies strongly along the walk with the signs of the columns), one
     // ahead, so that the atomic's round trip overlaps the work.  A unit is
-    // 2^log_unit batches of 2^log_steps chunks, aligned.
+    // 2^log_unit batches of 2^log_steps chunks from all over the walk (an odd
+    // multiple of their number modulo a power of two): neighbours share their
+    // zero rows and would leave whole units empty and others full.
     const uint64_t c_lo = a.state_lo >> LOW;
     const uint64_t c_hi = (a.state_hi + (1u << LOW) - 1) >> LOW;
-    const int log_all = a.log_steps + a.log_unit;
-    const uint64_t units = ((c_hi - 1) >> log_all) - (c_lo >> log_all) + 1;
-    const char *zl = reinterpret_cast<const char *>(ztab + lane * W);
+    const uint64_t units = 1ull << (a.log_batches - a.log_unit);
+    const char *zl = reinterpret_cast<const char *>(ztab + lane);
     bool aborted = false;
     uint32_t polls = 0;
     for (uint64_t unit = (uint64_t)warp * gridDim.x + blockIdx.x; unit < units && !aborted;) {
         unsigned long long nx = 0;
         if (lane == 0) nx = (uint64_t)gridDim.x * warps + atomicAdd(a.next, 1ull);
-        for (uint32_t bb = 0; bb < (1u << a.log_unit); bb++) {
+        // the unit's batches, one a lane: not those beyond the window, nor
+        // those with a batch row that is zero (in all of the batch)
+        const uint64_t number = ((unit << a.log_unit | lane) * 0x9e3779b97f4a7c15ull) &
+                                ((1ull << a.log_batches) - 1);
+        const uint64_t mine_c0 = ((c_lo >> a.log_steps) + number) << a.log_steps;
+        bool go;
+        {
+            const uint64_t b5 = mine_c0 >> 5;
+            const uint32_t hw = (uint32_t)(b5 ^ (b5 >> 1));
+            go = lane < (1 << a.log_unit) && mine_c0 < c_hi;
+            for (int r = 0; r < a.batch_rows; r++)
+                go &= (int)s_trk[r].half != __popc((uint32_t)(s_trk[r].high >> 5) & hw);
+        }
+        // the host-mapped abort word is read once per 128 batches that are
+        // searched (4096 units without one), from the warp's second period on
+        polls++;
+        for (uint32_t todo = __ballot_sync(0xffffffffu, go); todo; todo &= todo - 1) {
             // chunks c0 + k0 .. c0 + k1 - 1 of the batch lie in the window
-            const uint64_t c0 = (((c_lo >> log_all) + unit) << log_all) + ((uint64_t)bb << a.log_steps);
-            const int k1 = c_hi <= c0 ? 0 : c_hi - c0 < (1ull << a.log_steps) ? (int)(c_hi - c0)
-                                                                             : 1 << a.log_steps;
-            const int kfirst = c_lo > c0 ? (c_lo - c0 < (uint64_t)k1 ? (int)(c_lo - c0) : k1) : 0;
-            if (kfirst >= k1) continue;
-            // the host-mapped abort word is read once per 128 batches that are
-            // searched (4096 that are not), from the warp's second period on
-            if (++polls >= 4096) {
-                polls = 0;
-                if (__any_sync(0xffffffffu, *a.abort_flag != 0)) {
-                    aborted = true;
-                    break;
-                }
-            }
+            const uint64_t c0 = __shfl_sync(0xffffffffu, mine_c0, __ffs(todo) - 1);
+            const int k1 = c_hi - c0 < (1ull << a.log_steps) ? (int)(c_hi - c0) : 1 << a.log_steps;
+            const int kfirst = c_lo > c0 ? (int)(c_lo - c0) : 0;
+            polls += 32;
             // the batch's common high signs: gray(c0 >> 5) in columns HI and up
             const uint64_t b5 = c0 >> 5;
             const uint32_t hw = (uint32_t)(b5 ^ (b5 >> 1));
             auto ones = [&](uint64_t m) { return __popc((uint32_t)m & hw); };
-            // a batch row that is zero now is zero in the whole batch
-            bool dead = false;
-            for (int r = lane; r < a.batch_rows; r += 32)
-                dead |= (int)s_trk[r].half == ones(s_trk[r].high >> 5);
-            if (__any_sync(0xffffffffu, dead)) continue;
             for (int r = a.batch_rows + lane; r < a.ntracked; r += 32)
                 reinterpret_cast<uint8_t *>(xcnt)[r] = (uint8_t)(128 + s_trk[r].half - ones(s_trk[r].high >> 5));
             __syncwarp();
@@ -363,7 +329,6 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD, W), 1) binary_glynn_k
             uint32_t chunks = __ballot_sync(0xffffffffu, zero == 0 && lane >= kfirst && lane < k1);
             __syncwarp();               // xcnt is read
             if (!chunks) continue;
-            polls += 31;
             c_odd = (uint32_t)c0;
             const bool edge = ((c0 + kfirst) << LOW) < a.state_lo || ((c0 + k1) << LOW) > a.state_hi;
             for (int r = lane; r < NPAD; r += 32)
@@ -371,13 +336,9 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD, W), 1) binary_glynn_k
             __syncwarp();
             {
                 const uint32_t *cb = ctab + x5 * LS;
-                uint32_t *o = base + lane * W * LS;
+                uint32_t *o = base + lane * LS;
 #pragma unroll
-                for (int v = 0; v < NW; v++) {
-                    const uint32_t b = ucnt[v] - cb[v];
-                    o[v] = b;
-                    if (W > 1) o[LS + v] = b - h_bytes[v];
-                }
+                for (int v = 0; v < NW; v++) o[v] = ucnt[v] - cb[v];
             }
             {
                 uint32_t *ll = list + lane * a.list_words;
@@ -407,70 +368,51 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD, W), 1) binary_glynn_k
                 const bool pair = chunks != 0;
                 kk[1] = pair ? __ffs(chunks) - 1 : kk[0];
                 chunks &= chunks - 1;
-                uint32_t alive[2][W];
-#pragma unroll
-                for (int h = 0; h < W; h++) {
-                    alive[0][h] = 0xffffffffu;
-                    alive[1][h] = pair ? 0xffffffffu : 0u;
-                }
+                uint32_t alive[2] = {0xffffffffu, pair ? 0xffffffffu : 0u};
                 for (int v = 0; v < a.list_words; v += 4) {
-                    uint32_t any = 0;
 #pragma unroll
                     for (int t = 0; t < 2; t++) {
                         const uint4 o = *reinterpret_cast<const uint4 *>(list + kk[t] * a.list_words + v);
-                        if constexpr (W > 1) {
-                            const auto at = [&](uint32_t off) {
-                                return *reinterpret_cast<const uint2 *>(zl + off);
-                            };
-                            const uint2 z0 = at(o.x), z1 = at(o.y), z2 = at(o.z), z3 = at(o.w);
-                            alive[t][0] &= z0.x & z1.x & z2.x & z3.x;
-                            alive[t][W - 1] &= z0.y & z1.y & z2.y & z3.y;
-                        } else {
-                            const auto at = [&](uint32_t off) {
-                                return *reinterpret_cast<const uint32_t *>(zl + off);
-                            };
-                            alive[t][0] &= at(o.x) & at(o.y) & at(o.z) & at(o.w);
-                        }
-#pragma unroll
-                        for (int h = 0; h < W; h++) any |= alive[t][h];
+                        const auto at = [&](uint32_t off) {
+                            return *reinterpret_cast<const uint32_t *>(zl + off);
+                        };
+                        alive[t] &= at(o.x) & at(o.y) & at(o.z) & at(o.w);
                     }
-                    if ((v & 4) && !__any_sync(0xffffffffu, any != 0)) break;
+                    if ((v & 4) && !__any_sync(0xffffffffu, (alive[0] | alive[1]) != 0)) break;
                 }
                 if (edge) {             // a window that starts or ends inside a chunk
 #pragma unroll
-                    for (int t = 0; t < 2; t++)
-#pragma unroll
-                        for (int h = 0; h < W; h++) {
-                            const uint64_t c = c0 + kk[t];
-                            uint32_t in = 0;
-                            for (int k = 0; k < 32; k++) {
-                                uint32_t i = (uint32_t)(k | (lane << 5) | (h << 10)) ^
-                                             (uint32_t)((c & 1) << (LOW - 1));
-                                i ^= i >> 1;
-                                i ^= i >> 2;
-                                i ^= i >> 4;
-                                i ^= i >> 8;
-                                const uint64_t g = (c << LOW) | i;
-                                in |= (uint32_t)(g >= a.state_lo && g < a.state_hi) << k;
-                            }
-                            alive[t][h] &= in;
+                    for (int t = 0; t < 2; t++) {
+                        const uint64_t c = c0 + kk[t];
+                        uint32_t in = 0;
+                        for (int k = 0; k < 32; k++) {
+                            uint32_t i = (uint32_t)(k | (lane << 5)) ^ (uint32_t)((c & 1) << (LOW - 1));
+                            i ^= i >> 1;
+                            i ^= i >> 2;
+                            i ^= i >> 4;
+                            i ^= i >> 8;
+                            const uint64_t g = (c << LOW) | i;
+                            in |= (uint32_t)(g >= a.state_lo && g < a.state_hi) << k;
                         }
+                        alive[t] &= in;
+                    }
                 }
 #pragma unroll
-                for (int t = 0; t < 2; t++)
-#pragma unroll
-                    for (int h = 0; h < W; h++)
-                        append(alive[t][h], (uint32_t)(kk[t] << LOW) | (uint32_t)(h << BIN_TAB));
+                for (int t = 0; t < 2; t++) append(alive[t], (uint32_t)(kk[t] << LOW));
             }
             if (qn > 0) evaluate(qn);       // the next batch has other base bytes
             __syncwarp();
+        }
+        if (polls >= 4096) {
+            polls = 0;
+            aborted = __any_sync(0xffffffffu, *a.abort_flag != 0);
         }
         unit = __shfl_sync(0xffffffffu, nx, 0);
     }
     if (terms > 0) FoldCols<NR, NL>::apply(acc, col, colt);
 
     // block reduction and result words: as the exact kernel
-    __shared__ long long red[binary_max_threads(NPAD, W) / 32][NL];
+    __shared__ long long red[binary_max_threads(NPAD) / 32][NL];
     __shared__ int any_abort;
     if (threadIdx.x == 0) any_abort = 0;
     __syncthreads();
@@ -486,19 +428,14 @@ __global__ void __launch_bounds__(binary_max_threads(NPAD, W), 1) binary_glynn_k
     exact_epilogue<NL>(red, any_abort, a.acc, a.part, a.status);
 }
 
-template <int NPAD, int G, int W>
-cudaError_t launch_binary_words(const BinaryArgs &args, int blocks, cudaStream_t stream) {
-    const size_t smem = binary_smem(NPAD, W, args.entries, args.list_words, args.warps);
-    cudaError_t e = cudaFuncSetAttribute(binary_glynn_kernel<NPAD, G, W>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    binary_glynn_kernel<NPAD, G, W><<<blocks, 32 * args.warps, smem, stream>>>(args);
-    return cudaGetLastError();
-}
 template <int NPAD, int G>
 cudaError_t launch_binary_glynn(const BinaryArgs &args, int blocks, cudaStream_t stream) {
-    return args.words == 2 ? launch_binary_words<NPAD, G, 2>(args, blocks, stream)
-                           : launch_binary_words<NPAD, G, 1>(args, blocks, stream);
+    const size_t smem = binary_smem(NPAD, args.entries, args.list_words, args.warps);
+    cudaError_t e = cudaFuncSetAttribute(binary_glynn_kernel<NPAD, G>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    binary_glynn_kernel<NPAD, G><<<blocks, 32 * args.warps, smem, stream>>>(args);
+    return cudaGetLastError();
 }
 
 // Compiled shapes (binary_inst_*.cu): NPAD in {24, 28, ..., 48}, G in {5, 6,
@@ -521,6 +458,6 @@ cudaError_t launch_binary_any(int NPAD, int G, const BinaryArgs &args, int block
 // tables to fit beside the NPAD kernel's other shared memory, with the most
 // warps that allow it; group[e] = the row's group.  Returns the number of
 // groups, -1 if there is no such packing.
-int binary_pack_groups(int NPAD, int W, const int *caps, int rows, int *group, int *warps);
+int binary_pack_groups(int NPAD, const int *caps, int rows, int *group, int *warps);
 
 }  // namespace pg

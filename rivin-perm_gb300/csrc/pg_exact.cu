@@ -194,8 +194,8 @@ struct ExactPlan {
     // 0/1 kernel (binary_glynn.cuh): bits of the largest even row's half
     // degree (0: the general kernel), tracked (even-degree) rows, padded
     // rows, table entries and list words, Gray window
-    int planes = 0, batch_rows = 0, uniform_rows = 0, ntracked = 0, npad = 0, entries = 0, list_words = 0, warps = 0,
-        words = 1, sparse = 0;
+    int planes = 0, batch_rows = 0, uniform_rows = 0, ntracked = 0, npad = 0, entries = 0, list_words = 0, warps = 0;
+    double batches_left = 1;
     size_t off_deg = 0, off_trk = 0;
     uint64_t lo = 0, hi = 0;
     ChunkPlan chunks{};
@@ -217,7 +217,7 @@ struct ExactPlan {
 
 // Sixteen warps keep the kernel within 2 % of its best (12..24 measured).
 constexpr int BIN_WARPS_MIN = 16;
-int binary_pack_groups(int NPAD, int W, const int *caps, int rows, int *group, int *warps) {
+int binary_pack_groups(int NPAD, const int *caps, int rows, int *group, int *warps) {
     std::vector<int> by(rows);
     for (int e = 0; e < rows; e++) by[e] = e;
     std::stable_sort(by.begin(), by.end(), [&](int x, int y) { return caps[x] > caps[y]; });
@@ -235,14 +235,14 @@ int binary_pack_groups(int NPAD, int W, const int *caps, int rows, int *group, i
     };
     // the fewest lookups (a multiple of four) with at least BIN_WARPS_MIN
     // warps, then the most warps for them; fewer warps only where nothing fits
-    const int most = binary_max_threads(NPAD, W) / 32;
+    const int most = binary_max_threads(NPAD) / 32;
     int best = 0;
     *warps = most;
     if (rows == 0) return 0;
     for (int w = most; w >= 2 && (w >= BIN_WARPS_MIN || !best); w -= 2)
         for (int T = 4; T < rows + 4 && (!best || T < best); T += 4) {
             const int groups = T < rows ? T : rows;
-            if (binary_smem(NPAD, W, (int)pack(groups), T, w) > BIN_SMEM) continue;
+            if (binary_smem(NPAD, (int)pack(groups), T, w) > BIN_SMEM) continue;
             best = T;
             *warps = w;
         }
@@ -302,13 +302,12 @@ static void binary_rows(const int64_t *A, int n, bool transposed, BinaryRows *B)
 // Reorders the columns, from the last down: the columns of the even row that
 // has the fewest left (of equals, the one whose columns other even rows share
 // most), the most shared first, until `low` are left.  Each row that ends
-// above `low` decides whole chunks (binary_glynn.cuh).  The batches that are
-// left take longer and are fewer: from 2^15 batches on they still fill every
-// warp evenly.  4x4x5 grid with shuffled columns 25.7 -> 6.8 ms, 5x7x2
-// 0.66 -> 0.21, 36 x 36 Bernoulli(1/2) 25.0/21.2/21.0 -> 22.2/19.3/18.0;
-// Bernoulli(1/2) at order 31, with 2^15 batches, 1.02/0.95/0.88 ->
-// 1.03/0.92/0.86, at order 29 0.34 -> 0.40 (so not below).
-constexpr int BINARY_ORDER_LOG = 15;
+// above `low` decides whole chunks (binary_glynn.cuh).  Not below 2^11
+// batches (order 27), where a few batches hold all that is left: at order 24
+// Bernoulli(1/2) 0.048/0.037/0.040 -> 0.044/0.056/0.068 ms, but at order 28
+// 0.21/0.18/0.21 -> 0.16/0.12/0.13, and the 4x4x5 grid with shuffled columns
+// 20 -> 2-3.
+constexpr int BINARY_ORDER_LOG = 11;
 static void binary_order_columns(int n, int low, BinaryRows *B) {
     uint64_t left = (1ull << n) - 1;
     int order[48], at = n;               // order[new column] = old column
@@ -360,10 +359,7 @@ static bool plan_build_binary(const int64_t *A, int n, bool whole, ExactPlan *P)
         binary_rows(A, n, true, &T);
         if (!T.tracked.empty() && T.survive < B.survive) B = std::move(T);
     }
-    P->sparse = B.survive * 64 < BINARY_SAMPLES;
-    P->words = P->sparse ? 2 : 1;
-    const int low = bin_low(P->words);
-    if (whole && n - 1 >= low + 5 + BINARY_ORDER_LOG) binary_order_columns(n, low, &B);
+    if (whole && n - 1 >= BIN_LOW + 5 + BINARY_ORDER_LOG) binary_order_columns(n, BIN_LOW, &B);
     for (uint64_t &m : B.rows) m &= (1ull << (n - 1)) - 1;       // the last column's sign is fixed
     const std::vector<uint64_t> &deg = B.deg, &rows = B.rows;
     const std::vector<int> &tracked = B.tracked;
@@ -374,7 +370,7 @@ static bool plan_build_binary(const int64_t *A, int n, bool whole, ExactPlan *P)
         if (exact_group_rows(deg.data(), NPAD, g, order.data())) { G = g; break; }
     }
     if (!G) return false;
-    const uint64_t low_mask = (1ull << low) - 1, batch_mask = (1ull << (low + 5)) - 1;
+    const uint64_t low_mask = (1ull << BIN_LOW) - 1, batch_mask = (1ull << (BIN_LOW + 5)) - 1;
     // rows without ones in the low columns need no table (binary_glynn.cuh)
     std::vector<int> batch, chunk, table;
     for (int r : tracked)
@@ -382,7 +378,7 @@ static bool plan_build_binary(const int64_t *A, int n, bool whole, ExactPlan *P)
     const int nt = (int)table.size();
     std::vector<int> caps(nt), group(nt);
     for (int e = 0; e < nt; e++) caps[e] = __builtin_popcountll(rows[table[e]] & low_mask) + 1;
-    const int groups = binary_pack_groups(NPAD, P->words, caps.data(), nt, group.data(), &P->warps);
+    const int groups = binary_pack_groups(NPAD, caps.data(), nt, group.data(), &P->warps);
     if (groups < 0) return false;
     P->planes = K;
     P->npad = NPAD;
@@ -400,10 +396,18 @@ static bool plan_build_binary(const int64_t *A, int n, bool whole, ExactPlan *P)
         rm[i] = rows[order[i]];
         dg[i] = (int32_t)deg[order[i]];
     }
+    // share of the batches without a zero row, its rows taken as independent:
+    // C(d, d/2) / 2^d of a row's signs balance
+    P->batches_left = 1;
+    for (int r : batch) {
+        double p = 1;
+        for (uint64_t i = 1; i <= deg[r] / 2; i++) p *= (double)(2 * i - 1) / (double)(2 * i);
+        P->batches_left *= 1 - p;
+    }
     int w = 0, entries = 1;                      // entry 0: all ones
     const auto record = [&](int row, int cap, int stride, int base) {
         BinTrack &t = trk[w++];
-        t.high = rows[row] >> low;
+        t.high = rows[row] >> BIN_LOW;
         t.low = (uint16_t)(rows[row] & low_mask);
         t.half = (uint8_t)(deg[row] / 2);
         t.cap = (uint8_t)cap;
@@ -513,7 +517,7 @@ static int plan_build(const int64_t *A, int n, ExactPlan *P, bool whole = true) 
         P->total = align_up(P->off_out + (size_t)(P->NL + 1) * 8, 256);
         P->image.resize(P->total, 0);
         // one block per SM: the warps share its tables
-        P->chunks.log_len = bin_low(P->words);
+        P->chunks.log_len = BIN_LOW;
         P->chunks.chunks = 1ull << (n - 1 - P->chunks.log_len);
         P->blocks = (uint64_t)dev.sm_count;
         add_block_slots(P);
@@ -594,8 +598,6 @@ static int plan_launch(ExactPlan *P, cudaStream_t stream) {
         b.entries = P->entries;
         b.list_words = P->list_words;
         b.warps = P->warps;
-        b.sparse = P->sparse;
-        b.words = P->words;
         b.acc = (unsigned long long *)(P->dev + P->off_acc);
         b.status = (int *)(P->dev + P->off_status);
         b.part = (unsigned long long *)(P->dev + P->off_part);
@@ -604,15 +606,30 @@ static int plan_launch(ExactPlan *P, cudaStream_t stream) {
         b.abort_flag = P->abort_dev;
         b.state_lo = P->lo;
         b.state_hi = P->hi;
-        // batches of 32 chunks (one per lane) while every warp gets two of
-        // them, shorter ones below; several batches to a unit on long walks,
-        // so that the counter's atomics stay rare
-        const uint64_t chunks = ((P->hi - P->lo) >> bin_low(P->words)) + 1;
+        // batches of 32 chunks (one per lane) while every warp gets eight of
+        // those that the batch rows leave, shorter ones below (28 x 28
+        // Bernoulli(1/2) 0.18-0.21 ms with two of all, 0.12-0.16 so), but
+        // not where the tests of the others would then take the time (8x10
+        // grid: 2.81 ms in batches of two chunks, 0.39 of 32)
+        const uint64_t chunks = ((P->hi - P->lo) >> BIN_LOW) + 1;
         const uint64_t warps = P->blocks * (uint64_t)P->warps;
         b.log_steps = 5;
-        while (b.log_steps > 1 && (chunks >> b.log_steps) < 2 * warps) b.log_steps--;
+        while (b.log_steps > 1 && P->batches_left * (chunks >> b.log_steps) < 8 * warps &&
+               (chunks >> b.log_steps) < 64 * warps)
+            b.log_steps--;
+        const uint64_t batches = (((P->hi - 1) >> (BIN_LOW + b.log_steps)) - (P->lo >> (BIN_LOW + b.log_steps))) + 1;
+        b.log_batches = 0;
+        while ((1ull << b.log_batches) < batches) b.log_batches++;
         b.log_unit = 0;
         while (b.log_unit < 3 && (chunks >> (6 + b.log_unit)) >= 32 * warps) b.log_unit++;
+        // several batches to a unit on long walks, so that the counter's
+        // atomics stay rare; up to 32 (they are tested one a lane) while at
+        // most one of them is expected to be left and every warp gets four
+        // units: 8x10 grid 1.31 -> 0.39 ms; with sixteen units 8x8 takes 88
+        // us instead of 55
+        while (b.log_unit < 5 && P->batches_left * (2 << b.log_unit) <= 1 &&
+               (batches >> (b.log_unit + 1)) >= 4 * warps)
+            b.log_unit++;
         PG_CUDA(launch_binary_any(P->npad, P->G, b, (int)P->blocks, stream));
         PG_CUDA(exact_finish(b.part, (int)P->blocks, P->NL, b.acc, b.status,
                              P->out, stream, b.next));
