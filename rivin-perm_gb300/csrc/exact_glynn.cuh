@@ -152,6 +152,17 @@ __device__ __forceinline__ void exact_term_col(const int32_t *s, uint64_t *col, 
     colt = first ? pt : colt + pt;
 }
 
+// Two of a fold's four steps always add the same column, and the compiler
+// keeps it in registers where it can; beyond eight product words (or with
+// float rows and a last group that is not full) that spills up to 150 words,
+// and the walk hides the table offset from the compiler instead: groups of
+// 2 at order 32 37.4 -> 35.4 ms, of 3 21.2 -> 19.4, of 4 at order 33 33.8 ->
+// 30.9.  Where nothing spills the registers are the better place (groups of
+// 5 at order 32: 11.0 ms, 11.8 without).
+__host__ __device__ constexpr bool exact_hoist(int N, int G, int FR) {
+    return (N + G - 1) / G <= 8 && (FR == 0 || N % G == 0);
+}
+
 // Walk chunks [c_begin, c_end) (row sums s already at state c_begin*2^log_len)
 // adding every term into acc.  Returns false if the abort word was seen.
 template <int N, int G, int FR = 0>
@@ -192,8 +203,9 @@ __device__ __forceinline__ bool exact_walk(const int32_t *tab, int32_t *s, uint3
                     sub = ((c >> (jc + 1)) & 1) == 0;
                 }
                 if (step) {
-                    const int4 *col =
-                        reinterpret_cast<const int4 *>(tab + (2 * j + sub) * NP);
+                    int at = (2 * j + sub) * NP;
+                    if (!exact_hoist(N, G, FR)) asm volatile("" : "+r"(at));
+                    const int4 *col = reinterpret_cast<const int4 *>(tab + at);
 #pragma unroll
                     for (int v = 0; v < NP / 4; v++) {
                         const int4 d = col[v];

@@ -206,3 +206,19 @@ def test_wide_engine_refuses_wider_rows(lib):
     assert err.value.status == lib.PG_EOVERFLOW
     with pytest.raises(lib.PermGpuError):
         lib.exact_wide_permanent(np.ones((33, 33), np.int64), 40)
+
+
+@pytest.mark.parametrize("n,mag", [(n, mag) for n in range(24, 33) for mag in (8, 40, 1000)] + [(33, 8)])
+def test_windows_match_other_group_sizes(lib, n, mag):
+    # groups of 4 with float rows (mag 8), of 3 and of 2, with and without
+    # columns held in registers; a scaled row changes the groups
+    from permgpu import shard
+    a = np.random.default_rng(n * mag).integers(-mag, mag + 1, (n, n), dtype=np.int64)
+    b = a.copy()
+    f = 64 if mag < 1000 else 4
+    b[n // 2] *= f
+    top = 1 << (n - 1)
+    for lo, hi in ((0, 1 << 18), ((1 << 20) + 4, (1 << 20) + 70_000), (top - 4096, top)):
+        v = shard.words_value(shard.exact_partial_words(a, lo, hi))
+        w = shard.words_value(shard.exact_partial_words(b, lo, hi))
+        assert f * v == w, (lo, hi)
