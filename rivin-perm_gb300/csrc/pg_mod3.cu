@@ -34,6 +34,7 @@
 // the row-sliced walk, so no other path is kept.
 #include "pg_internal.h"
 
+#include <algorithm>
 #include <cstring>
 
 namespace pg {
@@ -42,13 +43,14 @@ constexpr int MOD3_THREADS = 1024;   // one block per SM: the tables take up to 
 constexpr int MOD3_LOW = 11;         // columns over word bits (5), lanes (5) and words (1)
 constexpr int MOD3_DIGITS = 81;      // states of a group of four rows' high sums
 
+constexpr unsigned long long MOD3_ABORTED = ~0ull;
 struct Mod3Args {
-    const uint64_t *cols;     // [2][n]: magnitude words, then sign words
+    uint64_t mags[64], sgns[64];   // the columns' magnitude and sign words
     int n;
-    uint64_t batches;         // 32 high states each
-    int steps;                // high states per batch: 32, fewer below order 16
-    unsigned long long *acc;  // zeroed
-    int *status;
+    uint64_t batches;         // 32 high states each (without tables: one)
+    // [gridDim], pinned host memory: each block's count (each warp's
+    // modulo 3), or MOD3_ABORTED
+    volatile unsigned long long *part;
     volatile const int *abort_flag;
 };
 
@@ -56,6 +58,13 @@ struct Mod3Args {
 __host__ __device__ constexpr int mod3_tables(int n) { return n > 20 && n <= 52 ? 6 : 5; }
 // per-row words [n][3][32] pairs; the lists hold six offsets a high state
 __host__ __device__ constexpr size_t mod3_row_bytes(int n) { return (size_t)n * 3 * 32 * 8; }
+// Few high states (up to 2^12, order 24): no tables, a high state a warp, every
+// row read in turn; building the tables took longer than the walk.  A call of
+// order 4..16 30 -> 15-18 us, 17..19 43 -> 19, 20..23 35 -> 21, about 10 of
+// them by passing the columns as arguments and leaving out both copies (the
+// row-sliced walk's: 20-23 us to order 19, 32 to 23).
+constexpr int MOD3_SHORT = 12;
+__host__ __device__ constexpr int mod3_threads(int GT) { return GT ? MOD3_THREADS : 256; }
 __host__ __device__ constexpr size_t mod3_smem(int n) {
     return (size_t)mod3_tables(n) * MOD3_DIGITS * 256 + 2 * mod3_row_bytes(n) + MOD3_THREADS * 24;
 }
@@ -83,7 +92,8 @@ __device__ __forceinline__ uint32_t mod3_pattern(int j) {
 }
 
 template <typename W, int GT>
-__global__ void __launch_bounds__(MOD3_THREADS, 1) mod3_kernel(Mod3Args a) {
+__global__ void __launch_bounds__(mod3_threads(GT), 1) mod3_kernel(const __grid_constant__ Mod3Args a) {
+    constexpr int THREADS = mod3_threads(GT);
     extern __shared__ uint4 mod3_shared[];
     const int n = a.n;
     uint2 *gtab = reinterpret_cast<uint2 *>(mod3_shared);            // [GT][81][32]
@@ -93,12 +103,12 @@ __global__ void __launch_bounds__(MOD3_THREADS, 1) mod3_kernel(Mod3Args a) {
     uint2 *lists2 = reinterpret_cast<uint2 *>(lists + MOD3_THREADS);
     __shared__ uint16_t dmap[256];      // (magnitudes | signs << 4) -> byte offset in a group
     __shared__ uint64_t cm_s[64], cs_s[64];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = MOD3_THREADS / 32;
-    for (int j = threadIdx.x; j < n; j += MOD3_THREADS) {
-        cm_s[j] = a.cols[j];
-        cs_s[j] = a.cols[n + j];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = THREADS / 32;
+    for (int j = threadIdx.x; j < n; j += THREADS) {
+        cm_s[j] = a.mags[j];
+        cs_s[j] = a.sgns[j];
     }
-    if (threadIdx.x < 256) {
+    if (GT > 0 && threadIdx.x < 256) {
         int idx = 0, p3 = 1;
         for (int t = 0; t < 4; t++, p3 *= 3)
             if ((threadIdx.x >> t) & 1) idx += p3 * (1 + ((threadIdx.x >> (t + 4)) & 1));
@@ -168,14 +178,15 @@ __global__ void __launch_bounds__(MOD3_THREADS, 1) mod3_kernel(Mod3Args a) {
     if (b_begin < b_end) {
         m = (W)cm_s[n - 1];
         s = (W)cs_s[n - 1];
-        const uint64_t minus = (uint64_t)lane | ((b_begin ^ (b_begin >> 1)) << 5);
+        // (without tables a batch is the one high state with the signs b)
+        const uint64_t minus = GT == 0 ? b_begin : (uint64_t)lane | ((b_begin ^ (b_begin >> 1)) << 5);
         for (int j = MOD3_LOW; j < n - 1; j++) {
             if ((minus >> (j - MOD3_LOW)) & 1) f3_sub(m, s, (W)cm_s[j], (W)cs_s[j]);
             else f3_add(m, s, (W)cm_s[j], (W)cs_s[j]);
         }
     }
 
-    // The states `alive` of high state k after the first 20 rows: the other
+    // The states `alive` of high state k after the tables' rows: the other
     // rows, then the signs.  Everything but the words is warp-uniform.
     auto finish = [&](int k, uint2 alive, uint32_t flip) {
         const W km = __shfl_sync(0xffffffffu, m, k), ks = __shfl_sync(0xffffffffu, s, k);
@@ -199,6 +210,10 @@ __global__ void __launch_bounds__(MOD3_THREADS, 1) mod3_kernel(Mod3Args a) {
                                       __popc(alive.y & neg.y));
     };
 
+    if constexpr (GT == 0) {
+        if (b_begin < b_end)
+            finish(0, make_uint2(exist, exist1), 0u - (uint32_t)(__popcll(b_begin) & 1));
+    } else
     for (uint64_t b = b_begin; b < b_end; b++) {
         if (b != b_begin) {
             // the host-mapped abort word is read once per 2^12 batches, from
@@ -220,11 +235,10 @@ __global__ void __launch_bounds__(MOD3_THREADS, 1) mod3_kernel(Mod3Args a) {
         list2[lane] = make_uint2(off[4] + 4 * GB, GT > 5 ? off[GT - 1] + (GT - 1) * GB : 0);
         __syncwarp();
         const uint32_t flip = 0u - (uint32_t)(b & 1);     // parity of gray(b)
-        for (int k0 = 0; k0 < a.steps; k0 += 4) {
+        for (int k0 = 0; k0 < 32; k0 += 4) {
             uint2 alive[4];
 #pragma unroll
             for (int t = 0; t < 4; t++) {
-                // beyond a.steps (below order 14) the list still holds valid offsets
                 const uint4 o = list[k0 + t];
                 const auto at = [&](uint32_t off) { return *reinterpret_cast<const uint2 *>(tab + off); };
                 const uint2 z0 = at(o.x), z1 = at(o.y), z2 = at(o.z), z3 = at(o.w);
@@ -239,13 +253,13 @@ __global__ void __launch_bounds__(MOD3_THREADS, 1) mod3_kernel(Mod3Args a) {
             }
 #pragma unroll
             for (int t = 0; t < 4; t++)
-                if (k0 + t < a.steps && __any_sync(0xffffffffu, (alive[t].x | alive[t].y) != 0))
+                if (__any_sync(0xffffffffu, (alive[t].x | alive[t].y) != 0))
                     finish(k0 + t, alive[t], flip);
         }
         __syncwarp();
     }
     count %= 3;
-    __shared__ unsigned long long red[MOD3_THREADS / 32];
+    __shared__ unsigned long long red[THREADS / 32];
     __shared__ int any_abort;
     if (threadIdx.x == 0) any_abort = 0;
     __syncthreads();
@@ -256,23 +270,23 @@ __global__ void __launch_bounds__(MOD3_THREADS, 1) mod3_kernel(Mod3Args a) {
     if (threadIdx.x == 0) {
         unsigned long long t = 0;
         for (int w = 0; w < warps; w++) t += red[w];
-        atomicAdd(a.acc, t);
-        if (any_abort) atomicExch(a.status, 1);
+        a.part[blockIdx.x] = any_abort ? MOD3_ABORTED : t;
     }
 }
 
 template <typename W, int GT>
-static cudaError_t launch_mod3(const Mod3Args &a, int sm_count, cudaStream_t s) {
-    const size_t smem = mod3_smem(a.n);
+static cudaError_t launch_mod3(const Mod3Args &a, int blocks, cudaStream_t s) {
+    const size_t smem = GT ? mod3_smem(a.n) : 2 * mod3_row_bytes(a.n);
     cudaError_t e = cudaFuncSetAttribute(mod3_kernel<W, GT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
-    const uint64_t blocks = a.batches < (uint64_t)sm_count ? a.batches : (uint64_t)sm_count;
-    mod3_kernel<W, GT><<<(unsigned)blocks, MOD3_THREADS, smem, s>>>(a);
+    mod3_kernel<W, GT><<<(unsigned)blocks, mod3_threads(GT), smem, s>>>(a);
     return cudaGetLastError();
 }
 
-// perm(A) mod 3 from the F_3 column encodings (n >= 3).
+// perm(A) mod 3 from the F_3 column encodings (n >= 3).  One launch and no
+// copies: the columns are kernel arguments, the blocks' counts go to pinned
+// host memory.
 static int mod3_impl(const uint64_t *mags, const uint64_t *sgns, int n, int *out) {
     DeviceInfo dev;
     int st = device_info(&dev);
@@ -280,37 +294,39 @@ static int mod3_impl(const uint64_t *mags, const uint64_t *sgns, int n, int *out
     volatile int *abort_dev;
     st = abort_flag_device(&abort_dev);
     if (st != PG_OK) return st;
-    const size_t off_acc = 2 * 64 * 8, off_status = off_acc + 64, total = off_status + 64;
-    Workspace *ws;
-    st = workspace(&ws, total, total);
-    if (st != PG_OK) return st;
-    char *h = (char *)ws->host;
-    char *d = (char *)ws->dev;
-    std::memset(h, 0, total);
-    std::memcpy(h, mags, (size_t)n * 8);
-    std::memcpy(h + (size_t)n * 8, sgns, (size_t)n * 8);
     const int high = n - 1 - MOD3_LOW;          // columns common to a warp
+    const bool tables = high > MOD3_SHORT;
     Mod3Args a;
-    a.cols = (const uint64_t *)d;
+    std::memcpy(a.mags, mags, (size_t)n * 8);
+    std::memcpy(a.sgns, sgns, (size_t)n * 8);
     a.n = n;
-    a.batches = high > 5 ? 1ull << (high - 5) : 1;
-    a.steps = high >= 5 ? 32 : high > 0 ? 1 << high : 1;
-    a.acc = (unsigned long long *)(d + off_acc);
-    a.status = (int *)(d + off_status);
+    // (without tables a batch is one high state)
+    a.batches = high <= 0 ? 1 : tables ? 1ull << (high - 5) : 1ull << high;
+    const uint64_t warps = mod3_threads(tables) / 32;
+    const uint64_t most = tables ? (uint64_t)dev.sm_count : a.batches;
+    const int blocks = (int)std::min((a.batches + (tables ? 1 : warps) - 1) / (tables ? 1 : warps), most);
+    Workspace *ws;
+    st = workspace(&ws, 0, (size_t)blocks * 8);
+    if (st != PG_OK) return st;
+    void *part;
+    PG_CUDA(cudaHostGetDevicePointer(&part, ws->host, 0));
+    a.part = (volatile unsigned long long *)part;
     a.abort_flag = abort_dev;
-    PG_CUDA(cudaMemcpyAsync(d, h, total, cudaMemcpyHostToDevice, ws->stream));
     const bool six = mod3_tables(n) == 6;
-    if (n <= 32 && six) PG_CUDA((launch_mod3<uint32_t, 6>(a, dev.sm_count, ws->stream)));
-    else if (n <= 32) PG_CUDA((launch_mod3<uint32_t, 5>(a, dev.sm_count, ws->stream)));
-    else if (six) PG_CUDA((launch_mod3<uint64_t, 6>(a, dev.sm_count, ws->stream)));
-    else PG_CUDA((launch_mod3<uint64_t, 5>(a, dev.sm_count, ws->stream)));
-    PG_CUDA(cudaMemcpyAsync(h + off_acc, d + off_acc, total - off_acc, cudaMemcpyDeviceToHost,
-                            ws->stream));
+    if (!tables) PG_CUDA((launch_mod3<uint32_t, 0>(a, blocks, ws->stream)));
+    else if (n <= 32 && six) PG_CUDA((launch_mod3<uint32_t, 6>(a, blocks, ws->stream)));
+    else if (n <= 32) PG_CUDA((launch_mod3<uint32_t, 5>(a, blocks, ws->stream)));
+    else if (six) PG_CUDA((launch_mod3<uint64_t, 6>(a, blocks, ws->stream)));
+    else PG_CUDA((launch_mod3<uint64_t, 5>(a, blocks, ws->stream)));
     PG_CUDA(cudaStreamSynchronize(ws->stream));
-    if (*(int *)(h + off_status)) return fail(PG_EABORT, "launch aborted by pg_abort()");
+    unsigned long long total = 0;
+    for (int i = 0; i < blocks; i++) {
+        const unsigned long long v = ((const unsigned long long *)ws->host)[i];
+        if (v == MOD3_ABORTED) return fail(PG_EABORT, "launch aborted by pg_abort()");
+        total += v;
+    }
     // 2^(1-n) = (-1)^(n-1) modulo 3
-    const unsigned long long total3 = *(unsigned long long *)(h + off_acc) % 3;
-    *out = (int)((n & 1) ? total3 : (3 - total3) % 3);
+    *out = (int)((n & 1) ? total % 3 : (3 - total % 3) % 3);
     return PG_OK;
 }
 
