@@ -758,15 +758,13 @@ def run_gpu_float28(args, world, rank, local):
     fwd_ms = statistics.mean(ms_fwd)
     cpu = cpu_f64_sample(A_host, args.cpu_seconds) if rank == 0 and not args.no_cpu else None
     # roofline: FP32-pipe instructions of the algorithm per state, counted
-    # from the kernel source for the n live rows (lanes): one double-float
-    # add per row update (11 FP32 instructions), 5 double-float products in
-    # the butterfly for the full product (7 each), one double-float division
-    # for the all-but-self product (10 FP32 instructions and a reciprocal),
-    # one add for the forward term and 1 + M (M = 4) for the gradient
-    # columns; the forward-only walk drops the division and 5 adds
-    df_add, df_mul, df_div = 11, 7, 10
-    fwd_bwd_ops = n * (df_add * (1 + 1 + 1 + 4) + df_mul * 5 + df_div)
-    fwd_ops = n * (df_add * 2 + df_mul * 5)
+    # from the kernel sources for the n rows.  Forward: three grid additions,
+    # a renormalisation (4) and one chain product (4) a row.  Gradient: three
+    # additions, a renormalisation, three products (7 each), the difference
+    # tree's additions and the first four columns (18), 46 a row; a call with
+    # the gradient runs the forward walk as well
+    fwd_ops = 11 * n
+    fwd_bwd_ops = 46 * n + fwd_ops
     achieved = states * fwd_bwd_ops / (step_ms * 1e-3)
     achieved_fwd = states * fwd_ops / (fwd_ms * 1e-3)
     if rank == 0:
@@ -775,7 +773,7 @@ def run_gpu_float28(args, world, rank, local):
             "value": world * states / (step_ms * 1e-3), "unit": "steps/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": step_ms,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "f64 (double-float on FP32 pipes, FP64 re-initialisation and Kahan flushes)",
+            "dtype": "f64 (exact FP32-grid row sums, double-float products, FP64 Kahan sums)",
             "data": "synthetic",
             "config": {"workload": "float28: 256 float64 matrices 28x28, entries N(0,1/28), "
                                    "numpy default_rng(5)", "states": states,
@@ -804,7 +802,7 @@ def run_gpu_float28(args, world, rank, local):
                     "h2d_bytes_per_step": int(A_host.nbytes),
                     "d2h_bytes_per_step": int(batch * 8 + A_host.nbytes),
                     "ms_per_step": 1e3 * e2e_s},
-            "clocks": clk, "gpu_launches": 2 * args.steps,
+            "clocks": clk, "gpu_launches": 4 * args.steps,    # two walks, two reductions
         }))
 
 
@@ -828,14 +826,14 @@ def run_gpu_poly(args, world, rank, local):
     bounds = poly._bounds(tuple((1,) * n for _ in range(n)), am)
     primes = poly._gpu_primes(max(bounds))
     states = len(primes) * (1 << (n - 1))
-    # C = J has equal rows, so the uniform kernel runs: per state the
-    # elementary-symmetric recurrence (factor r = 1..n-1: r Montgomery
-    # products), n - 1 powers of the common row sum and n weighted
-    # coefficients, n(n-1)/2 + 2n - 1 Montgomery products of mul.wide,
-    # mul.lo and mad.wide each; every 32x32->64 product is weighted by the
-    # measured mul.wide : mad.lo ratio
-    redc_per_state = n * (n - 1) // 2 + 2 * n - 1
-    imad_per_state = 3 * redc_per_state
+    # C = J and small row sums of L, so the exact kernel runs: one walk for
+    # all moduli, the elementary-symmetric recurrence E[d] += l_r E[d-1] on
+    # digits of 26 bits (E_r[d] bounded by C(r, d) B^d), one mad.lo a digit
+    top = int(a.sum(1).max())
+    top = next(b for b in (15, 20, 31) if top <= b)
+    imad_per_state = sum(
+        1 if d == 1 else -(-(math.comb(r - 1, d - 1) * top ** (d - 1)).bit_length() // 26)
+        for r in range(1, n + 1) for d in range(1, r + 1))
     for _ in range(args.warmup):
         got = permgpu.rook_polynomial(a.tolist())
         _lib.affine_residues(ones, a, primes)
@@ -843,8 +841,6 @@ def run_gpu_poly(args, world, rank, local):
         raise SystemExit("rook polynomial failed its r_1 = #ones check")
     peak_lo = _lib.probe_int_throughput(0)
     peak = peak_lo / 1e12                         # mad.lo.u32 ops/s -> Tops/s
-    w = peak_lo / _lib.probe_int_throughput(4)    # mul.wide.u32 weight
-    slots_per_state = redc_per_state * (2 * w + 1)
     clocks = ClockSampler(local).start()
     barrier(world)
     ts, te = [], []
@@ -882,12 +878,12 @@ def run_gpu_poly(args, world, rank, local):
                          f"{len(primes)} primes x 2^{n - 1} states",
                "time_to_exact_s_est": states / per_prime}
     if rank == 0:
-        achieved = states * slots_per_state / step_s / 1e12
+        achieved = (1 << (n - 1)) * imad_per_state / step_s / 1e12
         print(json.dumps({
             "metric": "polynomial Glynn prime-states/s (rook28)", "value": world * states / step_s,
             "unit": "prime-states/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": 1e3 * step_s, "higher_is_better": True,
-            "scaling": "weak", "vs_baseline": None, "dtype": "u32 Montgomery",
+            "scaling": "weak", "vs_baseline": None, "dtype": "exact integers, 26-bit digits",
             "data": "synthetic",
             "config": {"workload": "rook28: rook polynomial of a 28x28 Bernoulli(0.5) 0/1 "
                                    "matrix, numpy default_rng(28)", "crt_primes": len(primes),
@@ -896,8 +892,7 @@ def run_gpu_poly(args, world, rank, local):
             "roofline": {"bound": "imad", "achieved": achieved, "peak": peak, "unit": "Tops/s",
                          "frac": achieved / peak, "traffic": None,
                          "peak_source": "measured live: pg_probe_int_throughput mad.lo.u32",
-                         "work_per_state": {"imad_class_instructions": imad_per_state,
-                                            "wide_weight": w, "slots": slots_per_state}},
+                         "work_per_state": {"mad_lo": imad_per_state}},
             "cpu_baseline": cpu,
             "e2e": {"value": world * states / e2e_s, "unit": "prime-states/s",
                     "h2d_bytes_per_step": 2 * 8 * n * n, "d2h_bytes_per_step": 8 * (n + 1) * len(primes),
@@ -908,9 +903,9 @@ def run_gpu_poly(args, world, rank, local):
 
 def run_gpu_mod3(args, world, rank, local):
     """mod3_40: per(A) mod 3 of a 40x40 matrix with entries U{0,1,2}, numpy
-    default_rng(40 + rank), through permgpu.mod3.permanent_mod3_fast (Ryser
-    over F_3 with bit-sliced row sums, one launch).  value = subsets per
-    second (2^40 per evaluation); the call is timed from the host matrix to
+    default_rng(40 + rank), through permgpu.mod3.permanent_mod3_fast (Glynn
+    over F_3, one launch).  value = subsets per second (2^40 per evaluation,
+    as a Ryser walk counts them); the call is timed from the host matrix to
     the returned residue, so value and e2e coincide."""
     import numpy as np
     import torch
@@ -952,13 +947,11 @@ def run_gpu_mod3(args, world, rank, local):
                          "threads (bit-sliced F_3 Ryser, restatement of perm_mod3_omp.c:54-160)",
                "time_to_result_s_est": states / cpu_rate}
     if rank == 0:
-        # per subset: one 64-bit column update (3 three-input bitwise ops on
-        # two words), the full-magnitude test and a popcount
         print(json.dumps({
             "metric": f"Ryser subsets/s (perm mod 3, {n}x{n})", "value": world * states / step_s,
             "unit": "subsets/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
             "ms_per_step": 1e3 * step_s, "higher_is_better": True, "scaling": "weak",
-            "vs_baseline": None, "dtype": "F_3 bit-sliced (u64 words)", "data": "synthetic",
+            "vs_baseline": None, "dtype": "F_3 (two bits an element)", "data": "synthetic",
             "config": {"workload": f"mod3_40: {n}x{n} matrix, entries U{{0,1,2}}, numpy "
                                    f"default_rng({n})", "subsets": states},
             "time_to_result_s": step_s, "result": got, "cpu_baseline": cpu,

@@ -28,7 +28,7 @@
 // Bound by shared-memory loads (95 % of their rate): 17 wavefronts per 2048
 // states.  35 x 35 random, a call: 22.9 ms with the row-sliced Ryser walk
 // (17.5 instructions per subset, ALU pipe 91 % busy), 0.67 ms with single
-// words and tables for every row group, 0.66 with five groups, 0.52 now.  A
+// words and tables for every row group, 0.66 with five groups, 0.51 now.  A
 // matrix whose states all survive (equal rows) reads every row's words for
 // every high state, ~14 instructions per row and 2048 states, still well below
 // the row-sliced walk, so no other path is kept.
