@@ -496,7 +496,11 @@ struct NkQueue {
     }
 };
 
-constexpr int NK_QUEUE = 4;        // accepted words a lane may hold
+// accepted words a lane may hold: a longer queue costs more moves per round
+// than its fewer idle lanes save (one residue of S_37 29.6 ms with 4, 28.8 with
+// 3, 27.9 with 2, 29.1 with 1; S_41 405 -> 390 ms with 2).  Reading the middle
+// byte's table row per term instead of following its changes: 30.7 ms.
+constexpr int NK_QUEUE = 2;
 constexpr int NK_WALK_STEPS = 3;   // walker steps per evaluation (about 2.5 steps per word)
 
 // Resident blocks per SM requested from ptxas for orders up to 42: three
