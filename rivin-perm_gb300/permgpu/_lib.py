@@ -413,8 +413,12 @@ class ExactPlan:
 
 def pack_batch(matrices):
     """(A_packed int64, offsets int64, orders int32) for a list of square
-    integer matrices."""
+    integer matrices; ValueError for one that is not square (the offsets and
+    the native code count order**2 words)."""
     mats = [np.asarray(m, dtype=np.int64) for m in matrices]
+    for m in mats:
+        if m.ndim == 2 and m.size != m.shape[0] ** 2:
+            raise ValueError("matrix must be square")
     orders = np.array([m.shape[0] if m.ndim == 2 else 0 for m in mats], dtype=np.int32)
     sizes = orders.astype(np.int64) ** 2
     offsets = np.zeros(len(mats), dtype=np.int64)

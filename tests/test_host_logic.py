@@ -237,3 +237,24 @@ def test_matching_and_blocks_against_brute_force():
         if feasible:
             assert sum(len(b) for b in blocks) == k
             assert all(brute(b) > 0 for b in blocks)
+
+
+@pytest.mark.parametrize("shape", [(2, 3), (3, 2), (1, 0), (1, 5), (4, 1)])
+@pytest.mark.parametrize("at", [0, 1])
+def test_pack_batch_refuses_matrices_that_are_not_square(shape, at):
+    # offsets and orders count order^2 words: any other size would shift the
+    # matrices behind it or let the native code read past the packed words
+    from permgpu import _lib
+    mats = [np.arange(4).reshape(2, 2), np.ones((5, 5), dtype=np.int64)]
+    mats.insert(at, np.ones(shape, dtype=np.int64))
+    for call in (_lib.pack_batch, _lib.batch_limbs, _lib.batch_exact, _lib.BatchPlan):
+        with pytest.raises(ValueError):
+            call(mats)
+
+
+def test_pack_batch_layout():
+    from permgpu import _lib
+    mats = [np.arange(4).reshape(2, 2), np.zeros((0, 0)), [[7]], np.arange(9).reshape(3, 3).T]
+    packed, offsets, orders = _lib.pack_batch(mats)
+    assert orders.tolist() == [2, 0, 1, 3] and offsets.tolist() == [0, 4, 4, 5]
+    assert packed.tolist() == [0, 1, 2, 3, 7, 0, 3, 6, 1, 4, 7, 2, 5, 8]
