@@ -173,7 +173,8 @@ __global__ void __launch_bounds__(32 * FWD_WARPS) glynn_forward_kernel(FwdArgs a
     bool aborted = false;
     const uint64_t first = (uint64_t)part * FWD_WARPS + warp;
     for (uint64_t k = first; k < blocks; k += (uint64_t)a.blocks_per * FWD_WARPS) {
-        if (k != first && *a.abort_flag) { aborted = true; break; }
+        // voted: the lanes must leave the loop together
+        if (k != first && __any_sync(0xffffffffu, *a.abort_flag != 0)) { aborted = true; break; }
         const uint64_t g0 = (k << a.log_block) + ((uint64_t)(active ? lane : 0) << R);
         float s[C][N];
 #pragma unroll

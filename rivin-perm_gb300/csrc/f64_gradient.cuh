@@ -189,7 +189,8 @@ __global__ void __launch_bounds__(32 * GRAD_WARPS, 2) glynn_gradient_kernel(Grad
     bool aborted = false;
     const uint64_t first = (uint64_t)part * GRAD_WARPS + warp;
     for (uint64_t k = first; k < tasks; k += (uint64_t)a.blocks_per * GRAD_WARPS) {
-        if (k != first && *a.abort_flag) { aborted = true; break; }
+        // voted: the lanes must leave the loop together
+        if (k != first && __any_sync(0xffffffffu, *a.abort_flag != 0)) { aborted = true; break; }
         const uint64_t g0 = active ? ((k << LW) + w) << R : 0;
         // row sums of two states: u (column 0 plus) and v (column 0 minus)
         f2 s[3][RW];

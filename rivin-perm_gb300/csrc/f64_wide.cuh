@@ -96,7 +96,8 @@ __global__ void __launch_bounds__(128) glynn_wide_kernel(WideArgs a) {
     double sre = 0.0, cre = 0.0, sim = 0.0, cim = 0.0, asum = 0.0;
     bool aborted = false;
     for (uint64_t g0 = g_begin; g0 < g_end; g0 += block_len) {
-        if (*a.abort_flag) { aborted = true; break; }
+        // voted: the lanes must leave the loop together
+        if (__any_sync(0xffffffffu, *a.abort_flag != 0)) { aborted = true; break; }
         const uint64_t g1 = g_end - g0 < block_len ? g_end : g0 + block_len;
         // exact FP64 row sums at g0 (rows beyond N: s = 1, table entries 0)
         const uint64_t gr = g0 ^ (g0 >> 1);

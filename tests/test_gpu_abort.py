@@ -87,3 +87,46 @@ def test_abort_flag_left_set_stops_the_next_launch_at_once(lib):
         h.pg_clear_abort()
     c = np.random.default_rng(9).integers(-8, 9, (20, 20), dtype=np.int64)
     assert lib.exact_permanent(c, lib.exact_limbs(c)) == oracle.exact_permanent(c.tolist())
+
+
+def _raised_before(lib, fn):
+    # status of a call that starts with the word already raised
+    lib.load().pg_abort()
+    try:
+        with pytest.raises(lib.PermGpuError) as err:
+            fn()
+    finally:
+        lib.load().pg_clear_abort()
+    return err.value.status
+
+
+def _fp64(kind, n, batch):
+    import torch
+    from permgpu import f64
+    a = torch.from_numpy(np.random.default_rng(n).normal(0, n ** -0.5, (batch, n, n))).cuda()
+    if kind == "complex":
+        return f64.permanent_c64(a.to(torch.complex128) * (1 - 0.5j))
+    return f64.permanent_f64(a, want_grad=kind == "gradient")
+
+
+@pytest.mark.parametrize("kind,n,batch", [
+    ("forward", 32, 1), ("complex", 30, 1), ("gradient", 28, 1),    # several ranges a warp
+    ("forward", 34, 1), ("complex", 34, 1),                         # the kernel of orders 33..63
+])
+def test_abort_word_raised_before_fp64_walks(lib, kind, n, batch):
+    # the lanes of a warp vote on the word and leave together: a status, not a
+    # partial sum, and the next call is right again
+    want = [x.cpu() for x in _fp64(kind, 12, 2) if x is not None]
+    assert _raised_before(lib, lambda: _fp64(kind, n, batch)) == lib.PG_EABORT
+    got = [x.cpu() for x in _fp64(kind, 12, 2) if x is not None]
+    assert all((x == y).all() for x, y in zip(want, got))
+
+
+@pytest.mark.parametrize("kind,n,batch", [("forward", 30, 512), ("complex", 28, 512),
+                                          ("gradient", 28, 512)])
+def test_abort_fp64_walks(lib, kind, n, batch):
+    # two to four seconds uninterrupted
+    lib.load().pg_clear_abort()
+    status, took = _aborted_after(lib, lambda: _fp64(kind, n, batch))
+    assert status == lib.PG_EABORT
+    assert took < 1.5
