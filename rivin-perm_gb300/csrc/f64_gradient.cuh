@@ -25,6 +25,13 @@
 // adds its walkers' sums (shuffles, double-float) and folds them into the
 // warp's FP64 Kahan sums in global memory.
 //
+// Where a warp's walkers cover a whole matrix in one range each (orders up to
+// GRAD_WHOLE_N) a thread block is one warp, takes one matrix and writes its
+// gradient itself: no slots and no reduction.  Four warps on one matrix left
+// three of them idle and cost slots that were zeroed and reduced: 65536
+// matrices 5x5 3.72 -> 0.76 ms, 8x8 7.86 -> 1.38, 14x14 48.1 -> 17.9 (a lane
+// per row: 0.73, 1.96, 97.9), 16 of order 4 95 -> 73 us (77).
+//
 // FP32-pipe bound: about 46 operations per row and state.  16 x 26x26 with
 // the forward walk: 114.3 -> 37.9 ms against a lane per row with a shuffle
 // butterfly for the product and a double-float division per row for E_i;
@@ -41,12 +48,15 @@ struct GradArgs {
     int blocks_per;            // thread blocks per matrix
     int log_range;             // 2^R states of a walker's range, R <= GradShape::RMAX
     double *slots;             // [batch][blocks_per][GRAD_WARPS][grad_slot(n)], zeroed
+    double *grad, *grad_abs;   // results of the one-warp blocks (grad_abs may be null)
     volatile const int *abort_flag;
     int *status;
 };
 
 constexpr int GRAD_WARPS = 4;  // warps of a thread block
 constexpr int GRAD_TREE = 4;   // levels of the pairwise tree
+constexpr int GRAD_WHOLE_N = 14;   // largest order whose matrices a warp can take whole
+constexpr int GRAD_SPLIT_N = 11;   // smallest order with more than one range a walker
 
 // per-warp slot: per entry the Kahan sum and its compensation, then the
 // rows' sums of |E|
@@ -55,18 +65,21 @@ __host__ __device__ constexpr int grad_slot(int n) { return 2 * n * n + n; }
 template <int N>
 struct GradShape {
     static constexpr int LP = N <= 8 ? 0 : N <= 16 ? 1 : 2;    // log2 of a walker's lanes
-    static constexpr int P = 1 << LP, LW = 5 - LP, WK = 1 << LW;
+    // log2 of a warp's walkers, each with two states or more (fewer than 32
+    // lanes work below order 7)
+    static constexpr int P = 1 << LP, LW = N - 2 < 5 - LP ? N - 2 : 5 - LP, WK = 1 << LW;
     static constexpr int RW = (N + P - 1) / P;
     static constexpr int RP = (RW + 3) & ~3;
     static constexpr int COL = P * 3 * RP;                     // floats of a column
     // two blocks of 128 threads per SM: (RMAX + waiting slots) rows of 8
     // bytes per thread and the table in 113 KB
     static constexpr int RCAP = RW == 8 ? 8 : 10;
-    static constexpr int RMAX = N - 1 - LW < 1 ? 1 : N - 1 - LW < RCAP ? N - 1 - LW : RCAP;
+    static constexpr int RMAX = N - 1 - LW < RCAP ? N - 1 - LW : RCAP;
     static constexpr int WAIT = LW + 1 > GRAD_TREE - 1 ? LW + 1 : GRAD_TREE - 1;
     static constexpr int SLOTS = RMAX + WAIT;
-    static constexpr size_t smem =
-        sizeof(float) * (size_t)N * COL + (size_t)SLOTS * RW * 32 * GRAD_WARPS * sizeof(float2);
+    static constexpr size_t smem(int warps) {
+        return sizeof(float) * (size_t)N * COL + (size_t)SLOTS * RW * 32 * warps * sizeof(float2);
+    }
 };
 
 // sum += f x, f = +-1
@@ -135,11 +148,13 @@ __device__ __forceinline__ df2 df2_shfl_xor(df2 a, int off) {
     return df2{f2_shfl_xor(a.hi, off), f2_shfl_xor(a.lo, off)};
 }
 
-template <int N>
-__global__ void __launch_bounds__(32 * GRAD_WARPS, 2) glynn_gradient_kernel(GradArgs a) {
+// WARPS = GRAD_WARPS: slots for the reduction; 1: a matrix a block, the result
+template <int N, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, 8 / WARPS) glynn_gradient_kernel(GradArgs a) {
     using S = GradShape<N>;
+    constexpr bool WHOLE = WARPS == 1;
     constexpr int P = S::P, RW = S::RW, RP = S::RP, COL = S::COL, WK = S::WK, LW = S::LW;
-    constexpr int BL = fwd_bound_log(false), BT = 32 * GRAD_WARPS;
+    constexpr int BL = fwd_bound_log(false), BT = 32 * WARPS;
     extern __shared__ float4 grad_smem[];
     float *tab = reinterpret_cast<float *>(grad_smem);   // [N][P][3][RP]; column N-1: all-plus sums
     __shared__ int row_exp[N];
@@ -148,7 +163,8 @@ __global__ void __launch_bounds__(32 * GRAD_WARPS, 2) glynn_gradient_kernel(Grad
     // this thread's column of the slots: slot t, row r at [(t RW + r) BT]
     float2 *mine = reinterpret_cast<float2 *>(tab + N * COL) + threadIdx.x;
     const float2 *warp0 = mine - lane;
-    const int b = blockIdx.x / a.blocks_per, part = blockIdx.x - b * a.blocks_per;
+    const int b = WHOLE ? blockIdx.x : blockIdx.x / a.blocks_per;
+    const int part = WHOLE ? 0 : blockIdx.x - b * a.blocks_per;
     const double *A = a.A + (size_t)b * N * N;
     for (int r = threadIdx.x; r < N; r += BT) row_exp[r] = fwd_row_exponent(A + r * N, nullptr, N, BL);
     __syncthreads();
@@ -177,18 +193,20 @@ __global__ void __launch_bounds__(32 * GRAD_WARPS, 2) glynn_gradient_kernel(Grad
     __syncthreads();
 
     const int R = a.log_range, M = R < GRAD_TREE ? R : GRAD_TREE;
-    // where there are fewer ranges than walkers the others are idle
-    const bool active = N - 1 - R >= LW || w < (1 << (N - 1 - R));
-    const uint64_t states = 1ull << (N - 1);
-    const uint64_t tasks = states >> R >> LW ? states >> R >> LW : 1;
-    double *slot = a.slots + ((size_t)blockIdx.x * GRAD_WARPS + warp) * grad_slot(N);
+    const bool active = w < WK;
+    const uint64_t tasks = 1ull << (N - 1 - R - LW);
+    double *slot = WHOLE ? nullptr : a.slots + ((size_t)blockIdx.x * WARPS + warp) * grad_slot(N);
+    int exps = 0;              // of all rows; E_i was formed from the rows l != i
+    if (WHOLE)
+        for (int r = 0; r < N; r++) exps += row_exp[r];
+    auto unscaled = [&](double v, int row) { return ldexp(v, row_exp[row] - exps - (N - 1)); };
     const float *own = tab + p * 3 * RP;
     double gabs[RW];
 #pragma unroll
     for (int r = 0; r < RW; r++) gabs[r] = 0.0;
     bool aborted = false;
-    const uint64_t first = (uint64_t)part * GRAD_WARPS + warp;
-    for (uint64_t k = first; k < tasks; k += (uint64_t)a.blocks_per * GRAD_WARPS) {
+    const uint64_t first = (uint64_t)part * WARPS + warp;
+    for (uint64_t k = first; k < (WHOLE ? 1 : tasks); k += (uint64_t)a.blocks_per * WARPS) {
         // voted: the lanes must leave the loop together
         if (k != first && __any_sync(0xffffffffu, *a.abort_flag != 0)) { aborted = true; break; }
         const uint64_t g0 = active ? ((k << LW) + w) << R : 0;
@@ -332,26 +350,38 @@ __global__ void __launch_bounds__(32 * GRAD_WARPS, 2) glynn_gradient_kernel(Grad
 
         // The walkers' sums, added over the warp; lanes of walker 0 leave
         // them in their slots: columns 0..R-1, then the total W signed by
-        // each of the LW columns that differ between walkers, then W.
+        // each of the LW columns that differ between walkers, then W.  Those
+        // come by pairs, as in the tree: two walkers of a pair (halves of a
+        // pair of pairs, ...) have opposite signs of the level's column.
         if (!active) {
 #pragma unroll
             for (int r = 0; r < RW; r++) V0[r] = WT[r] = df{0.f, 0.f};
         }
-        auto total = [&](df v, float f) {
-            v = df{f * v.hi, f * v.lo};
-#pragma unroll
-            for (int o = P; o < 32; o <<= 1) v = df_add(v, df_shfl_xor(v, o));
-            return v;
-        };
-        const uint64_t gw = g0 ^ (g0 >> 1);
 #pragma unroll
         for (int r = 0; r < RW; r++) {
-            for (int t = 0; t < R + LW + 1; t++) {
-                float2 &vv = mine[((t < R ? t : S::RMAX + t - R) * RW + r) * BT];
-                const bool neg = t >= R && t < R + LW && ((gw >> t) & 1);
-                const df v = total(t == 0 ? V0[r] : t < R ? df{vv.x, vv.y} : WT[r],
-                                   neg ? -1.f : 1.f);
+            for (int t = 0; t < R; t++) {
+                float2 &vv = mine[(t * RW + r) * BT];
+                df v = t == 0 ? V0[r] : df{vv.x, vv.y};
+#pragma unroll
+                for (int l = 0; l < LW; l++) v = df_add(v, df_shfl_xor(v, P << l));
                 if (w == 0) vv = make_float2(v.hi, v.lo);
+            }
+            df d[LW > 0 ? LW : 1], v = WT[r];
+#pragma unroll
+            for (int l = 0; l < LW; l++) {
+#pragma unroll
+                for (int t = 0; t < l; t++) d[t] = df_add(d[t], df_shfl_xor(d[t], P << l));
+                const df o = df_shfl_xor(v, P << l);
+                // column R + l is minus where the bits of g at it and above differ
+                const bool neg = (((g0 >> (R + l)) ^ (g0 >> (R + l + 1))) & 1) != 0;
+                d[l] = df_add(neg ? df_neg(v) : v, neg ? o : df_neg(o));
+                v = df_add(v, o);
+            }
+            if (w == 0) {
+#pragma unroll
+                for (int t = 0; t < LW; t++)
+                    mine[((S::RMAX + t) * RW + r) * BT] = make_float2(d[t].hi, d[t].lo);
+                mine[((S::RMAX + LW) * RW + r) * BT] = make_float2(v.hi, v.lo);
             }
         }
         __syncwarp();
@@ -362,6 +392,10 @@ __global__ void __launch_bounds__(32 * GRAD_WARPS, 2) glynn_gradient_kernel(Grad
             const float2 v = warp0[(t * RW + rr) * BT + ln];
             double x = (double)v.x + (double)v.y;
             if (j < N - 1 && j >= R + LW && ((gtm >> j) & 1)) x = -x;
+            if constexpr (WHOLE) {
+                a.grad[(size_t)b * N * N + e] = unscaled(x, i);
+                continue;
+            }
             double sm = slot[e], cp = slot[N * N + e];
             kahan(sm, cp, x);
             slot[e] = sm;
@@ -372,26 +406,42 @@ __global__ void __launch_bounds__(32 * GRAD_WARPS, 2) glynn_gradient_kernel(Grad
         for (int r = 0; r < RW; r++) gabs[r] += active ? (double)ga[r] : 0.0;
     }
 #pragma unroll
-    for (int o = P; o < 32; o <<= 1)
+    for (int o = P; o < P << LW; o <<= 1)
 #pragma unroll
         for (int r = 0; r < RW; r++) gabs[r] += __shfl_xor_sync(0xffffffffu, gabs[r], o);
     if (lane == 0 && aborted) atomicExch(a.status, 1);
-    if (w == 0)
+    if (w != 0) return;
 #pragma unroll
-        for (int r = 0; r < RW; r++)
-            if (p * RW + r < N) slot[2 * N * N + p * RW + r] = gabs[r];
+    for (int r = 0; r < RW; r++) {
+        const int row = p * RW + r;
+        if (row >= N) continue;
+        if constexpr (!WHOLE) slot[2 * N * N + row] = gabs[r];
+        else if (a.grad_abs) a.grad_abs[(size_t)b * N + row] = unscaled(gabs[r], row);
+    }
 }
 
-template <int N>
-cudaError_t launch_glynn_gradient(const GradArgs &a, cudaStream_t s) {
-    constexpr size_t smem = GradShape<N>::smem;
+template <int N, int WARPS>
+cudaError_t launch_glynn_gradient_warps(const GradArgs &a, cudaStream_t s) {
+    constexpr size_t smem = GradShape<N>::smem(WARPS);
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(glynn_gradient_kernel<N>,
+        cudaError_t e = cudaFuncSetAttribute(glynn_gradient_kernel<N, WARPS>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    glynn_gradient_kernel<N><<<(unsigned)(a.batch * a.blocks_per), 32 * GRAD_WARPS, smem, s>>>(a);
+    glynn_gradient_kernel<N, WARPS>
+        <<<(unsigned)(a.batch * a.blocks_per), 32 * WARPS, smem, s>>>(a);
     return cudaGetLastError();
+}
+// a.slots null: one-warp blocks, which need one range a walker at most
+template <int N>
+cudaError_t launch_glynn_gradient(const GradArgs &a, cudaStream_t s) {
+    if constexpr (N <= GRAD_WHOLE_N) {
+        if (!a.slots) return launch_glynn_gradient_warps<N, 1>(a, s);
+    }
+    if constexpr (N >= GRAD_SPLIT_N) {
+        if (a.slots) return launch_glynn_gradient_warps<N, GRAD_WARPS>(a, s);
+    }
+    return cudaErrorInvalidValue;
 }
 
 // log2 of a warp's walkers and of the longest range at order n

@@ -47,7 +47,7 @@ __global__ void glynn_forward_reduce(const double *Are, const double *Aim, const
 
 // Launch shape of the forward walk of `batch` matrices of order 2..32 (Aim
 // null: real): fills a.batch, a.log_block, a.blocks_per; returns the slots'
-// bytes.
+// bytes, 0 where a warp takes a whole real matrix and writes its result.
 static size_t forward_shape(const double *Are, const double *Aim, int batch, int n, int sms,
                             FwdArgs *out) {
     FwdArgs &a = *out;
@@ -65,17 +65,21 @@ static size_t forward_shape(const double *Are, const double *Aim, int batch, int
     // same number of blocks of states
     const uint64_t tasks = 1ull << (n - 1 - a.log_block);
     a.blocks_per = 1;
+    if (!Aim && tasks == 1) return 0;
     while ((uint64_t)a.blocks_per * FWD_WARPS < tasks &&
            (uint64_t)batch * a.blocks_per * 2 <= (uint64_t)sms * 64)
         a.blocks_per *= 2;
     return (size_t)batch * a.blocks_per * FWD_WARPS * FWD_SLOT * sizeof(double);
 }
 
-// The walk and its reduction, asynchronous on s.
-static int forward_launch(const FwdArgs &a, int n, double *re, double *im, double *abs_sum,
+// The walk and its reduction, asynchronous on s; a.slots null: no slots.
+static int forward_launch(FwdArgs a, int n, double *re, double *im, double *abs_sum,
                           cudaStream_t s) {
+    a.re = re;
+    a.abs_sum = abs_sum;
     PG_CUDA(!a.Aim ? launch_forward_real(n, a, s)
             : n <= 22 ? launch_forward_cplx_lo(n, a, s) : launch_forward_cplx_hi(n, a, s));
+    if (!a.slots) return PG_OK;
     glynn_forward_reduce<<<a.batch, 32, 0, s>>>(a.Are, a.Aim, a.slots, n, a.blocks_per * FWD_WARPS,
                                                 re, im, abs_sum);
     PG_CUDA(cudaGetLastError());
@@ -100,13 +104,13 @@ static int glynn_forward_run(const double *Are, const double *Aim, int batch, in
     volatile int *abort_dev;
     st = abort_flag_device(&abort_dev);
     if (st != PG_OK) return st;
-    const size_t bytes = forward_shape(Are, Aim, batch, n, dev.sm_count, &a) + 256;
+    const size_t bytes = forward_shape(Are, Aim, batch, n, dev.sm_count, &a);
     Workspace *ws;
-    st = workspace(&ws, bytes, 64);
+    st = workspace(&ws, bytes + 256, 64);
     if (st != PG_OK) return st;
     cudaStream_t s = stream ? stream : ws->stream;
     a.status = (int *)ws->dev;
-    a.slots = (double *)((char *)ws->dev + 256);
+    a.slots = bytes ? (double *)((char *)ws->dev + 256) : nullptr;
     a.abort_flag = abort_dev;
     PG_CUDA(cudaMemsetAsync(a.status, 0, sizeof(int), s));
     if ((st = forward_launch(a, n, re, im, abs_sum, s)) != PG_OK) return st;
@@ -174,11 +178,28 @@ static int glynn_gradient_run(const double *A, int batch, int n, double *per, do
     while (a.log_range > 5 &&
            (uint64_t)batch * tasks_of(a.log_range) < 2 * GRAD_WARPS * resident)
         a.log_range--;
+    const uint64_t tasks = tasks_of(a.log_range);
+    FwdArgs f;
+    const size_t fwd_bytes = forward_shape(A, nullptr, batch, n, dev.sm_count, &f);
+    Workspace *ws;
+    a.abort_flag = f.abort_flag = abort_dev;
+    a.blocks_per = 1;
+    if (tasks == 1) {                    // a warp a matrix, no slots
+        if ((st = workspace(&ws, 256 + fwd_bytes, 64)) != PG_OK) return st;
+        cudaStream_t s = stream ? stream : ws->stream;
+        a.status = f.status = (int *)ws->dev;
+        f.slots = fwd_bytes ? (double *)((char *)ws->dev + 256) : nullptr;
+        a.slots = nullptr;
+        a.grad = grad;
+        a.grad_abs = grad_abs;
+        PG_CUDA(cudaMemsetAsync(a.status, 0, sizeof(int), s));
+        if ((st = forward_launch(f, n, per, nullptr, abs_sum, s)) != PG_OK) return st;
+        PG_CUDA(launch_gradient_lo(n, a, s));
+        return f64_finish(a.status, s);
+    }
     // blocks per matrix: the fewest waves times ranges per warp; more blocks
     // also cost slots and their reduction, so ties go to fewer
-    const uint64_t tasks = tasks_of(a.log_range);
     uint64_t best = ~0ull;
-    a.blocks_per = 1;
     for (uint64_t p = 1; p <= resident && (p == 1 || (p - 1) * GRAD_WARPS < tasks); p++) {
         if (p > 1 && (uint64_t)batch * p > 8 * resident) break;
         const uint64_t waves = ((uint64_t)batch * p + resident - 1) / resident;
@@ -190,16 +211,12 @@ static int glynn_gradient_run(const double *A, int batch, int n, double *per, do
     }
     const size_t warps = (size_t)a.blocks_per * GRAD_WARPS;
     const size_t bytes = (size_t)batch * warps * grad_slot(n) * sizeof(double) + 256;
-    FwdArgs f;
-    const size_t fwd_bytes = forward_shape(A, nullptr, batch, n, dev.sm_count, &f);
-    Workspace *ws;
-    st = workspace(&ws, bytes + fwd_bytes, 64);
-    if (st != PG_OK) return st;
+    if ((st = workspace(&ws, bytes + fwd_bytes, 64)) != PG_OK) return st;
     cudaStream_t s = stream ? stream : ws->stream;
     a.status = f.status = (int *)ws->dev;
     a.slots = (double *)((char *)ws->dev + 256);
-    f.slots = (double *)((char *)ws->dev + bytes);
-    a.abort_flag = f.abort_flag = abort_dev;
+    a.grad = a.grad_abs = nullptr;
+    f.slots = fwd_bytes ? (double *)((char *)ws->dev + bytes) : nullptr;
     PG_CUDA(cudaMemsetAsync(ws->dev, 0, bytes, s));
     if ((st = forward_launch(f, n, per, nullptr, abs_sum, s)) != PG_OK) return st;
     PG_CUDA(n <= 16 ? launch_gradient_lo(n, a, s)

@@ -307,3 +307,62 @@ def test_walk_shapes_against_exact_values(lib, n):
         want = np.array([float(v) for v in lib.batch_exact(minors)]).reshape(n, n)
         err = np.abs(grad[b].cpu().numpy() - want)
         assert (err <= TOL * gs[b].cpu().numpy()[:, None]).all(), err.max()
+
+
+@pytest.mark.parametrize("n", [2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14])
+def test_many_small_matrices(lib, n):
+    # batches whose matrices are taken whole by one warp each (orders 10..14:
+    # only from some thousands on), against exact permanents and minors and
+    # against the same matrices in a batch of five; all copies alike
+    import torch
+    from permgpu.f64 import permanent_f64
+    rng = np.random.default_rng(1300 + n)
+    A = rng.integers(-3, 4, (5, n, n)).astype(np.int64)
+    A[1, n // 2] = 0
+    copies = 1000
+    few = permanent_f64(_t(A))
+    per, grad, s, gs = permanent_f64(_t(A).repeat(copies, 1, 1))
+    fwd, _, sf, _ = permanent_f64(_t(A).repeat(copies, 1, 1), want_grad=False)
+    assert torch.equal(fwd, per) and torch.equal(sf, s)
+    for x in (per, grad, s, gs):
+        x = x.reshape(copies, 5, *x.shape[1:])
+        assert (x == x[:1]).all()
+    exact = lib.batch_exact(list(A))
+    for b in range(5):
+        assert abs(per[b].item() - exact[b]) <= TOL * s[b].item()
+        assert abs(few[0][b].item() - exact[b]) <= TOL * s[b].item()
+        assert abs(s[b].item() - few[2][b].item()) <= 1e-5 * s[b].item()
+        assert ((gs[b] - few[3][b]).abs() <= 1e-5 * gs[b]).all()
+        minors = [np.delete(np.delete(A[b], i, 0), j, 1) for i in range(n) for j in range(n)]
+        want = _t([float(v) for v in lib.batch_exact(minors)]).reshape(n, n)
+        for g in (grad[b], few[1][b]):
+            assert ((g - want).abs() <= TOL * gs[b][:, None]).all()
+
+
+def _workspace_bytes(fn):
+    # device memory that the library keeps for a new host thread after fn(),
+    # whose own tensors come from torch's cache the second time
+    import threading
+    import torch
+    fn()
+    torch.cuda.synchronize()
+    grown = []
+
+    def run():
+        before = torch.cuda.mem_get_info()[0]
+        fn()
+        grown.append(before - torch.cuda.mem_get_info()[0])
+
+    t = threading.Thread(target=run)
+    t.start()
+    t.join()
+    return grown[0]
+
+
+def test_gradient_workspace_of_many_small_matrices(lib):
+    # no more than a slot of sums, their compensations and scales a matrix
+    import torch
+    from permgpu.f64 import permanent_f64
+    n, batch = 8, 1 << 19
+    a = torch.rand(batch, n, n, dtype=torch.float64, device="cuda")
+    assert _workspace_bytes(lambda: permanent_f64(a)) <= batch * 8 * (2 * n * n + n + 4)
