@@ -366,3 +366,23 @@ def test_gradient_workspace_of_many_small_matrices(lib):
     n, batch = 8, 1 << 19
     a = torch.rand(batch, n, n, dtype=torch.float64, device="cuda")
     assert _workspace_bytes(lambda: permanent_f64(a)) <= batch * 8 * (2 * n * n + n + 4)
+
+
+def test_gradient_in_parts(lib):
+    # slots of 2.2 GB if all matrices were taken at once: parts of 256 MB, the
+    # last one shorter, all copies alike and right
+    import torch
+    from permgpu.f64 import permanent_f64
+    n, batch = 16, (1 << 17) + 5
+    A = np.random.default_rng(1600).normal(0, 1 / np.sqrt(n), (n, n))
+    a = _t(A).expand(batch, n, n).contiguous()
+    assert _workspace_bytes(lambda: permanent_f64(a)) <= batch * 8 * (2 * n * n + n + 4)
+    per, grad, s, gs = permanent_f64(a)
+    for x in (per, grad, s, gs):
+        assert (x == x[:1]).all()
+    want, _ = oracle.glynn_f64(A, 8)
+    assert abs(per[0].item() - want) <= TOL * s[0].item()
+    _, one, _, scale = permanent_f64(a[:1])
+    assert ((grad[0] - one[0]).abs() <= TOL * scale[0][:, None]).all()
+    expansion = (a[0] * grad[0]).sum(1)
+    assert ((expansion - per[0]).abs() <= 1e-9 * (a[0].abs() * gs[0][:, None]).sum(1)).all()
