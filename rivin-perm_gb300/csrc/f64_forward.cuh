@@ -53,7 +53,20 @@ struct FwdArgs {
     double *re, *abs_sum;      // a matrix each, that write the results (abs_sum may be null)
     volatile const int *abort_flag;
     int *status;
+    int resident;              // blocks of the first wave, at most
 };
+
+// Blocks beyond the first wave ask before they start (a batch of small
+// matrices is one range a warp, which polls only between ranges): every 64th
+// reads the host-mapped word and passes it on through the status.
+template <class Args>
+__device__ __forceinline__ bool f64_stopped(const Args &a) {
+    if ((int)blockIdx.x < a.resident) return false;
+    if (*(volatile const int *)a.status) return true;
+    if ((blockIdx.x & 63) || !*a.abort_flag) return false;
+    atomicExch(a.status, 1);
+    return true;
+}
 
 constexpr int FWD_WARPS = 4;       // warps of a thread block
 constexpr int FWD_SLOT = 3;        // re, im, sum |term|
@@ -147,6 +160,8 @@ __global__ void __launch_bounds__(32 * WARPS) glynn_forward_kernel(FwdArgs a) {
     // columns 0..N-2 hold 2 a'_ij, column N-1 the all-plus row sums
     float *tab = reinterpret_cast<float *>(fwd_smem);
     __shared__ int row_exp[N];
+    __shared__ bool stop;
+    if (threadIdx.x == 0) stop = f64_stopped(a);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int b = blockIdx.x / a.blocks_per, part = blockIdx.x - b * a.blocks_per;
     const double *Ar = a.Are + (size_t)b * N * N;
@@ -154,6 +169,7 @@ __global__ void __launch_bounds__(32 * WARPS) glynn_forward_kernel(FwdArgs a) {
     for (int r = threadIdx.x; r < N; r += BT)
         row_exp[r] = fwd_row_exponent(Ar + r * N, CPLX ? Ai + r * N : nullptr, N, BL);
     __syncthreads();
+    if (stop) return;
     for (int idx = threadIdx.x; idx < N * NP; idx += BT) {
         const int j = idx / NP, r = idx - j * NP;
         float *t = tab + j * COL + r;

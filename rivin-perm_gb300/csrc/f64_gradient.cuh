@@ -51,6 +51,7 @@ struct GradArgs {
     double *grad, *grad_abs;   // results of the one-warp blocks (grad_abs may be null)
     volatile const int *abort_flag;
     int *status;
+    int resident;              // blocks of the first wave, at most
 };
 
 constexpr int GRAD_WARPS = 4;  // warps of a thread block
@@ -158,6 +159,8 @@ __global__ void __launch_bounds__(32 * WARPS, 8 / WARPS) glynn_gradient_kernel(G
     extern __shared__ float4 grad_smem[];
     float *tab = reinterpret_cast<float *>(grad_smem);   // [N][P][3][RP]; column N-1: all-plus sums
     __shared__ int row_exp[N];
+    __shared__ bool stop;
+    if (threadIdx.x == 0) stop = f64_stopped(a);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int p = lane & (P - 1), w = lane >> S::LP;
     // this thread's column of the slots: slot t, row r at [(t RW + r) BT]
@@ -168,6 +171,7 @@ __global__ void __launch_bounds__(32 * WARPS, 8 / WARPS) glynn_gradient_kernel(G
     const double *A = a.A + (size_t)b * N * N;
     for (int r = threadIdx.x; r < N; r += BT) row_exp[r] = fwd_row_exponent(A + r * N, nullptr, N, BL);
     __syncthreads();
+    if (stop) return;
     for (int idx = threadIdx.x; idx < N * P * RP; idx += BT) {
         const int j = idx / (P * RP), q = idx - j * (P * RP), lp = q / RP, r = q - lp * RP;
         float *t = tab + j * COL + lp * 3 * RP + r;

@@ -45,6 +45,8 @@ __global__ void glynn_forward_reduce(const double *Are, const double *Aim, const
     if (abs_sum) abs_sum[b] = ldexp(as, -e - (n - 1));
 }
 
+constexpr int F64_BLOCKS_SM = 32;    // resident blocks of an SM, at most
+
 // Launch shape of the forward walk of `batch` matrices of order 2..32 (Aim
 // null: real): fills a.batch, a.log_block, a.blocks_per; returns the slots'
 // bytes, 0 where a warp takes a whole real matrix and writes its result.
@@ -54,6 +56,7 @@ static size_t forward_shape(const double *Are, const double *Aim, int batch, int
     a.Are = Are;
     a.Aim = Aim;
     a.batch = batch;
+    a.resident = F64_BLOCKS_SM * sms;
     a.log_block = std::min(FWD_LOG_BLOCK, n - 1);
     // shorter real blocks (down to 8 states a thread) while fewer than four
     // waves of warps are busy; complex ones keep the length that fixes the
@@ -170,6 +173,7 @@ static int glynn_gradient_run(const double *A, int batch, int n, double *per, do
     GradArgs a;
     a.A = A;
     a.batch = batch;
+    a.resident = F64_BLOCKS_SM * dev.sm_count;
     int lw, rmax;
     gradient_shape(n, &lw, &rmax);
     // shorter ranges (down to 2^5 states) while a warp per range leaves less

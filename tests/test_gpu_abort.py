@@ -130,3 +130,17 @@ def test_abort_fp64_walks(lib, kind, n, batch):
     status, took = _aborted_after(lib, lambda: _fp64(kind, n, batch))
     assert status == lib.PG_EABORT
     assert took < 1.5
+
+
+@pytest.mark.parametrize("kind,n,batch", [
+    ("forward", 4, 200_000), ("forward", 12, 20_000), ("forward", 13, 200_000),
+    ("complex", 5, 200_000), ("complex", 12, 50_000),
+    ("gradient", 4, 200_000), ("gradient", 10, 50_000), ("gradient", 15, 10_000),
+])
+def test_abort_word_raised_before_batches_of_small_matrices(lib, kind, n, batch):
+    # a warp walks one range only: blocks beyond the first wave ask before
+    # they start
+    want = [x.cpu() for x in _fp64(kind, n, 4) if x is not None]
+    assert _raised_before(lib, lambda: _fp64(kind, n, batch)) == lib.PG_EABORT
+    got = [x.cpu() for x in _fp64(kind, n, 4) if x is not None]
+    assert all((x == y).all() for x, y in zip(want, got))
