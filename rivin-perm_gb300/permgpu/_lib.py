@@ -440,11 +440,11 @@ def batch_row_sums(packed: np.ndarray, orders: np.ndarray):
     return sums, np.concatenate(([0], np.cumsum(rows)[:-1]))
 
 
-def batch_limbs(matrices, packed=None) -> int:
-    """Output words that hold any matrix's permanent; ``packed``: the
-    matrices' pack_batch, if at hand."""
+def batch_limbs(matrices, packed=None, rows=None) -> int:
+    """Output words that hold any matrix's permanent; ``packed`` and ``rows``:
+    the matrices' pack_batch and batch_row_sums, if at hand."""
     packed, _, orders = packed or pack_batch(matrices)
-    sums, first = batch_row_sums(packed, orders)
+    sums, first = rows or batch_row_sums(packed, orders)
     if not first.size:
         return 2
     bits = np.add.reduceat(np.log2(np.maximum(1.0, sums)), first)
@@ -456,10 +456,10 @@ class BatchPlan:
     persistent work-stealing launch per evaluation, replayed from a CUDA
     graph."""
 
-    def __init__(self, matrices, tune: tuple | None = None):
+    def __init__(self, matrices, tune: tuple | None = None, packed=None, rows=None):
         self.count = len(matrices)
-        packed, offsets, orders = pack_batch(matrices)
-        self.limbs = batch_limbs(matrices, (packed, offsets, orders))
+        packed, offsets, orders = packed or pack_batch(matrices)
+        self.limbs = batch_limbs(matrices, (packed, offsets, orders), rows)
         self.orders = orders
         t = BatchTune(*(tune or (0, 0, 0)))
         h = ctypes.c_void_p()

@@ -39,20 +39,24 @@ def batch_permanents(matrices: Sequence, tune="auto", cache_path=None) -> List[i
     """
     mats = [np.asarray(m, dtype=np.int64).reshape(len(m), len(m)) if len(m) else
             np.zeros((0, 0), np.int64) for m in matrices]
-    packed, _, orders = _lib.pack_batch(mats)
-    sums, first = _lib.batch_row_sums(packed, orders)
+    packed = _lib.pack_batch(mats)
+    orders = packed[2]
+    rows = sums, first = _lib.batch_row_sums(packed[0], orders)
     top = np.zeros(len(mats))
     if first.size:
         top[orders > 0] = np.maximum.reduceat(sums, first)
-    ok = [i for i, m in enumerate(mats)
-          if _lib.row_bounds_fit(top[i], int(orders[i])) or _exact_ok(m)]
+    ok = [i for i, (t, n) in enumerate(zip(top.tolist(), orders.tolist()))
+          if _lib.row_bounds_fit(t, n) or _exact_ok(mats[i])]
     out: List[int] = [0] * len(mats)
     if ok:
-        sub = [mats[i] for i in ok]
+        # packed and summed once, unless some matrices go another way
+        sub, given = mats, (packed, rows)
+        if len(ok) < len(mats):
+            sub, given = [mats[i] for i in ok], ()
         if tune == "auto":
             from .autotune import tuned_parameters
             tune = tuned_parameters(sub, cache_path=cache_path)
-        plan = _lib.BatchPlan(sub, tune)
+        plan = _lib.BatchPlan(sub, tune, *given)
         try:
             plan.launch()
             for i, v in zip(ok, plan.results()):

@@ -258,3 +258,28 @@ def test_pack_batch_layout():
     packed, offsets, orders = _lib.pack_batch(mats)
     assert orders.tolist() == [2, 0, 1, 3] and offsets.tolist() == [0, 4, 4, 5]
     assert packed.tolist() == [0, 1, 2, 3, 7, 0, 3, 6, 1, 4, 7, 2, 5, 8]
+
+
+def test_batch_permanents_packs_and_sums_once(monkeypatch):
+    # the plan takes the packed words and row sums of the route decision
+    from unittest import mock
+    from permgpu import _lib, batch
+    native = mock.MagicMock()
+    for name in _lib.SIGNATURES:
+        getattr(native, name).return_value = 0
+    monkeypatch.setattr(_lib, "load", lambda: native)
+    pack = mock.MagicMock(side_effect=_lib.pack_batch)
+    sums = mock.MagicMock(side_effect=_lib.batch_row_sums)
+    monkeypatch.setattr(_lib, "pack_batch", pack)
+    monkeypatch.setattr(_lib, "batch_row_sums", sums)
+    mats = [np.full((n, n), n) for n in (2, 5, 0, 1, 7)]
+    assert batch.batch_permanents(mats, tune=None) == [0] * 5
+    assert pack.call_count == 1 and sums.call_count == 1
+    args = native.pg_batch_plan_create.call_args[0]
+    assert [args[0][i] for i in range(4)] == [2] * 4 and args[3] == 5
+    # one matrix beyond the batch's range: the others are packed for the plan
+    pack.reset_mock()
+    monkeypatch.setattr(batch, "matrix_permanent", lambda m: 99)
+    mats[1] = np.full((5, 5), 1 << 45)
+    assert batch.batch_permanents(mats, tune=None) == [0, 99, 0, 0, 0]
+    assert native.pg_batch_plan_create.call_args[0][3] == 4
