@@ -236,8 +236,22 @@ static int glynn_m32_batch(const uint64_t *mats, int n, const uint64_t *moduli,
     while ((2ull << log_T) <= bpm * 256) log_T++;
     ChunkPlan pl;
     pl.log_len = log_states - (log_T + 7);
-    // chunks of 16 states where 64 would leave a thread less than eight
-    const int floor_len = (span >> 9) < bpm * 256 ? 4 : 6;
+    // Chunks of 64 states at least; where they leave a thread less than eight,
+    // of 64, 32 and 16 states the length with the least work for the busiest
+    // thread, a chunk's first step taken as three states (the lanes toggle
+    // different columns there): one modulus at order 14 65 us of 64, 48 of 16;
+    // 16 80 and 84; 17 79 and 86
+    int floor_len = 6;
+    if ((span >> 9) < bpm * 256) {
+        uint64_t least = ~0ull;
+        for (int len = 6; len >= 4; len--) {
+            const uint64_t work = ((span >> len) + bpm * 256 - 1) / (bpm * 256) * ((1ull << len) + 3);
+            if (work < least && (span >> len) > 0) {
+                least = work;
+                floor_len = len;
+            }
+        }
+    }
     const int min_len = log_states < floor_len ? log_states : floor_len;
     if (pl.log_len < min_len) pl.log_len = min_len;
     if (pl.log_len > 30) pl.log_len = 30;

@@ -225,3 +225,15 @@ def test_gpu_ext_drop_in(lib):
     m = [[rng.randrange(-101, 101) for _ in range(17)] for _ in range(17)]
     assert ext.permanent_mod_p(m, 101) == oracle.permanent_mod_p(m, 101, 8)
     assert BinaryGpuExt().binary_permanent_mod_p([[1, 1], [1, 1]], 101) == 2
+
+
+@pytest.mark.parametrize("n", [8, 13, 14, 15, 16, 17, 18, 19, 20, 21, 22, 23])
+def test_chunk_lengths_of_short_walks(lib, n):
+    # 1, 5 and 34 moduli share the blocks differently: chunks of 16, 32 and 64
+    # states, and more threads than chunks
+    from permgpu.crt import descending_primes
+    a = np.random.default_rng(2300 + n).integers(-9, 10, (n, n), dtype=np.int64)
+    want = lib.exact_permanent(a, lib.exact_limbs(a))
+    primes = descending_primes(1 << (31 * 34))[:34]
+    for k in (1, 5, 34):
+        assert lib.residues(a, primes[:k]) == [want % p for p in primes[:k]]
