@@ -455,9 +455,10 @@ cudaError_t launch_binary_any(int NPAD, int G, const BinaryArgs &args, int block
 
 // Packs even-degree rows with caps[e] + 1 table entries each into few enough
 // table groups (a multiple of four where that takes no more lookups) for the
-// tables to fit beside the NPAD kernel's other shared memory, with the most
-// warps that allow it; group[e] = the row's group.  Returns the number of
+// tables to fit beside the NPAD kernel's other shared memory, and for a walk
+// of `chunks` chunks a block not to spend its time on their entries, with the
+// most warps that allow it; group[e] = the row's group.  Returns the number of
 // groups, -1 if there is no such packing.
-int binary_pack_groups(int NPAD, const int *caps, int rows, int *group, int *warps);
+int binary_pack_groups(int NPAD, const int *caps, int rows, double chunks, int *group, int *warps);
 
 }  // namespace pg

@@ -217,7 +217,11 @@ struct ExactPlan {
 
 // Sixteen warps keep the kernel within 2 % of its best (12..24 measured).
 constexpr int BIN_WARPS_MIN = 16;
-int binary_pack_groups(int NPAD, const int *caps, int rows, int *group, int *warps) {
+// SM clocks of a table entry, and of one more lookup for a chunk.  Fitted to
+// launches and windows of orders 24..36: 4 or 14 clocks a lookup cost up to 9 %
+// at single sizes, 1.5 up to 8 % on windows of 2^26 states.
+constexpr double BIN_ENTRY_CLOCKS = 55, BIN_LOOKUP_CLOCKS = 8;
+int binary_pack_groups(int NPAD, const int *caps, int rows, double chunks, int *group, int *warps) {
     std::vector<int> by(rows);
     for (int e = 0; e < rows; e++) by[e] = e;
     std::stable_sort(by.begin(), by.end(), [&](int x, int y) { return caps[x] > caps[y]; });
@@ -233,17 +237,26 @@ int binary_pack_groups(int NPAD, const int *caps, int rows, int *group, int *war
         for (double v : size) total += v;
         return total < 65536 ? (size_t)total : 65536;
     };
-    // the fewest lookups (a multiple of four) with at least BIN_WARPS_MIN
-    // warps, then the most warps for them; fewer warps only where nothing fits
+    // Lookups (a multiple of four) against table entries: the least time of
+    // both with at least BIN_WARPS_MIN warps, then the most warps for it; fewer
+    // warps only where nothing fits.  Long walks take the fewest lookups that
+    // fit, shorter ones small tables: a launch of 24 x 24 Bernoulli(1/2) 52 us
+    // with four lookups and some 1000 entries, 35 with twelve and 80; a window
+    // of 4096 states 88 and 70.
     const int most = binary_max_threads(NPAD) / 32;
     int best = 0;
+    double least = 0;
     *warps = most;
     if (rows == 0) return 0;
-    for (int w = most; w >= 2 && (w >= BIN_WARPS_MIN || !best); w -= 2)
-        for (int T = 4; T < rows + 4 && (!best || T < best); T += 4) {
-            const int groups = T < rows ? T : rows;
-            if (binary_smem(NPAD, (int)pack(groups), T, w) > BIN_SMEM) continue;
+    for (int floor = BIN_WARPS_MIN; floor > 0 && !best; floor -= 2)
+        for (int T = 4; T < rows + 4; T += 4) {
+            const size_t entries = pack(T < rows ? T : rows);
+            int w = most;
+            while (w >= floor && binary_smem(NPAD, (int)entries, T, w) > BIN_SMEM) w -= 2;
+            const double time = entries * BIN_ENTRY_CLOCKS + chunks * T * BIN_LOOKUP_CLOCKS;
+            if (w < floor || (best && time >= least)) continue;
             best = T;
+            least = time;
             *warps = w;
         }
     if (!best) return -1;
@@ -268,6 +281,7 @@ struct BinaryRows {
     int maxh = 0, survive = 0;           // largest half degree, survivors of 1024 samples
 };
 constexpr int BINARY_SAMPLES = 1024;
+constexpr int BIN_BLOCKS = 152;      // blocks of a launch, one an SM
 static void binary_rows(const int64_t *A, int n, bool transposed, BinaryRows *B) {
     const int NPAD = binary_npad(n);
     B->deg.assign(NPAD, 1);
@@ -343,7 +357,7 @@ static void binary_order_columns(int n, int low, BinaryRows *B) {
     }
 }
 
-static bool plan_build_binary(const int64_t *A, int n, bool whole, ExactPlan *P) {
+static bool plan_build_binary(const int64_t *A, int n, bool whole, uint64_t states, ExactPlan *P) {
     if (!EXACT_BINARY || n < BINARY_MIN_N || n > 48) return false;
     for (size_t i = 0; i < (size_t)n * n; i++)
         if (A[i] != 0 && A[i] != 1) return false;
@@ -378,7 +392,8 @@ static bool plan_build_binary(const int64_t *A, int n, bool whole, ExactPlan *P)
     const int nt = (int)table.size();
     std::vector<int> caps(nt), group(nt);
     for (int e = 0; e < nt; e++) caps[e] = __builtin_popcountll(rows[table[e]] & low_mask) + 1;
-    const int groups = binary_pack_groups(NPAD, caps.data(), nt, group.data(), &P->warps);
+    const double chunks = (double)(states >> BIN_LOW) / BIN_BLOCKS;
+    const int groups = binary_pack_groups(NPAD, caps.data(), nt, chunks, group.data(), &P->warps);
     if (groups < 0) return false;
     P->planes = K;
     P->npad = NPAD;
@@ -503,8 +518,9 @@ static void add_block_slots(ExactPlan *P) {
     P->image.resize(P->total, 0);
 }
 
-static int plan_build(const int64_t *A, int n, ExactPlan *P, bool whole = true) {
-    if (plan_build_binary(A, n, whole, P)) {
+// states: those of the walk (a window's, where not the whole one's)
+static int plan_build(const int64_t *A, int n, ExactPlan *P, bool whole = true, uint64_t states = 0) {
+    if (plan_build_binary(A, n, whole, whole ? 1ull << (n - 1) : states, P)) {
         DeviceInfo dev;
         int st = device_info(&dev);
         if (st != PG_OK) return st;
@@ -756,7 +772,7 @@ int pg_exact_partial(const int64_t *A, int n, uint64_t state_lo, uint64_t state_
     using namespace pg;
     if (!A || !words || !nwords || n < 2 || n >= 64) return fail(PG_EINVAL, "bad arguments");
     ExactPlan P;
-    int st = plan_build(A, n, &P, false);
+    int st = plan_build(A, n, &P, false, state_hi > state_lo ? state_hi - state_lo : 0);
     if (st != PG_OK) return st;
     if ((st = plan_restrict(&P, state_lo, state_hi)) != PG_OK) return st;
     if (max_words < P.NL) return fail(PG_ERANGE, "words buffer too small");

@@ -172,3 +172,20 @@ def test_rows_outside_the_low_columns(lib, n, degree):
         w = shard.words_value(shard.exact_partial_words(b, lo, hi))
         assert 2 * v == w, (lo, hi)
     assert _exact(lib, a) == _via_general_kernel(lib, a)
+
+
+@pytest.mark.parametrize("n", [24, 25, 28, 31, 33])
+def test_table_packings_of_short_and_long_walks(lib, n):
+    # a window's length decides how the even rows share tables: a row each,
+    # eight or twelve groups, or the fewest that fit
+    from permgpu import shard
+    a = (np.random.default_rng(2400 + n).random((n, n)) < 0.5).astype(np.int64)
+    assert _planes(lib, a) >= 2
+    b = a.copy()
+    b[0] *= 2
+    top = 1 << (n - 1)
+    for lo, hi in ((4, 4096), (1 << 20, 1 << 22), (1 << 20, min(top, 1 << 25)), (0, min(top, 1 << 29))):
+        v = shard.words_value(shard.exact_partial_words(a, lo, hi))
+        w = shard.words_value(shard.exact_partial_words(b, lo, hi))
+        assert 2 * v == w, (lo, hi)
+    assert _exact(lib, a) == _via_general_kernel(lib, a)
