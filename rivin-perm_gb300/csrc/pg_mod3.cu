@@ -16,8 +16,8 @@
 // lane l is the state with low signs (k | l << 5 | h << 10).  The high
 // columns are common to the warp, so row i's sum is h_i + low_i(lane, h, bit),
 // and "row i is nonzero" is a pair of words that depends only on the lane and
-// on h_i in {0, 1, 2}.  For the first six groups of four rows (five up to
-// order 20 and above 52) the 81 AND-ed pairs per lane sit in shared memory
+// on h_i in {0, 1, 2}.  For the first six groups of four rows (five above
+// order 52) the 81 AND-ed pairs per lane sit in shared memory
 // ([81][32] pairs, lane-minor: no bank conflicts): one high state (2048 sign
 // vectors) is six 8-byte loads and ANDs for the first 24 rows.  (2/3)^24 of
 // the states, in one of eight high states, go on row by row, and only states
@@ -39,7 +39,7 @@
 
 namespace pg {
 
-constexpr int MOD3_THREADS = 1024;   // one block per SM: the tables take up to 212 KB
+constexpr int MOD3_THREADS = 1024;   // one block per SM: the tables take up to 224 KB
 constexpr int MOD3_LOW = 11;         // columns over word bits (5), lanes (5) and words (1)
 constexpr int MOD3_DIGITS = 81;      // states of a group of four rows' high sums
 
@@ -54,8 +54,9 @@ struct Mod3Args {
     volatile const int *abort_flag;
 };
 
-// row groups with tables: six (24 rows) where rows and memory allow, else five
-__host__ __device__ constexpr int mod3_tables(int n) { return n > 20 && n <= 52 ? 6 : 5; }
+// row groups with tables, from order 25 on (MOD3_SHORT): six (24 rows) where
+// memory allows, else five
+__host__ __device__ constexpr int mod3_tables(int n) { return n <= 52 ? 6 : 5; }
 // per-row words [n][3][32] pairs; the lists hold six offsets a high state
 __host__ __device__ constexpr size_t mod3_row_bytes(int n) { return (size_t)n * 3 * 32 * 8; }
 // Few high states (up to 2^12, order 24): no tables, a high state a warp, every
@@ -314,8 +315,7 @@ static int mod3_impl(const uint64_t *mags, const uint64_t *sgns, int n, int *out
     a.abort_flag = abort_dev;
     const bool six = mod3_tables(n) == 6;
     if (!tables) PG_CUDA((launch_mod3<uint32_t, 0>(a, blocks, ws->stream)));
-    else if (n <= 32 && six) PG_CUDA((launch_mod3<uint32_t, 6>(a, blocks, ws->stream)));
-    else if (n <= 32) PG_CUDA((launch_mod3<uint32_t, 5>(a, blocks, ws->stream)));
+    else if (n <= 32) PG_CUDA((launch_mod3<uint32_t, 6>(a, blocks, ws->stream)));
     else if (six) PG_CUDA((launch_mod3<uint64_t, 6>(a, blocks, ws->stream)));
     else PG_CUDA((launch_mod3<uint64_t, 5>(a, blocks, ws->stream)));
     PG_CUDA(cudaStreamSynchronize(ws->stream));

@@ -67,3 +67,17 @@ def test_expansion_beyond_one_word(lib):
         want = lib.permanent_mod3(a[:k, :k]) * lib.permanent_mod3(a[k:, k:]) % 3
         p, q = rng.permutation(n), rng.permutation(n)
         assert lib.permanent_mod3(a[p][:, q]) == want
+
+
+@pytest.mark.parametrize("n", [25, 26, 28, 29, 31, 32, 33, 34])
+def test_many_survivors_with_tables(lib, n):
+    # orders that take tables, rows of one word and of two, the last batch and
+    # row group; rows that differ in few places, so that many states keep every
+    # row nonzero; against the exact engine
+    rng = np.random.default_rng(2500 + n)
+    row = rng.integers(1, 3, n)
+    a = np.where(rng.random((n, n)) < 0.12, rng.integers(0, 3, (n, n)), row)
+    a *= rng.integers(1, 3, (n, 1))
+    want = lib.exact_permanent(a, lib.exact_limbs(a)) % 3
+    assert lib.permanent_mod3(a) == want
+    assert lib.permanent_mod3(a.T.copy()) == want
