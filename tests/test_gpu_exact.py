@@ -222,3 +222,22 @@ def test_windows_match_other_group_sizes(lib, n, mag):
         v = shard.words_value(shard.exact_partial_words(a, lo, hi))
         w = shard.words_value(shard.exact_partial_words(b, lo, hi))
         assert f * v == w, (lo, hi)
+
+
+@pytest.mark.parametrize("n", [2, 11] + list(range(13, 33)))
+def test_wide_engine_every_shape(lib, n):
+    # every compiled order in every row class: a small-entry matrix with its
+    # rows multiplied up to the class bound, against the 32-bit engine's value
+    # (per is multilinear in the rows); signed entries, and positive ones,
+    # whose first state has every row at its bound
+    rng = np.random.default_rng(4700 + n)
+    for signed in (True, False):
+        a = rng.integers(-8 if signed else 1, 9, (n, n))
+        value = lib.exact_permanent(a, lib.exact_limbs(a))
+        for bits in (36, 40, 44, 48):
+            f = ((1 << bits) - 1) // np.maximum(1, np.abs(a).sum(1))
+            want = value
+            for v in f:
+                want *= int(v)
+            w = a * f[:, None]
+            assert lib.exact_wide_permanent(w, lib.exact_limbs(w)) == want, (signed, bits)

@@ -202,3 +202,17 @@ def test_exact_symmetric_sums_against_exact_permanents(lib, n, top):
         a = 3 + x * L
         want = lib.exact_permanent(a, lib.exact_limbs(a)) % m
         assert sum(c * pow(x, d, m) for d, c in enumerate(coef)) % m == want
+
+
+@pytest.mark.parametrize("top", [15, 20, 31])
+@pytest.mark.parametrize("n", [18, 19, 20, 21, 22, 23, 24])
+def test_exact_symmetric_sums_at_padded_orders(lib, n, top):
+    # orders at and below each compiled one, every row-sum class
+    rng = np.random.default_rng(31 * n + top)
+    L = _small_rows(rng, n, top)
+    m = (1 << 30) - 35
+    coef = lib.affine_residues(np.full((n, n), -2, dtype=np.int64), L, [m])[0]
+    for x in (1, -1, 3):
+        a = -2 + x * L
+        want = lib.exact_permanent(a, lib.exact_limbs(a)) % m
+        assert sum(c * pow(x, d, m) for d, c in enumerate(coef)) % m == want
