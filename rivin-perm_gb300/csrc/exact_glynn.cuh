@@ -158,10 +158,13 @@ __device__ __forceinline__ void exact_term_col(const int32_t *s, uint64_t *col, 
 // and the walk hides the table offset from the compiler instead: groups of
 // 2 at order 32 37.4 -> 35.4 ms, of 3 21.2 -> 19.4, of 4 at order 33 33.8 ->
 // 30.9.  Where nothing spills the registers are the better place (groups of
-// 5 at order 32: 11.0 ms, 11.8 without); of the larger shapes only nine full
-// groups of 4 are near that (7 words: 243 ms, 252 without).
+// 5 at order 32: 11.0 ms, 11.8 without).  Of the larger shapes only nine full
+// groups of an even size are near that (3 and 7 words more): 36 x 36 in fours
+// 243 ms, 252 without, 18 x 18 in pairs 20.5 us either way.
 __host__ __device__ constexpr bool exact_hoist(int N, int G, int FR) {
-    return ((N + G - 1) / G <= 8 && (FR == 0 || N % G == 0)) || (N == 36 && G == 4 && FR == 0);
+    const int groups = (N + G - 1) / G;
+    return groups <= 8 ? FR == 0 || N % G == 0
+                       : groups == 9 && N % G == 0 && G % 2 == 0 && FR == 0;
 }
 
 // Walk chunks [c_begin, c_end) (row sums s already at state c_begin*2^log_len)

@@ -241,3 +241,11 @@ def test_wide_engine_every_shape(lib, n):
                 want *= int(v)
             w = a * f[:, None]
             assert lib.exact_wide_permanent(w, lib.exact_limbs(w)) == want, (signed, bits)
+
+
+@pytest.mark.parametrize("n,mag", [(17, 1000), (18, 1000), (20, 1000), (18, 8)])
+def test_groups_of_two_at_nine_groups(lib, n, mag):
+    import permgpu
+    a = np.random.default_rng(n * mag).integers(-mag, mag + 1, (n, n), dtype=np.int64)
+    want = permgpu.matrix_permanent(a.tolist(), engine="residue")
+    assert permgpu.matrix_permanent(a.tolist(), engine="exact") == want
