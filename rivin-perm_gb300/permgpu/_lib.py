@@ -442,8 +442,12 @@ def batch_row_sums(packed: np.ndarray, orders: np.ndarray):
 
 def batch_limbs(matrices, packed=None, rows=None) -> int:
     """Output words that hold any matrix's permanent; ``packed`` and ``rows``:
-    the matrices' pack_batch and batch_row_sums, if at hand."""
-    packed, _, orders = packed or pack_batch(matrices)
+    the matrices' pack_batch and batch_row_sums, if at hand (entries beyond
+    int64, which cannot be packed, are summed matrix by matrix)."""
+    if packed is None:
+        mats = map(np.asarray, matrices)
+        return max([exact_limbs(m) for m in mats if m.size] or [2])
+    packed, _, orders = packed
     sums, first = rows or batch_row_sums(packed, orders)
     if not first.size:
         return 2

@@ -247,7 +247,7 @@ def test_pack_batch_refuses_matrices_that_are_not_square(shape, at):
     from permgpu import _lib
     mats = [np.arange(4).reshape(2, 2), np.ones((5, 5), dtype=np.int64)]
     mats.insert(at, np.ones(shape, dtype=np.int64))
-    for call in (_lib.pack_batch, _lib.batch_limbs, _lib.batch_exact, _lib.BatchPlan):
+    for call in (_lib.pack_batch, _lib.batch_exact, _lib.BatchPlan):
         with pytest.raises(ValueError):
             call(mats)
 
@@ -283,3 +283,13 @@ def test_batch_permanents_packs_and_sums_once(monkeypatch):
     mats[1] = np.full((5, 5), 1 << 45)
     assert batch.batch_permanents(mats, tune=None) == [0, 99, 0, 0, 0]
     assert native.pg_batch_plan_create.call_args[0][3] == 4
+
+
+def test_batch_limbs_of_entries_beyond_int64():
+    from permgpu import _lib
+    assert _lib.batch_limbs([[[2 ** 64, 1], [1, 3]], [[1, 2], [3, 4]]]) == 4
+    assert _lib.batch_limbs([np.array([[2 ** 70, 1], [1, 2 ** 70]], dtype=object)]) == 6
+    assert _lib.batch_limbs([]) == 2
+    mats = [np.arange(9).reshape(3, 3), np.zeros((0, 0)), np.full((20, 20), 99)]
+    assert _lib.batch_limbs(mats) == _lib.batch_limbs(mats, _lib.pack_batch(mats)) \
+        == max(_lib.exact_limbs(m) for m in mats)
