@@ -144,3 +144,40 @@ def test_abort_word_raised_before_batches_of_small_matrices(lib, kind, n, batch)
     assert _raised_before(lib, lambda: _fp64(kind, n, batch)) == lib.PG_EABORT
     got = [x.cpu() for x in _fp64(kind, n, 4) if x is not None]
     assert all((x == y).all() for x, y in zip(want, got))
+
+
+@pytest.mark.parametrize("kind", ["general40", "binary44", "mod3_48"])
+def test_abort_integer_walks_of_seconds(lib, kind):
+    # three to five seconds uninterrupted
+    rng = np.random.default_rng(44)
+    a = {"general40": lambda: rng.integers(-8, 9, (40, 40)),
+         "binary44": lambda: (rng.random((44, 44)) < 0.5).astype(np.int64),
+         "mod3_48": lambda: rng.integers(0, 3, (48, 48))}[kind]()
+    call = lib.permanent_mod3 if kind == "mod3_48" else lambda m: lib.exact_permanent(m, lib.exact_limbs(m))
+    if kind == "binary44":
+        plan = lib.ExactPlan(a)
+        assert lib.load().pg_exact_plan_bit_planes(plan._h) >= 2
+        plan.close()
+    lib.load().pg_clear_abort()
+    status, took = _aborted_after(lib, lambda: call(a))
+    assert status == lib.PG_EABORT
+    assert took < 1.0
+    b = a[:18, :18].copy()
+    want = oracle.exact_permanent(b.tolist())
+    assert call(b) == (want % 3 if kind == "mod3_48" else want)
+
+
+def test_abort_word_raised_before_wide_and_polynomial_walks(lib):
+    # the 64-bit exact kernel asks in blocks beyond the first wave, the exact
+    # polynomial kernel from a block's second task on
+    rng = np.random.default_rng(45)
+    a = rng.integers(-(1 << 42), 1 << 42, (28, 28))
+    assert _raised_before(lib, lambda: lib.exact_wide_permanent(a, lib.exact_limbs(a))) == lib.PG_EABORT
+    L = (rng.random((28, 28)) < 0.5).astype(np.int64)
+    ones = np.ones((28, 28), dtype=np.int64)
+    assert _raised_before(lib, lambda: lib.affine_residues(ones, L, [1_000_003])) == lib.PG_EABORT
+    b = a[:14, :14].copy()
+    assert lib.exact_wide_permanent(b, 40) == oracle.exact_permanent(b.tolist())
+    m = L[:14, :14].copy()
+    assert lib.affine_residues(ones[:14, :14], m, [1_000_003])[0] == \
+        oracle.affine_mod_p(ones[:14, :14], m, 1_000_003)
