@@ -708,7 +708,7 @@ def run_gpu_float28(args, world, rank, local):
             gw = Fraction(permgpu.matrix_permanent(minor), 1 << (sum(ks) - ks[i]))
             exact_grad.append(abs(Fraction(float(g[b, i, j])) - gw) /
                               Fraction(gs[b, i].item()))
-    # forward-only arm (the same traversal without the gradient columns)
+    # forward-only arm (the forward walk, which a call with the gradient runs too)
     for _ in range(2):
         permanent_f64(A, want_grad=False)
     torch.cuda.synchronize()

@@ -46,9 +46,11 @@ const char *pg_last_error(void);
 int pg_device_info(int *sm_count, int *cc_major, int *cc_minor);
 
 /* Ask running launches to stop at their next poll; they return PG_EABORT.
- * A kernel thread reads the abort word once per 2^16 states (per chunk
- * for longer chunks) from its second period on, so launches whose threads
- * walk fewer states complete.  pg_clear_abort() re-arms the library. */
+ * A kernel thread reads the abort word once per 2^16 states (per chunk,
+ * range, batch or task where the kernel works by those) from its second
+ * period on, and blocks beyond a launch's first wave of FP64 matrices or
+ * 64-bit exact ranges before they start, so launches whose threads walk
+ * fewer states in one wave complete.  pg_clear_abort() re-arms the library. */
 void pg_abort(void);
 void pg_clear_abort(void);
 

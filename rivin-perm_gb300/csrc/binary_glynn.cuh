@@ -29,8 +29,8 @@
 // batches at once, one a lane; then the chunk rows, by bytes.  A whole walk
 // orders its columns so that such rows exist (binary_order_columns).  4x4x5
 // grid with a few bonds removed and columns shuffled: 34.9 ms without these
-// tests, 25.7 with them (one batch at a time), 6.2 with ordered columns; 2-3
-// with the batches of a unit tested together and taken from all over the
+// tests, 25.7 with them (one batch at a time), 6.2 with ordered columns; 2.6-4.3
+// by which bonds are removed with the batches of a unit tested together and taken from all over the
 // walk (neighbours are zero together, and warps ran dry).
 //
 // Evaluation.  Surviving states are appended to a per-warp queue; whenever
@@ -48,8 +48,8 @@
 //
 // Issue bound (65-80 % of the issue slots).  Whole calls against a
 // bit-sliced tracker that updated one state per lane and step and evaluated
-// by popcount: 4x4x5 grid (40 x 40, 0.08 % survive) 441 -> 3.0 ms, 36 x 36
-// Bernoulli(1/2) (6-13 % survive) 67-76 -> 18-22 ms.
+// by popcount: 4x4x5 grid (40 x 40, 0.08 % survive) 441 -> 3.9 ms, 36 x 36
+// Bernoulli(1/2) (6-13 % survive) 67-76 -> 18-29 ms by the matrix.
 #pragma once
 
 #include "exact_glynn.cuh"

@@ -32,8 +32,9 @@
 // matrices 5x5 3.72 -> 0.76 ms, 8x8 7.86 -> 1.38, 14x14 48.1 -> 17.9 (a lane
 // per row: 0.73, 1.96, 97.9), 16 of order 4 95 -> 73 us (77).
 //
-// FP32-pipe bound: about 46 operations per row and state.  16 x 26x26 with
-// the forward walk: 114.3 -> 37.9 ms against a lane per row with a shuffle
+// About 46 FP32 operations per row and state; two warps a scheduler wait on
+// dependent ones (issue 62 %, FMA pipe 46 %).  16 x 26x26 with the forward
+// walk: 114.3 -> 36.1 ms against a lane per row with a shuffle
 // butterfly for the product and a double-float division per row for E_i;
 // error against 64 bits 9.5e-12 -> 5.5e-13.
 #pragma once

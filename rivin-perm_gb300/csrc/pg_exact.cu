@@ -320,7 +320,7 @@ static void binary_rows(const int64_t *A, int n, bool transposed, BinaryRows *B)
 // batches (order 27), where a few batches hold all that is left: at order 24
 // Bernoulli(1/2) 0.048/0.037/0.040 -> 0.044/0.056/0.068 ms, but at order 28
 // 0.21/0.18/0.21 -> 0.16/0.12/0.13, and the 4x4x5 grid with shuffled columns
-// 20 -> 2-3.
+// 20 -> 2-4.
 constexpr int BINARY_ORDER_LOG = 11;
 static void binary_order_columns(int n, int low, BinaryRows *B) {
     uint64_t left = (1ull << n) - 1;

@@ -8,16 +8,16 @@
                                  (perm_parallel.py:104-164), real matrices
     glynn_window(A, lo, hi)      Glynn sum over a Gray window (one matrix)
 
-Orders up to 32 run the forward and the gradient in one traversal; orders
-33..63 run the forward only (two rows per lane), as the reference's
-permanent_parallel_real / _complex accept n <= 63.
+Orders up to 32 run the forward walk and, where it is asked for, a gradient
+walk beside it; orders 33..63 run the forward only (two rows per lane), as
+the reference's permanent_parallel_real / _complex accept n <= 63.
 
 The forward and the gradient d per / d a_ij = per(A without row i, column j)
-come out of one Glynn traversal (pg_glynn_f64_dev).  The backward of the
-autograd Function is the hand-written gradient from that traversal, scaled
-by the incoming gradient.  Every result carries the sum of |terms| it was
-accumulated from (scaled by 2^(1-n)), the scale against which its relative
-error is stated.
+come out of one call (pg_glynn_f64_dev), the permanents always from the
+forward walk.  The backward of the autograd Function is that call's
+hand-written gradient, scaled by the incoming gradient.  Every result carries
+the sum of |terms| it was accumulated from (scaled by 2^(1-n)), the scale
+against which its relative error is stated.
 """
 
 from __future__ import annotations
@@ -90,7 +90,7 @@ def _function():
 
     class GlynnPermanent(torch.autograd.Function):
         """per(A) over the last two dimensions, FP64, with the hand-written
-        Glynn gradient computed in the same GPU traversal as the forward."""
+        Glynn gradient computed in the same call as the forward."""
 
         @staticmethod
         def forward(ctx, A):
