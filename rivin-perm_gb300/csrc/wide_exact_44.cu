@@ -6,14 +6,14 @@ namespace pg {
 // Every order from 16 on (and 12, for short walks): a padded row is one more
 // factor of the product tree and often one more word of its products.  Odd
 // orders against the next even one's shape: 17..29 2 to 10 % faster (27 x 27 of
-// 38 bits 7.13 -> 6.65 ms), order 29 below 2^44 4 % slower.
+// 38 bits 7.13 -> 6.65 ms), but 29 below 2^44 31.6 ms against 30.5 and left out.
 bool wide_entry_44(int n, WideEntry *out) {
     return wide_entry<12, 44>(n, out) || wide_entry<16, 44>(n, out) || wide_entry<17, 44>(n, out) ||
            wide_entry<18, 44>(n, out) || wide_entry<19, 44>(n, out) || wide_entry<20, 44>(n, out) ||
            wide_entry<21, 44>(n, out) || wide_entry<22, 44>(n, out) || wide_entry<23, 44>(n, out) ||
            wide_entry<24, 44>(n, out) || wide_entry<25, 44>(n, out) || wide_entry<26, 44>(n, out) ||
-           wide_entry<27, 44>(n, out) || wide_entry<28, 44>(n, out) || wide_entry<29, 44>(n, out) ||
-           wide_entry<30, 44>(n, out) || wide_entry<31, 44>(n, out) || wide_entry<32, 44>(n, out);
+           wide_entry<27, 44>(n, out) || wide_entry<28, 44>(n, out) || wide_entry<30, 44>(n, out) ||
+           wide_entry<31, 44>(n, out) || wide_entry<32, 44>(n, out);
 }
 
 }  // namespace pg
