@@ -633,6 +633,11 @@ static int plan_launch(ExactPlan *P, cudaStream_t stream) {
         while (b.log_steps > 1 && P->batches_left * (chunks >> b.log_steps) < 8 * warps &&
                (chunks >> b.log_steps) < 64 * warps)
             b.log_steps--;
+        // single chunks where less than a quarter of the warps would get two
+        // (one warp evaluates all that survive of a batch): a window of 4096
+        // states at order 24 55 -> 49 us, 34 70 -> 61; at a half and more the
+        // second chunk's preparation costs 2-6 %
+        if (b.log_steps == 1 && (chunks >> 1) < warps / 4) b.log_steps = 0;
         const uint64_t batches = (((P->hi - 1) >> (BIN_LOW + b.log_steps)) - (P->lo >> (BIN_LOW + b.log_steps))) + 1;
         b.log_batches = 0;
         while ((1ull << b.log_batches) < batches) b.log_batches++;
