@@ -29,7 +29,7 @@
 // batches at once, one a lane; then the chunk rows, by bytes.  A whole walk
 // orders its columns so that such rows exist (binary_order_columns).  4x4x5
 // grid with a few bonds removed and columns shuffled: 34.9 ms without these
-// tests, 25.7 with them (one batch at a time), 6.2 with ordered columns; 2.6-4.3
+// tests, 25.7 with them (one batch at a time), 6.2 with ordered columns; 2.6-4.7
 // by which bonds are removed with the batches of a unit tested together and taken from all over the
 // walk (neighbours are zero together, and warps ran dry).
 //
